@@ -70,9 +70,9 @@ struct cupic_batch {
   // the batched solve's layout knobs in use: halo depth cap, CTA multiple;
   // tuned_n: the member count they were tuned for (0: not tuned)
   int knob_depth = 4, knob_mult = 1, tuned_n = 0;
-  // batched steps since d_halo was last zeroed: a halo word's epoch holds
-  // the solve count in 16 bits, so the words are zeroed before it can wrap
-  int64_t epoch_steps = 0;
+  // exchanges of a member since d_halo was last zeroed: a halo word's epoch
+  // counts them in 32 bits, so the words are zeroed before it can come round
+  int64_t epoch_use = 0, max_exchanges = 0;  // max_exchanges: most a step's solve can make
   size_t nhalo = 0;
 };
 
@@ -277,7 +277,10 @@ int layout_solve(cupic_batch *b, const Knobs &kn) {
   // a region may hold another instance's words with a matching epoch
   CU(cudaMemsetAsync(b->d_halo, 0, sizeof(unsigned long long) * nhalo, b->stream));
   b->nhalo = nhalo;
-  b->epoch_steps = 0;
+  b->epoch_use = 0;
+  b->max_exchanges = 0;
+  for (const cupic_ctx *c : b->members)
+    b->max_exchanges = std::max<int64_t>(b->max_exchanges, (int64_t)c->p.max_sweeps + 4);
   b->nflags = nflags;
   std::vector<JacobiArgs> jargs(n);
   size_t of = 0, orr = 0, oh = 0;
@@ -611,9 +614,9 @@ int cupic_batch_step(cupic_batch *b, int32_t nsteps) {
     if (rc) return rc;
   }
   for (int s = 0; s < nsteps; ++s) {
-    if (++b->epoch_steps > 65000) {  // before the members' solve counts can wrap
+    if ((b->epoch_use += b->max_exchanges) > (1ll << 30)) {  // before the epochs can come round
       CU(cudaMemsetAsync(b->d_halo, 0, sizeof(unsigned long long) * b->nhalo, b->stream));
-      b->epoch_steps = 1;
+      b->epoch_use = b->max_exchanges;
     }
     if (b->graph_ok) {
       CU(cudaGraphLaunch(b->graph, b->stream));

@@ -299,44 +299,51 @@ int jacobi_rows(const cupic_ctx *c, int G, int K, int P, long long rows_fit) {
   return B;
 }
 
-int alloc_jacobi_scratch(cupic_ctx *c, int G, long long GK, int P) {
+// exchange words, residual slots and counters of a layout, zeroed
+int alloc_jacobi_scratch(cupic_ctx *c, int G, size_t words) {
   dfree(c, c->jflags);
   dfree(c, c->jres);
   dfree(c, c->jhalo);
+  dfree(c, c->jgmax);
   c->jflags = nullptr;
   c->jres = nullptr;
   c->jhalo = nullptr;
+  c->jgmax = nullptr;
   CU(dalloc(c, &c->jflags, (size_t)G + 1));
   CU(dalloc(c, &c->jres, (size_t)2 * G));
-  CU(dalloc(c, &c->jhalo, (size_t)4 * GK * P));
-  c->jhalo_words = (size_t)4 * GK * P;
+  CU(dalloc(c, &c->jhalo, words));
+  CU(dalloc(c, &c->jgmax, (size_t)130));
+  c->jhalo_words = words;
   // epoch 0 is never valid; the solves on the context's stream follow the clearing
-  CU(cudaMemsetAsync(c->jhalo, 0, sizeof(unsigned long long) * c->jhalo_words, c->stream));
-  c->epoch_solves = 0;
+  CU(cudaMemsetAsync(c->jhalo, 0, sizeof(unsigned long long) * words, c->stream));
+  CU(cudaMemsetAsync(c->jgmax, 0, sizeof(unsigned long long) * 130, c->stream));
+  c->epoch_use = 0;
   return CUPIC_OK;
 }
 
-// A halo word carries the epoch (solve count << 16) + exchange index in 32
-// bits, so the solve count wraps every 65,536 solves.  A slot that the
-// solves since stopped rewriting (tolerance-stopped solves end after
-// different numbers of exchanges) could then hold a word whose epoch matches
-// again.  Before `solves` more solves are enqueued, the halo words are
-// zeroed (epoch 0 never matches) whenever the count since the last clearing
-// would reach kEpochGuard, ordered on the context's stream before them.
-constexpr int64_t kEpochGuard = 65000;
-int epoch_guard(cupic_ctx *c, int64_t solves) {
-  if (c->jhalo && c->epoch_solves + solves > kEpochGuard) {
+// A halo word carries the epoch of its exchange in 32 bits, counted over all
+// solves of the context, so epochs come round again after about 3e9
+// exchanges.  A slot that the solves since stopped rewriting (solves end
+// after different numbers of exchanges) could then hold a word whose epoch
+// matches again.  Before a solve is enqueued, the halo words are zeroed
+// (epoch 0 never matches) whenever the exchanges since the last clearing
+// could reach kEpochGuard, ordered on the context's stream before it.
+// exchanges: an upper bound of those the enqueued solves can make.
+constexpr int64_t kEpochGuard = 1ll << 30;
+int epoch_guard(cupic_ctx *c, int64_t exchanges) {
+  if (c->jhalo && c->epoch_use + exchanges > kEpochGuard) {
     CU(cudaMemsetAsync(c->jhalo, 0, sizeof(unsigned long long) * c->jhalo_words, c->stream));
-    c->epoch_solves = 0;
+    c->epoch_use = 0;
   }
-  c->epoch_solves += solves;
+  c->epoch_use += exchanges;
   return CUPIC_OK;
 }
 
-// solves (Jacobi launches) one solve of at most mx sweeps enqueues
+// exchanges one solve of at most mx sweeps can make, over its Jacobi launches
 int64_t solves_of(const cupic_ctx *c, int mx) {
   const int m = c->p.refine_every;
-  return m > 0 ? 1 + (std::max(mx, 0) + m - 1) / m : 1;
+  const int64_t launches = m > 0 ? 1 + (std::max(mx, 0) + m - 1) / m : 1;
+  return std::max(mx, 0) + 4 * launches;
 }
 
 int set_jacobi_plan(cupic_ctx *c, int G, int B, int K, int P) {
@@ -344,8 +351,26 @@ int set_jacobi_plan(cupic_ctx *c, int G, int B, int K, int P) {
   c->jB = B;
   c->jK = G > 1 ? K : 1;
   c->jP = P;
+  c->tile.R = 0;
   CU(jacobi_set_smem(jacobi_smem_bytes(B, c->jK, P)));
-  return alloc_jacobi_scratch(c, G, (long long)G * c->jK, P);
+  return alloc_jacobi_scratch(c, G, (size_t)4 * G * c->jK * P);
+}
+
+int set_tile_plan(cupic_ctx *c, const TilePlan &t) {
+  c->jG = t.G;
+  c->jB = t.B;
+  c->jK = t.K;
+  c->jP = (c->a.nnx + 3) / 4 * 4;
+  c->tile = t;
+  int n = 0;
+  CU(tile_max_ctas(t, c->num_sms, &n));
+  if (t.G > n) return CUPIC_ERR_ARG;
+  return alloc_jacobi_scratch(c, t.G, t.words);
+}
+
+// whether the context's solves may run as register tiles
+bool tiles_apply(const cupic_ctx *c) {
+  return c->p.refine_every == 0 && !getenv("CUPIC_JACOBI_NOSTRIP") && !getenv("CUPIC_JACOBI_SCALAR");
 }
 
 // The fixed rule, used when tuning is off or a layout is forced with
@@ -381,6 +406,15 @@ int plan_jacobi_rule(cupic_ctx *c, int P, long long rows_fit) {
   }
   if (B + 2 * K > rows_fit) return CUPIC_ERR_ARG;
   if (!jacobi_rows(c, G, K, P, rows_fit)) return CUPIC_ERR_ARG;
+  // the same CTAs and depth as register tiles, where a division of the CTAs
+  // into columns of blocks allows it
+  if (tiles_apply(c))
+    for (int nbx = 1; nbx <= G; ++nbx) {
+      TilePlan t;
+      if (G % nbx == 0 && tile_plan(c->a.nnx, c->a.nny, nbx, G / nbx, K, 0, true, &t) &&
+          set_tile_plan(c, t) == CUPIC_OK)
+        return CUPIC_OK;
+    }
   return set_jacobi_plan(c, G, B, K, P);
 }
 
@@ -442,7 +476,7 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
     }
   }
   if (cands.empty()) return plan_jacobi_rule(c, P, rows_fit);
-  int rc = alloc_jacobi_scratch(c, maxG, maxGK, P);
+  int rc = alloc_jacobi_scratch(c, maxG, (size_t)4 * maxGK * P);
   if (rc) return rc;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CU(cudaEventCreate(&e0));
@@ -492,6 +526,89 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
   return set_jacobi_plan(c, pick.G, pick.B, pick.K, P);
 }
 
+// Register tiles: the layouts with the lowest estimated cost are timed on
+// the context's buffers, with the checks of the solve it will run, and the
+// fastest is kept, per device, mesh shape and check interval.  Returns
+// CUPIC_ERR_CAPACITY when no layout holds the mesh.
+struct TileKey {
+  int device, nnx, nny, chk, sweeps, early;
+  bool operator<(const TileKey &o) const {
+    return std::tie(device, nnx, nny, chk, sweeps, early) <
+           std::tie(o.device, o.nnx, o.nny, o.chk, o.sweeps, o.early);
+  }
+};
+std::map<TileKey, TilePlan> g_tiles;
+constexpr int kTileTrials = 16;
+
+int tune_tiles(cupic_ctx *c, int dev_max) {
+  const int chk = std::max(1, c->p.check_every);
+  const int S = std::max(1, std::min(std::max(c->p.max_sweeps, c->p.init_max_sweeps), 256));
+  const int early = c->p.tol > 0.0 && c->p.min_sweeps < c->p.max_sweeps;
+  const TileKey key{c->device, c->a.nnx, c->a.nny, chk, S, early};
+  {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_tiles.find(key);
+    if (it != g_tiles.end()) return set_tile_plan(c, it->second);
+  }
+  const std::vector<TilePlan> all = tile_plans(c->a.nnx, c->a.nny, c->num_sms, true, (size_t)dev_max - 1024);
+  std::vector<TilePlan> cands;
+  size_t words = 0;
+  int maxG = 1;
+  for (const TilePlan &t : all) {
+    int n = 0;
+    if (tile_max_ctas(t, c->num_sms, &n) != cudaSuccess || t.G > n) {
+      cudaGetLastError();
+      continue;
+    }
+    cands.push_back(t);
+    words = std::max(words, t.words);
+    maxG = std::max(maxG, t.G);
+    if ((int)cands.size() >= kTileTrials) break;
+  }
+  if (cands.empty()) return CUPIC_ERR_CAPACITY;
+  TilePlan pick = cands.front();
+  if (cands.size() > 1) {
+    const int rc = alloc_jacobi_scratch(c, maxG, words);
+    if (rc) return rc;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    CU(cudaEventCreate(&e0));
+    CU(cudaEventCreate(&e1));
+    float best = 1e30f;
+    for (const TilePlan &t : cands) {
+      c->tile = t;
+      JacobiArgs J = jargs(c, early ? 1.0 : 0.0, early ? 1 : S, S, chk, 1);
+      J.trial = 1;
+      float ms_best = 1e30f;
+      bool ok = true;
+      for (int rep = 0; rep < 3 && ok; ++rep) {
+        ok = cudaEventRecord(e0, c->stream) == cudaSuccess &&
+             launch_tile(c->a, J, t, c->stream) == cudaSuccess &&
+             cudaEventRecord(e1, c->stream) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess;
+        float ms = 0.0f;
+        if (ok && rep > 0 && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess) ms_best = std::min(ms_best, ms);
+      }
+      if (!ok) {
+        cudaGetLastError();
+        continue;
+      }
+      if (ms_best < best) {
+        best = ms_best;
+        pick = t;
+      }
+    }
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    // a solve that gave up waiting leaves a flag: clear what the trials raised
+    CU(cudaMemsetAsync(&c->ctl->step_flags, 0, sizeof(uint32_t), c->stream));
+    CU(cudaStreamSynchronize(c->stream));
+  }
+  {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    g_tiles[key] = pick;
+  }
+  return set_tile_plan(c, pick);
+}
+
 int plan_jacobi(cupic_ctx *c) {
   int dev_max = 0;
   CU(cudaDeviceGetAttribute(&dev_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
@@ -501,6 +618,10 @@ int plan_jacobi(cupic_ctx *c) {
   const char *tune = getenv("CUPIC_JACOBI_TUNE");
   if (getenv("CUPIC_JACOBI_CTAS") || getenv("CUPIC_JACOBI_DEPTH") || (tune && atoi(tune) == 0))
     return plan_jacobi_rule(c, P, rows_fit);
+  if (tiles_apply(c)) {
+    const int rc = tune_tiles(c, dev_max);
+    if (rc != CUPIC_ERR_CAPACITY) return rc;
+  }
   return tune_jacobi(c, P, rows_fit);
 }
 
@@ -524,7 +645,16 @@ JacobiArgs jargs(const cupic_ctx *c, double tol, int mn, int mx, int chk, int fi
   J.bar = c->jflags + c->jG;
   J.res_cta = c->jres;
   J.halo = c->jhalo;
+  J.gmax = c->jgmax;
+  J.tbar = reinterpret_cast<unsigned *>(c->jgmax + 128);
+  if (c->tile.R) tile_args(c->tile, &J);
   return J;
+}
+
+// one solve with the context's layout
+cudaError_t launch_solve(const cupic_ctx *c, const JacobiArgs &J) {
+  if (J.max_sweeps < 1 && !J.r64_phi && !J.phi) return launch_field(c->a, J.do_field, J.write_stats, c->stream);
+  return c->tile.R ? launch_tile(c->a, J, c->tile, c->stream) : launch_jacobi(c->a, J, c->stream);
 }
 
 int set_phi_both(cupic_ctx *c, const double *phi) {
@@ -636,7 +766,7 @@ int run_solve(cupic_ctx *c, double tol, int mn, int mx, int chk, int field, int 
                                    : refine_solve(c, tol, mn, mx, field, write_stats);
   JacobiArgs J = jargs(c, tol, mn, mx, chk, field);
   J.write_stats = write_stats;
-  CU(launch_jacobi(c->a, J, c->stream));
+  CU(launch_solve(c, J));
   return CUPIC_OK;
 }
 
@@ -647,9 +777,9 @@ int run_step_solve(cupic_ctx *c, bool *zeroed) {
   *zeroed = false;
   if (p.refine_every > 0) return run_solve(c, p.tol, p.min_sweeps, p.max_sweeps, p.check_every, 1);
   JacobiArgs J = jargs(c, p.tol, p.min_sweeps, p.max_sweeps, p.check_every, 1);
-  J.zero_next = 1;
-  CU(launch_jacobi(c->a, J, c->stream));
-  *zeroed = true;
+  J.zero_next = p.max_sweeps > 0;
+  CU(launch_solve(c, J));
+  *zeroed = J.zero_next;
   return CUPIC_OK;
 }
 
@@ -1184,6 +1314,7 @@ int cupic_destroy(cupic_ctx *c) {
   dfree(c, c->jflags);
   dfree(c, c->jres);
   dfree(c, c->jhalo);
+  dfree(c, c->jgmax);
   dfree(c, c->io_buf);
   dfree(c, c->phi64);
   dfree(c, c->b64);
@@ -1442,11 +1573,7 @@ int cupic_field_solver(cupic_ctx *c) {
   if (c->p.refine_every > 0) {
     CU(launch_r64_field(c->a, c->phi64, c->stream));
   } else {
-    JacobiArgs J = jargs(c, 0.0, 0, 0, 1, 1);
-    J.write_stats = 0;
-    int rc = epoch_guard(c, 1);
-    if (rc) return rc;
-    CU(launch_jacobi(c->a, J, c->stream));
+    CU(launch_field(c->a, 1, 0, c->stream));
   }
   return finish(c);
 }

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "cupic_internal.cuh"
+#include "kernels.h"
 
 using cupic::Ctl;
 using cupic::SimArgs;
@@ -26,13 +27,15 @@ struct cupic_ctx {
   int64_t total_cap[2] = {0, 0};
   // Jacobi geometry and exchange buffers
   int jG = 1, jB = 1, jK = 1, jP = 0;
+  cupic::TilePlan tile{};  // register-tile layout (R == 0: the shared-memory sweep of jacobi.cu)
+  unsigned long long *jgmax = nullptr;  // [128] maxima of checked sweeps, then [4] counters; zeroed
   bool jNoStrip = false;  // the tuner found the shared-memory sweep faster than register strips
   unsigned *jflags = nullptr;  // [G+1]: per-CTA sweep counters, then the barrier
   float *jres = nullptr;
   unsigned long long *jhalo = nullptr;  // halo words, zeroed at allocation
   size_t jhalo_words = 0;
-  // solves enqueued since the halo words were last zeroed (see epoch_guard)
-  int64_t epoch_solves = 0;
+  // exchanges enqueued since the halo words were last zeroed (see epoch_guard)
+  int64_t epoch_use = 0;
   // precision form of the solve (refine_every > 0): FP64 potential, FP32
   // residual source and correction, the residual's max norm
   double *phi64 = nullptr;

@@ -37,7 +37,7 @@ struct Ctl {
   int32_t abort;          // a bounded wait gave up: kernels bail out
   int32_t halt;           // a row cannot take the step's arrivals: the rest of the run is idle
   int32_t skipped;        // steps whose bookkeeping found the run halted (the halted one included)
-  uint32_t jepoch;        // solves run so far: the base of the halo words' epochs
+  uint32_t jepoch;        // exchanges of all solves so far: the base of the halo words' epochs
   uint32_t idle;          // never written: the bounded-wait self-test waits on it
   int32_t refine_done;    // precision-form solve: the stop test passed, later corrections idle
   uint32_t jdone;         // CTAs of the running solve that have finished (the last one resets it)
@@ -88,6 +88,15 @@ struct JacobiArgs {
   double tol;
   int32_t min_sweeps, max_sweeps, check_every;
   int32_t G;              // CTAs (cooperative)
+  // register tiles (tile.cuh): rows of a strip (0: the shared-memory sweep of
+  // jacobi.cu), tile mode, blocks in x and y (G = nbx * nby), lanes of a
+  // strip, strips per warp, warps, exchange row pitch in words
+  int32_t tile, mode, nbx, nby, nl, segs, warps, ip;
+  int32_t trows, tpairs, ppairs;  // rows of the exchange image, entries of the tables of words in and out
+  uint32_t pwords;        // exchange words of one parity
+  int32_t trial;          // 1: a timing run, checked but never stopped
+  unsigned long long *gmax;  // [4][32] {epoch, max |dphi|} of the checked sweeps of 4 blocks in turn
+  unsigned int *tbar;        // [4] CTAs whose maxima are in, zero between solves
   int32_t rows_per_cta;   // most interior rows owned by one CTA: ceil((nny-2)/G)
   int32_t depth;          // temporal blocking: sweeps between halo exchanges (G > 1)
   int32_t pitch;          // smem row pitch in floats (a multiple of 4)
@@ -118,6 +127,12 @@ struct JacobiArgs {
   double r64_tol;
   int32_t r64_done, r64_mn, r64_mx, r64_stats;
 };
+
+// The epochs of the halo words: exchange e of a solve writes ctl->jepoch + e
+// (e >= 1), and the solve's last CTA moves the base past them.  The base goes
+// back to 0 once it has passed kEpochEnd; the host zeroes the words (epoch 0
+// never matches) more often than that.
+constexpr unsigned kEpochEnd = 0xc0000000u;
 
 // a group of CTAs of the batched solve and its instances (list[begin..end))
 struct JGroup {

@@ -357,10 +357,10 @@ __device__ __forceinline__ void jacobi_body(const SimArgs &a, const JacobiArgs &
 
   float *const phi = J.phi ? J.phi : a.phi;
   const long long *acc = reinterpret_cast<const long long *>(a.rho[ctl->cur]);
-  // epochs of this solve's exchanges e = 1, 2, ...: (solve count << 16) + e,
-  // never 0 (the cleared buffer) and never those of an earlier solve's
-  // words still in the buffer
-  const unsigned ebase = *reinterpret_cast<volatile unsigned *>(&ctl->jepoch) << 16;
+  // epochs of this solve's exchanges e = 1, 2, ...: ebase + e, never 0 (the
+  // cleared buffer) and never those of an earlier solve's words still in
+  // the buffer
+  const unsigned ebase = *reinterpret_cast<volatile unsigned *>(&ctl->jepoch);
   if (J.zero_next) {
     // the accumulator the step's push deposits into: this CTA's rows, and
     // the boundary rows from the first and last CTA
@@ -737,7 +737,10 @@ __device__ __forceinline__ void jacobi_body(const SimArgs &a, const JacobiArgs &
     __threadfence();
     if (atomicAdd(&ctl->jdone, 1u) == (unsigned)G - 1u) {
       ctl->jdone = 0u;
-      atomicAdd(&ctl->jepoch, 1u);
+      const unsigned next = ebase + (unsigned)(done / K) + 2u;
+      ctl->jepoch = next > kEpochEnd ? 0u : next;
+      if (next > kEpochEnd && J.gmax)
+        for (int k = 0; k < 128; ++k) J.gmax[k] = 0ull;
     }
   }
 }

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <vector>
+
 #include "cupic_internal.cuh"
 
 namespace cupic {
@@ -49,6 +51,28 @@ int jacobi_strip_rows(int nnx, int urows);
 cudaError_t jacobi_set_smem(size_t bytes);
 cudaError_t jacobi_max_ctas(size_t smem, int *per_sm);
 cudaError_t launch_jacobi(const SimArgs &a, const JacobiArgs &J, cudaStream_t st);
+
+// the register-tile solve (tile.cuh, tile.cu)
+constexpr int kTileWarps = 16;  // most warps of a CTA
+constexpr int kTileDepth = 16;  // deepest halo
+struct TilePlan {
+  int R;                   // rows of a strip
+  int mode;                // 0 halo, 1 ring, 2 ragged ring
+  int nbx, nby, G, K;      // blocks in x and y, their product, halo depth
+  int B;                   // most rows a block owns
+  int nl, segs, warps, ip; // lanes of a strip, strips per warp, warps, exchange row pitch
+  int trows, tpairs, ppairs;  // rows of the exchange image, entries of the tables of words in and out
+  size_t smem, words;      // dynamic shared memory; exchange words
+  double cost;             // estimated SM cycles per sweep
+};
+// early: the solve may stop on its tolerance (and then keeps snapshots)
+bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, bool early, TilePlan *out);
+std::vector<TilePlan> tile_plans(int nnx, int nny, int max_ctas, bool early, size_t max_smem);
+void tile_args(const TilePlan &t, JacobiArgs *J);
+cudaError_t tile_max_ctas(const TilePlan &t, int num_sms, int *ctas);
+cudaError_t launch_tile(const SimArgs &a, const JacobiArgs &J, const TilePlan &t, cudaStream_t st);
+// the field of the stored potential, and the report of a solve of no sweeps
+cudaError_t launch_field(const SimArgs &a, int do_field, int write_stats, cudaStream_t st);
 
 // many contexts in one launch (batch.cu): SimArgs / JacobiArgs arrays in
 // device memory, work lists of {instance, row}

@@ -20,6 +20,8 @@
 #include <string.h>
 
 #include <algorithm>
+#include <map>
+#include <tuple>
 
 #include "cupic_internal.cuh"
 #include "kernels.h"
@@ -32,19 +34,23 @@ constexpr size_t kCtlHeadBytes = 256;  // the part of Ctl the solver touches
 static_assert(offsetof(Ctl, ring) <= kCtlHeadBytes, "solver status block");
 
 static __device__ __align__(256) unsigned char g_solver_scratch[kStaticScratchBytes];
+// the register tiles' maxima and counters (JacobiArgs::gmax, tbar), apart
+// from the scratch so that no layout's words lie over them
+static __device__ unsigned long long g_solver_sync[130];
 
-// device address of g_solver_scratch for each device, looked up once
+// device addresses of the arrays for each device, looked up once
 std::mutex g_mu;
 constexpr int kMaxDevices = 64;
 void *g_scratch_addr[kMaxDevices] = {};
-// calls since the array's halo words were last zeroed, per device: a halo
-// word's epoch holds the solve count in 16 bits, so the words are zeroed
-// before the count can wrap (epoch 0 never matches)
-long long g_calls[kMaxDevices] = {};
+void *g_sync_addr[kMaxDevices] = {};
+// exchanges since the array's halo words were last zeroed, per device: a
+// halo word's epoch counts them in 32 bits, so the words are zeroed before
+// the count can come round (epoch 0 never matches)
+long long g_exchanges[kMaxDevices] = {};
 
 // the array's device address on the current device; *clear: the call must
 // zero the halo words first
-int scratch_for_current_device(unsigned char **out, bool *clear) {
+int scratch_for_current_device(unsigned char **out, unsigned long long **sync, long long exchanges, bool *clear) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return CUPIC_ERR_CUDA;
   std::lock_guard<std::mutex> lock(g_mu);
@@ -54,15 +60,45 @@ int scratch_for_current_device(unsigned char **out, bool *clear) {
       cudaGetLastError();
       return CUPIC_ERR_CUDA;
     }
+    if (cudaGetSymbolAddress(&g_sync_addr[dev], g_solver_sync) != cudaSuccess) {
+      cudaGetLastError();
+      return CUPIC_ERR_CUDA;
+    }
     g_scratch_addr[dev] = ptr;
   }
-  *clear = ++g_calls[dev] > 65000;
-  if (*clear) g_calls[dev] = 1;
+  *clear = (g_exchanges[dev] += exchanges) > (1ll << 30);
+  if (*clear) g_exchanges[dev] = exchanges;
   *out = static_cast<unsigned char *>(g_scratch_addr[dev]);
+  *sync = static_cast<unsigned long long *>(g_sync_addr[dev]);
   return CUPIC_OK;
 }
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
+
+// The register tiles of a mesh: the layout of least estimated cost whose
+// words fit the scratch, on at most max_ctas CTAs; R == 0 when there is none.
+// Layouts depend only on the mesh and the device, and are kept.
+TilePlan tiles_for(int dev, int num_sms, int dev_max, int nnx, int nny, int max_ctas, bool early) {
+  static std::map<std::tuple<int, int, int, int, bool>, TilePlan> kept;
+  std::lock_guard<std::mutex> lock(g_mu);
+  const auto key = std::make_tuple(dev, nnx, nny, max_ctas, early);
+  const auto it = kept.find(key);
+  if (it != kept.end()) return it->second;
+  TilePlan pick{};
+  for (const TilePlan &t : tile_plans(nnx, nny, max_ctas, early, (size_t)dev_max - 1024)) {
+    int n = 0;
+    if (kCtlHeadBytes + sizeof(unsigned long long) * t.words > kStaticScratchBytes || t.G > max_ctas) continue;
+    if (tile_max_ctas(t, num_sms, &n) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    if (t.G > n) continue;
+    pick = t;
+    break;
+  }
+  if (kept.size() >= 256) kept.clear();
+  return kept[key] = pick;
+}
 
 }  // namespace
 }  // namespace cupic
@@ -78,8 +114,9 @@ extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t 
   if (p->ncx < 2 || p->ncy < 2 || p->ncx > 4096 || !(p->ds > 0) || !(p->eps0 > 0))
     return CUPIC_ERR_ARG;
   unsigned char *scratch = nullptr;
+  unsigned long long *sync = nullptr;
   bool clear_halo = false;
-  int rc = scratch_for_current_device(&scratch, &clear_halo);
+  int rc = scratch_for_current_device(&scratch, &sync, (long long)max_sweeps + 4, &clear_halo);
   if (rc) return rc;
   int dev = 0, num_sms = 0, dev_max = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -167,6 +204,17 @@ extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t 
   J.bar = flags + G;
   J.res_cta = res;
   J.halo = halo;
+  J.gmax = sync;
+  J.tbar = reinterpret_cast<unsigned *>(sync + 128);
+  // the mesh is one that the scratch holds; most run faster as register tiles
+  const bool early = max_error > 0.0 && min_sweeps < max_sweeps;
+  const TilePlan tile = max_sweeps > 0 ? tiles_for(dev, num_sms, dev_max, a.nnx, a.nny,
+                                                   std::min(forced > 0 ? forced : num_sms, num_sms), early)
+                                       : TilePlan{};
+  if (tile.R) {
+    tile_args(tile, &J);
+    J.halo = reinterpret_cast<unsigned long long *>(scratch + kCtlHeadBytes);
+  }
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // the array keeps the previous call's contents: clear the status block
@@ -177,7 +225,7 @@ extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t 
   if (clear_halo && cudaMemsetAsync(scratch + kCtlHeadBytes, 0, kStaticScratchBytes - kCtlHeadBytes, st) !=
                         cudaSuccess)
     return CUPIC_ERR_CUDA;
-  if (launch_jacobi(a, J, st) != cudaSuccess) return CUPIC_ERR_CUDA;
+  if ((tile.R ? launch_tile(a, J, tile, st) : launch_jacobi(a, J, st)) != cudaSuccess) return CUPIC_ERR_CUDA;
   struct {
     uint32_t step_flags;
     int32_t sweeps;

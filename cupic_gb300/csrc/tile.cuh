@@ -1,0 +1,771 @@
+// tile.cuh -- the Poisson solve with the whole tile in registers.
+//
+// CTA (bx, by) of an nbx x nby grid owns a block of the mesh and keeps it,
+// with a halo of K nodes on the sides that have neighbours, in registers for
+// the whole solve: a strip of R rows is held by one lane group, 4 columns a
+// lane, so a sweep (jacobi_iteration, mesh.cu:297-381) takes its west and
+// east neighbours from two shuffles a row, the rows inside a strip from
+// registers, and only the rows just below and above a strip from shared
+// memory (two 16-byte stores and loads a thread, one block barrier).
+//   nbx == 1 (rings)  the lanes of a strip hold a full mesh row and the
+//                     shuffles go around it (column 0's west neighbour is
+//                     column nnx-2); W = nnx-1 <= 128 columns, and several
+//                     strips share a warp where W is small.
+//   nbx > 1 (halo)    K (a multiple of 4) halo columns on each side, updated
+//                     redundantly like the halo rows, so no lane needs more
+//                     than its two neighbours, for every W.
+// Every K sweeps the blocks trade the K nodes inside each boundary as 64-bit
+// words {value, epoch} (one L2 round trip, no flag and no fence), written
+// from and read into registers.  Every value is computed with the same
+// operands in the same order on every layout, so all layouts give the same
+// bits.
+//
+// Convergence checks never wait in the sweep loop: the maxima of a block of
+// K sweeps are combined over the grid while the next block runs, and when
+// a sweep turns out to have passed the stop test the state at the start of
+// its block (kept in shared memory) is restored and swept up to it.
+//
+// What bounds it: the latency of a sweep on a small tile (350 cycles with one
+// row a thread: barrier, shared-memory rows, shuffles) and instruction issue
+// on a large one (18 a row and warp), plus the exchange (2900 cycles with two
+// neighbours, 5500-7300 with eight) every K sweeps.  Against the
+// shared-memory sweep and register strips of jacobi.cu, 200 sweeps in a step:
+// 512x2048 0.334 -> 0.182 ms, 256x1024 0.191 -> 0.115, 301x700 (rows of no
+// multiple of 4) 0.325 -> 0.110, 32x128 0.127 -> 0.052 ms; with a check after
+// each of 2000 sweeps, 64x256 5.0 -> 0.95 ms.
+#pragma once
+
+#include <math.h>
+
+#include "cupic_internal.cuh"
+#include "kernels.h"
+
+namespace cupic {
+namespace tile {
+
+enum { kHalo = 0, kRing = 1, kRingRagged = 2 };  // ragged: W % 4 != 0
+
+constexpr unsigned kFull = 0xffffffffu;
+constexpr int kSoloBlock = 32;  // sweeps between stop tests of a solve on one CTA
+constexpr long long kSpinLimit = 1ll << 22;
+
+__device__ __forceinline__ void st_word(unsigned long long *p, float v, unsigned ep) {
+  const unsigned long long w = ((unsigned long long)ep << 32) | __float_as_uint(v);
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+__device__ __forceinline__ void st_word2(unsigned long long *p, float v0, float v1, unsigned ep) {
+  const unsigned long long h = (unsigned long long)ep << 32;
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(h | __float_as_uint(v0)),
+               "l"(h | __float_as_uint(v1))
+               : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_word(const unsigned long long *p) {
+  unsigned long long w;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+  return w;
+}
+__device__ __forceinline__ void ld_word2(const unsigned long long *p, unsigned long long &a,
+                                         unsigned long long &b) {
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ float4 lds4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ void sts4(float *p, const float4 &v) { *reinterpret_cast<float4 *>(p) = v; }
+
+// static shared scratch
+struct Scratch {
+  unsigned cm[4][32];  // per-sweep maxima of a block of sweeps, 4 blocks in turn
+  int dec[2];          // a block's stop decision: index of the stopping sweep, or -1
+  float decv[2];       // its residual
+  int bail;
+};
+
+// one thread's place in its tile
+struct Lane {
+  int nvalid;        // rows of the strip
+  int row0;          // its first mesh row
+  int i0;            // extended column of element 0 (-K .. W+K-1)
+  int rm;            // ragged ring, last lane: valid elements (1..3), else 0
+  int srcw, srce;    // rings: lanes of the west and east neighbours
+  int me;            // element whose east neighbour is the mirror column (-1: none)
+  unsigned own;      // elements this CTA owns (bits 0..3)
+  unsigned ownrows;  // rows this CTA owns (bits 0..R-1)
+  bool full;         // no lane of the warp has a partial strip
+};
+
+__device__ __forceinline__ float node(float b, float w, float e, float n, float s) {
+  return __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(b, w), e), n), s));
+}
+
+// One sweep of a strip: v = 1/4 ((((b + west) + east) + north) + south).
+// FULL: all R rows of the strip are in the tile (the row above the last is
+// then x[R]'s place, taken from n4); otherwise the rows past the strip's end
+// compute values nothing reads.  FIRST: the solve's first sweep, which reads
+// the caller's mirror column (its value may differ from column 0's; every
+// later one equals it).  Returns the max |v - old| over owned nodes (CHECK).
+template <int R, int MODE, bool FULL, bool CHECK, bool FIRST>
+__device__ __forceinline__ float sweep(float4 (&x)[R], const float4 (&b)[R], const float4 s4,
+                                       const float4 n4, const Lane &g, const float *mirror, int nnx) {
+  float4 prev = s4;
+  float md = 0.0f;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const float4 c = x[r];
+    float lf, rt;
+    float4 e = make_float4(c.y, c.z, c.w, 0.0f);  // east neighbours
+    if (MODE == kHalo) {
+      lf = __shfl_up_sync(kFull, c.w, 1);
+      rt = __shfl_down_sync(kFull, c.x, 1);
+    } else {
+      float last = c.w;
+      if (MODE == kRingRagged) last = g.rm == 0 ? c.w : (g.rm == 1 ? c.x : (g.rm == 2 ? c.y : c.z));
+      lf = __shfl_sync(kFull, last, g.srcw);
+      rt = __shfl_sync(kFull, c.x, g.srce);
+      if (MODE == kRingRagged) {
+        e.x = g.rm == 1 ? rt : e.x;
+        e.y = g.rm == 2 ? rt : e.y;
+        e.z = g.rm == 3 ? rt : e.z;
+      }
+    }
+    e.w = rt;
+    float mir = 0.0f;
+    if (FIRST && mirror && r < g.nvalid && (g.me >= 0 || g.i0 == 0)) mir = mirror[(size_t)(g.row0 + r) * nnx];
+    if (FIRST && g.me >= 0) {
+      e.x = g.me == 0 ? mir : e.x;
+      e.y = g.me == 1 ? mir : e.y;
+      e.z = g.me == 2 ? mir : e.z;
+      e.w = g.me == 3 ? mir : e.w;
+    }
+    const float4 nx = r + 1 < R ? x[r + 1 < R ? r + 1 : r] : n4;
+    const float4 n = (r + 1 < R && !FULL && r + 1 >= g.nvalid) ? n4 : nx;
+    float4 v;
+    v.x = node(b[r].x, lf, e.x, n.x, prev.x);
+    v.y = node(b[r].y, c.x, e.y, n.y, prev.y);
+    v.z = node(b[r].z, c.y, e.z, n.z, prev.z);
+    v.w = node(b[r].w, c.z, e.w, n.w, prev.w);
+    if (CHECK) {
+      float d = (g.own & 1u) ? fabsf(__fsub_rn(v.x, c.x)) : 0.0f;
+      d = (g.own & 2u) ? fmaxf(d, fabsf(__fsub_rn(v.y, c.y))) : d;
+      d = (g.own & 4u) ? fmaxf(d, fabsf(__fsub_rn(v.z, c.z))) : d;
+      d = (g.own & 8u) ? fmaxf(d, fabsf(__fsub_rn(v.w, c.w))) : d;
+      if (FIRST && g.i0 == 0 && (g.own & 1u)) d = fmaxf(d, fabsf(__fsub_rn(v.x, mir)));
+      md = (g.ownrows >> r) & 1u ? fmaxf(md, d) : md;
+    }
+    x[r] = v;
+    prev = c;
+  }
+  return md;
+}
+
+template <int R, int MODE>
+__device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, const int c, float *sm,
+                                      Scratch *js) {
+  Ctl *ctl = a.ctl;
+  if (halted(ctl)) return;
+  const int G = J.G, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
+  const int nnx = a.nnx, nny = a.nny, W = nnx - 1, M = nny - 2;
+  const int nbx = MODE == kHalo ? J.nbx : 1, nby = J.nby;
+  const int K = J.depth;
+  const int bx = MODE == kHalo ? c % nbx : 0, by = MODE == kHalo ? c / nbx : c;
+  const int r0 = 1 + (int)(((long long)by * M) / nby), r1 = 1 + (int)(((long long)(by + 1) * M) / nby);
+  int x0 = 0, x1 = W;
+  if (MODE == kHalo) {
+    const int W4 = (W + 3) >> 2;
+    x0 = 4 * ((bx * W4) / nbx);
+    x1 = min(W, 4 * (((bx + 1) * W4) / nbx));
+  }
+  const int KX = MODE == kHalo ? K : 0;  // halo columns on each side
+  // updated rows lo..hi; rows lo-1 and hi+1 are the tile's edge rows
+  const int lo = nby > 1 ? max(1, r0 - (K - 1)) : 1, hi = nby > 1 ? min(nny - 2, r1 + K - 2) : nny - 2;
+  // lane -> strip
+  const int nl = J.nl, segs = J.segs;
+  const int seg = segs == 1 ? 0 : lane / nl, li = segs == 1 ? lane : lane - seg * nl;
+  const bool act = segs == 1 ? lane < nl : seg < segs;
+  Lane g;
+  g.row0 = lo + (warp * segs + seg) * R;
+  g.nvalid = act ? min(max(hi + 1 - g.row0, 0), R) : 0;
+  g.i0 = x0 - KX + 4 * li;
+  g.rm = MODE == kRingRagged && act && li == nl - 1 ? W - 4 * (nl - 1) : 0;
+  g.srcw = !act ? lane : (li == 0 ? lane + nl - 1 : lane - 1);
+  g.srce = !act ? lane : (li == nl - 1 ? lane - (nl - 1) : lane + 1);
+  g.me = -1;
+  g.own = 0u;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = g.i0 + q;
+    if (act && (i == W - 1 || i == -1)) g.me = q;
+    if (act && i >= x0 && i < x1) g.own |= 1u << q;
+  }
+  g.ownrows = 0u;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (r < g.nvalid && g.row0 + r >= r0 && g.row0 + r < r1) g.ownrows |= 1u << r;
+  g.full = __all_sync(kFull, !act || g.nvalid == R);
+  // shared memory: first and last rows of every strip in two parities, the
+  // edge rows of 4 blocks of sweeps in turn, then (below) the received halo
+  // nodes, the table of halo words and two snapshots of the strips
+  const int par = nthr * 4;
+  float *const first = sm, *const last = sm + 2 * par;
+  float *const edge = sm + 4 * par;  // [4][south, north][128]
+  const int mine = tid * 4;
+  const int soff = seg > 0 ? mine - 4 * nl : (warp - 1) * 128 + 4 * ((segs - 1) * nl + li);
+  const int noff = seg < segs - 1 ? mine + 4 * nl : (warp + 1) * 128 + 4 * li;
+  const bool south_edge = g.row0 == lo, north_edge = g.nvalid > 0 && g.row0 + g.nvalid - 1 == hi;
+  const bool idle = g.nvalid == 0;
+
+  float *const phi = J.phi ? J.phi : a.phi;
+  const long long *acc = reinterpret_cast<const long long *>(a.rho[ctl->cur]);
+  const unsigned ebase = *reinterpret_cast<volatile unsigned *>(&ctl->jepoch);
+  if (J.zero_next) {  // the accumulator the step's push deposits into, in equal shares
+    unsigned long long *nx = a.rho[ctl->cur ^ 1];
+    const long long nodes = (long long)nnx * nny;
+    for (long long k = nodes * c / G + tid; k < nodes * (c + 1) / G; k += nthr) nx[k] = 0ull;
+  }
+
+  // real column of element q of this lane (-1: none)
+  auto column = [&](int q) {
+    int i = g.i0 + q;
+    if (!act) return -1;
+    if (MODE == kHalo) return i < 0 ? i + W : (i >= W ? (i - W < W ? i - W : -1) : i);
+    return i < W ? i : -1;
+  };
+  float4 x[R], b[R];
+  {
+    const int c0 = column(0), c1 = column(1), c2 = column(2), c3 = column(3);
+    auto ldphi = [&](int j, int i) { return i >= 0 ? phi[(size_t)j * nnx + i] : 0.0f; };
+    auto ldsrc = [&](int j, int i) {
+      if (i < 0) return 0.0f;
+      const size_t rb = (size_t)j * nnx;
+      if (J.src) return J.src[rb + i];
+      const long long f = i == 0 ? acc[rb] + acc[rb + W] : acc[rb + i];
+      return __double2float_rn((double)f * a.cb);
+    };
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      x[r] = b[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < g.nvalid) {
+        const int j = g.row0 + r;
+        if (!J.phi_zero) x[r] = make_float4(ldphi(j, c0), ldphi(j, c1), ldphi(j, c2), ldphi(j, c3));
+        b[r] = make_float4(ldsrc(j, c0), ldsrc(j, c1), ldsrc(j, c2), ldsrc(j, c3));
+      }
+    }
+    if (!idle) {
+      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (south_edge)
+          sts4(edge + (2 * q) * 128 + 4 * li,
+               J.phi_zero ? z : make_float4(ldphi(lo - 1, c0), ldphi(lo - 1, c1), ldphi(lo - 1, c2), ldphi(lo - 1, c3)));
+        if (north_edge)
+          sts4(edge + (2 * q + 1) * 128 + 4 * li,
+               J.phi_zero ? z : make_float4(ldphi(hi + 1, c0), ldphi(hi + 1, c1), ldphi(hi + 1, c2), ldphi(hi + 1, c3)));
+      }
+    }
+    sts4(first + mine, x[0]);
+    sts4(last + mine, x[R - 1]);
+  }
+
+  // exchange words, two parities of: rows [by][bottom, top][K][ip] by
+  // extended column, then (halo tiles) columns [row][bx][left, right][K]
+  const int ip = J.ip, ipad = MODE == kHalo ? 16 : 0;
+  const unsigned vbase = (unsigned)nby * 2u * K * ip, pwords = J.pwords;
+  auto hrow = [&](int b_, int side, int k) { return (unsigned)(((b_ * 2 + side) * K + k) * ip + ipad); };
+  auto vcol = [&](int j, int b_, int side) { return vbase + (unsigned)(((j * nbx + b_) * 2 + side) * K); };
+  // Words go out and come in as pairs by way of an image of the tile in shared
+  // memory, shared out evenly over the threads by tables of {word offset,
+  // place in the image}.  In: rows of the blocks below and above over all the
+  // tile's columns (the outermost one to the edge row), then the columns
+  // beside the owned rows.  Out: the owned nodes within K of a boundary, and
+  // the periodic images of those within K of column 0 or W.  kEdge marks a
+  // place in the edge rows, kOne a single word (odd widths).
+  constexpr unsigned kEdge = 1u << 30, kOne = 1u << 31;
+  const int nc = x1 - x0 + 2 * KX, nc2 = (nc + 1) >> 1, h = r1 - r0;
+  const int nlow = by > 0 ? K * nc2 : 0, nhigh = by < nby - 1 ? K * nc2 : 0;
+  const int npair = G > 1 ? nlow + nhigh + (MODE == kHalo ? h * K : 0) : 0;
+  float *const timg = edge + 4 * 2 * 128;  // [hi-lo+1][128]: halo nodes of the strips
+  uint2 *const table = reinterpret_cast<uint2 *>(timg + (size_t)J.trows * 128);
+  uint2 *const ptable = table + J.tpairs;
+  float4 *const snap = reinterpret_cast<float4 *>(ptable + J.ppairs);
+  for (int u = tid; u < npair; u += nthr) {
+    uint2 t;
+    int q, j, col;  // word offset, mesh row, tile column of the pair
+    bool one = false;
+    if (u < nlow + nhigh) {
+      const bool low = u < nlow;
+      const int v = low ? u : u - nlow, k = v / nc2;
+      col = 2 * (v - k * nc2);
+      one = col + 1 >= nc;
+      j = low ? r0 - K + k : r1 + k;
+      q = (int)hrow(low ? by - 1 : by + 1, low ? 1 : 0, k) + x0 - KX + col;
+    } else {
+      const int v = u - nlow - nhigh, row = v / K, k = v - row * K;  // K/2 pairs left, K/2 right
+      const bool left = k < (K >> 1);
+      const int kk = 2 * (left ? k : k - (K >> 1));
+      j = r0 + row;
+      col = left ? kk : nc - K + kk;
+      q = (int)(left ? vcol(j, bx == 0 ? nbx - 1 : bx - 1, 1) : vcol(j, bx + 1 == nbx ? 0 : bx + 1, 0)) + kk;
+    }
+    t.x = (unsigned)q;
+    if (j < lo) t.y = kEdge | (unsigned)col;
+    else if (j > hi) t.y = kEdge | (unsigned)(128 + col);
+    else t.y = (unsigned)((j - lo) * 128 + col);
+    if (one) t.y |= kOne;
+    table[u] = t;
+  }
+  const int w = x1 - x0, w2 = (w + 1) >> 1;
+  const int plow = by > 0 ? K * w2 : 0, phigh = by < nby - 1 ? K * w2 : 0;
+  // the image words of a row: as pairs when W is even, else one by one
+  const int ni = W & 1 ? K : K >> 1, istep = W & 1 ? 1 : 2;
+  const bool im0 = MODE == kHalo && x0 < K, im1 = MODE == kHalo && x1 > W - K;
+  const int nside = MODE == kHalo ? h * K : 0;
+  const int nimg = ((im0 ? 1 : 0) + (im1 ? 1 : 0)) * ni * ((by > 0 ? K : 0) + (by < nby - 1 ? K : 0));
+  const int nout = G > 1 ? plow + phigh + nside + nimg : 0;
+  for (int u = tid; u < nout; u += nthr) {
+    uint2 t;
+    int q, j, i;  // word offset, mesh row, owned column of the first word
+    bool one = false;
+    if (u < plow + phigh) {
+      const bool low = u < plow;
+      const int v = low ? u : u - plow, k = v / w2;
+      i = x0 + 2 * (v - k * w2);
+      one = i + 1 >= x1;
+      j = low ? r0 + k : r1 - K + k;
+      q = (int)hrow(by, low ? 0 : 1, k) + i;
+    } else if (u < plow + phigh + nside) {
+      const int v = u - plow - phigh, row = v / K, k = v - row * K;
+      const bool left = k < (K >> 1);
+      const int kk = 2 * (left ? k : k - (K >> 1));
+      j = r0 + row;
+      i = left ? x0 + kk : x1 - K + kk;
+      q = (int)vcol(j, bx, left ? 0 : 1) + kk;
+    } else {
+      int v = u - plow - phigh - nside;
+      const int per = (im0 ? ni : 0) + (im1 ? ni : 0), row = v / per;
+      v -= row * per;
+      const bool at0 = im0 && v < ni;  // columns 0..K-1 again at W..W+K-1
+      const int k = istep * (at0 ? v : v - (im0 ? ni : 0));
+      i = at0 ? k : W - K + k;
+      one = istep == 1;
+      const bool low = by > 0 && row < K;
+      const int kr = low ? row : row - (by > 0 ? K : 0);
+      j = low ? r0 + kr : r1 - K + kr;
+      q = (int)hrow(by, low ? 0 : 1, kr) + (at0 ? i + W : i - W);
+    }
+    t.x = (unsigned)q;
+    t.y = (unsigned)((j - lo) * 128 + i - x0 + KX);
+    if (one) t.y |= kOne;
+    ptable[u] = t;
+  }
+  // this thread's nodes that go out: rows within K of the block's bottom and
+  // top, and every owned row of the lanes within K of its sides
+  unsigned outrows = 0u;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int j = g.row0 + r;
+    if ((g.ownrows >> r) & 1u)
+      if ((by > 0 && j < r0 + K) || (by < nby - 1 && j >= r1 - K) ||
+          (MODE == kHalo && g.own && (g.i0 < x0 + K || g.i0 + 3 >= x1 - K)))
+        outrows |= 1u << r;
+  }
+  // owned nodes into the image; then, after a barrier, out of it
+  auto show = [&]() {
+    float *const q = timg + (g.row0 - lo) * 128 + 4 * li;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if ((outrows >> r) & 1u) sts4(q + r * 128, x[r]);
+  };
+  auto publish = [&](int e) {
+    const unsigned ep = ebase + (unsigned)e;
+    unsigned long long *const hw = J.halo + ((e & 1) ? pwords : 0u);
+#pragma unroll 4
+    for (int u = tid; u < nout; u += nthr) {
+      const uint2 t = ptable[u];
+      const float *from = timg + (t.y & ~kOne);
+      if (t.y & kOne)
+        st_word(hw + t.x, from[0], ep);
+      else
+        st_word2(hw + t.x, from[0], from[1], ep);
+    }
+  };
+  // elements of this lane beside the owned columns
+  unsigned need_side = 0u;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int i = g.i0 + q;
+    if (MODE == kHalo && act && ((i < x0 && i >= x0 - KX) || (i >= x1 && i < x1 + KX))) need_side |= 1u << q;
+  }
+  // waits for the words of exchange e and puts them in shared memory; false
+  // if the wait gave up
+  auto receive = [&](int e, int to_edge) -> bool {
+    const unsigned ep = ebase + (unsigned)e;
+    const unsigned long long *const hw = J.halo + ((e & 1) ? pwords : 0u);
+    constexpr int NB = 4;  // pairs of a thread in flight
+    for (int u0 = tid; u0 < npair; u0 += NB * nthr) {
+      uint2 t[NB];
+      unsigned long long w[NB][2];
+#pragma unroll
+      for (int q = 0; q < NB; ++q) t[q] = table[min(u0 + q * nthr, npair - 1)];
+      for (long long it = 0;; ++it) {
+        bool all = true;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) ld_word2(hw + t[q].x, w[q][0], w[q][1]);
+#pragma unroll
+        for (int q = 0; q < NB; ++q)
+          all = all && (unsigned)(w[q][0] >> 32) == ep && ((t[q].y & kOne) || (unsigned)(w[q][1] >> 32) == ep);
+        if (all) break;
+        if (it >= kSpinLimit || ((it & 255) == 255 && *(volatile int *)&ctl->abort)) return false;
+      }
+#pragma unroll
+      for (int q = 0; q < NB; ++q) {
+        float *to = (t[q].y & kEdge) ? edge + to_edge * 256 : timg;
+        to += t[q].y & ~(kEdge | kOne);
+        to[0] = __uint_as_float((unsigned)w[q][0]);
+        if (!(t[q].y & kOne)) to[1] = __uint_as_float((unsigned)w[q][1]);
+      }
+    }
+    return true;
+  };
+  // this thread's halo nodes from shared memory
+  auto take = [&]() {
+    const float *const q = timg + (g.row0 - lo) * 128 + 4 * li;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (r >= g.nvalid) continue;
+      if (!((g.ownrows >> r) & 1u)) {
+        x[r] = lds4(q + r * 128);
+      } else if (MODE == kHalo && need_side) {
+        const float4 v = lds4(q + r * 128);
+        x[r].x = (need_side & 1u) ? v.x : x[r].x;
+        x[r].y = (need_side & 2u) ? v.y : x[r].y;
+        x[r].z = (need_side & 4u) ? v.z : x[r].z;
+        x[r].w = (need_side & 8u) ? v.w : x[r].w;
+      }
+    }
+  };
+  auto fail = [&]() {
+    js->bail = 1;
+    if (!*(volatile int *)&ctl->abort) {
+      atomicExch(&ctl->abort, 1);
+      atomicOr(&ctl->step_flags, (uint32_t)CUPIC_FLAG_TIMEOUT);
+    }
+  };
+
+  // ---- sweeps ----------------------------------------------------------
+  // A checked sweep is one that the stop rule looks at; when the solve cannot
+  // stop early only its last sweep is checked, for the report.  Blocks of at
+  // most K sweeps end with an exchange; nq counts the blocks that had
+  // checked sweeps, whose maxima use slot nq & 3.
+  const bool report = J.write_stats || J.tol > 0.0;
+  const bool early = J.tol > 0.0 && J.min_sweeps < J.max_sweeps;
+  bool checks = report;  // cleared while a stopped solve sweeps up to its last sweep
+  const int KB = G > 1 ? K : kSoloBlock;
+  int maxs = J.max_sweeps, p = 0, es = 0, done = 0, e = 0, nq = 0;
+  float resv = INFINITY;
+  bool pend = false;  // the decision on block nq-1 is outstanding
+  int pstart = 0, pes = 0;
+  unsigned pmask = 0u;
+  // the stop decision on checked block q, taken by warp 0 once every CTA's
+  // maxima are in (usually long before it asks)
+  auto decide = [&](int q, unsigned mask) {
+    bool ok = true;
+    const unsigned target = (unsigned)G * ((unsigned)q / 4u + 1u);
+    if (lane == 0)
+      for (long long it = 0; ld_acquire(&J.tbar[q & 3]) < target; ++it)
+        if (it >= kSpinLimit || ((it & 255) == 255 && *(volatile int *)&ctl->abort)) {
+          ok = false;
+          break;
+        }
+    ok = __shfl_sync(kFull, ok, 0);
+    const bool mineck = (mask >> lane) & 1u;
+    const float v = mineck ? __uint_as_float((unsigned)ld_word(&J.gmax[(q & 3) * 32 + lane])) : 0.0f;
+    const unsigned pass = __ballot_sync(kFull, mineck && (double)v < J.tol && !J.trial);
+    const int k = pass ? __ffs(pass) - 1 : 31 - __clz(mask);
+    const float vk = __shfl_sync(kFull, v, k);
+    if (lane == 0) {
+      js->dec[q & 1] = pass ? k : -1;
+      js->decv[q & 1] = vk;
+      if (!ok) fail();
+    }
+  };
+  auto stop_at = [&](int start, int k, int slot, int es_) {
+    // back to the start of the block, then up to its sweep k
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[r] = snap[(slot * R + r) * nthr + tid];
+    es = es_;
+    done = start;
+    maxs = start + k + 1;
+    checks = false;
+    sts4(first + p * par + mine, x[0]);
+    sts4(last + p * par + mine, x[R - 1]);
+    __syncthreads();
+  };
+  for (int k = tid; k < 128; k += nthr) js->cm[k >> 5][k & 31] = 0u;
+  __syncthreads();
+  for (;;) {
+    if (done >= maxs) {
+      if (!pend) break;
+      if (warp == 0) decide(nq - 1, pmask);
+      __syncthreads();
+      pend = false;
+      if (js->bail) break;
+      resv = js->decv[(nq - 1) & 1];
+      const int k = js->dec[(nq - 1) & 1];
+      if (k < 0) break;
+      stop_at(pstart, k, (nq - 1) & 1, pes);
+    }
+    const int nsw = min(KB, maxs - done), start = done, es0 = es;
+    unsigned mask = 0u, keep = 0u;
+    if (checks) {
+      if (early)
+        for (int s = (start / J.check_every + 1) * J.check_every; s <= start + nsw; s += J.check_every)
+          if (s >= J.min_sweeps) mask |= 1u << (s - start - 1);
+      if (start + nsw == J.max_sweeps) mask |= 1u << (nsw - 1);
+      if (mask && early) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) snap[((nq & 1) * R + r) * nthr + tid] = x[r];
+      }
+    }
+    // smem places of the rows below and above the strip (read) and of its
+    // first and last rows (written), this sweep's (A) and the next one's (B)
+    const float *sA = south_edge ? edge + es * 256 + 4 * li : last + p * par + soff;
+    const float *nA = north_edge || idle ? edge + es * 256 + 128 + 4 * li : first + p * par + noff;
+    const float *sB = south_edge ? sA : last + (p ^ 1) * par + soff;
+    const float *nB = north_edge || idle ? nA : first + (p ^ 1) * par + noff;
+    float *wA = first + p * par + mine, *wB = first + (p ^ 1) * par + mine;
+    const int tolast = 2 * par;
+    // the rest of a sweep: the strip's first and last rows to shared memory
+    auto next = [&]() {
+      sts4(wB, x[0]);
+      sts4(wB + tolast, x[R - 1]);
+      const float *t = sA;
+      sA = sB;
+      sB = t;
+      t = nA;
+      nA = nB;
+      nB = t;
+      float *w = wA;
+      wA = wB;
+      wB = w;
+      __syncthreads();
+    };
+    auto note = [&](float md, int m) {
+      const unsigned u = __reduce_max_sync(kFull, __float_as_uint(md));
+      if (lane == m) keep = u;
+    };
+    int m = 0;
+    if (start == 0) {
+      note(sweep<R, MODE, false, true, true>(x, b, lds4(sA), lds4(nA), g, J.phi_zero ? nullptr : phi + W, nnx), 0);
+      next();
+      m = 1;
+    }
+    const int plain = mask >> m ? m + __ffs(mask >> m) - 1 : nsw;  // sweeps before the next checked one
+    if (g.full) {
+#pragma unroll 2
+      for (; m < plain; ++m) {
+        sweep<R, MODE, true, false, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0);
+        next();
+      }
+#pragma unroll 1
+      for (; m < nsw; ++m) {
+        note(sweep<R, MODE, true, true, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0), m);
+        next();
+      }
+    } else {
+#pragma unroll 2
+      for (; m < plain; ++m) {
+        sweep<R, MODE, false, false, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0);
+        next();
+      }
+#pragma unroll 1
+      for (; m < nsw; ++m) {
+        note(sweep<R, MODE, false, true, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0), m);
+        next();
+      }
+    }
+    p ^= nsw & 1;
+    done += nsw;
+    if ((mask >> lane) & 1u) atomicMax(&js->cm[nq & 3][lane], keep);
+    // the last exchange serves the field; a solve of less than K sweeps
+    // trades once too, so that no CTA stores its rows before its neighbours
+    // have loaded them
+    const bool trade = G > 1 && ((nsw == K && (done < maxs || J.do_field)) || (done >= maxs && e == 0));
+    if (trade) {
+      ++e;
+      show();
+      __syncthreads();
+      publish(e);
+      es = (es + 1) & 3;
+      if (!receive(e, es)) fail();
+    }
+    if (pend && warp == 0) decide(nq - 1, pmask);
+    __syncthreads();
+    if (trade) {
+      take();
+      p ^= 1;
+      sts4(first + p * par + mine, x[0]);
+      sts4(last + p * par + mine, x[R - 1]);
+      __syncthreads();
+    }
+    if (js->bail) break;
+    if (pend) {
+      pend = false;
+      const int k = js->dec[(nq - 1) & 1];
+      if (k >= 0) {
+        resv = js->decv[(nq - 1) & 1];
+        stop_at(pstart, k, (nq - 1) & 1, pes);
+        continue;
+      }
+    }
+    if (mask) {
+      if (G == 1) {
+        const float v = __uint_as_float(js->cm[nq & 3][lane]);
+        const unsigned pass = __ballot_sync(kFull, early && ((mask >> lane) & 1u) && (double)v < J.tol && !J.trial);
+        const int k = pass ? __ffs(pass) - 1 : 31 - __clz(mask);
+        resv = __shfl_sync(kFull, v, k);
+        if (warp == 0) js->cm[(nq + 2) & 3][lane] = 0u;
+        ++nq;
+        if (pass) stop_at(start, k, (nq - 1) & 1, es0);
+      } else {
+        if (warp == 0) {
+          if ((mask >> lane) & 1u)
+            atomicMax(&J.gmax[(nq & 3) * 32 + lane],
+                      ((unsigned long long)(ebase + (unsigned)nq + 1u) << 32) | js->cm[nq & 3][lane]);
+          js->cm[(nq + 2) & 3][lane] = 0u;
+          __threadfence();
+          __syncwarp();
+          if (lane == 0) atomicAdd(&J.tbar[nq & 3], 1u);
+        }
+        pend = early;
+        pstart = start;
+        pes = es0;
+        pmask = mask;
+        ++nq;
+      }
+    }
+  }
+
+  // ---- results ---------------------------------------------------------
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (!((g.ownrows >> r) & 1u)) continue;
+    float *const q = phi + (size_t)(g.row0 + r) * nnx + g.i0;
+    if (g.own & 1u) q[0] = x[r].x;
+    if (g.own & 2u) q[1] = x[r].y;
+    if (g.own & 4u) q[2] = x[r].z;
+    if (g.own & 8u) q[3] = x[r].w;
+    if (g.i0 == 0 && (g.own & 1u)) q[W] = x[r].x;
+  }
+  if (J.do_field) {  // E = -grad phi (mesh.cu:413-468)
+    const float4 s4 = lds4(south_edge ? edge + es * 256 + 4 * li : last + p * par + soff);
+    const float4 n4 = lds4(north_edge || idle ? edge + es * 256 + 128 + 4 * li : first + p * par + noff);
+    float4 prev = s4;
+    auto put = [&](int j, int q, float wv, float ev, float nv, float sv) {
+      if ((g.own >> q) & 1u)
+        a.E[(size_t)j * nnx + g.i0 + q] =
+            make_float2(__fdiv_rn(__fsub_rn(wv, ev), a.two_ds), __fdiv_rn(__fsub_rn(sv, nv), a.two_ds));
+    };
+    auto rim = [&](int j, const float4 &hi_, const float4 &lo_, float mhi, float mlo) {  // a Dirichlet row
+      float2 *const q = a.E + (size_t)j * nnx + g.i0;
+      if (g.own & 1u) q[0] = make_float2(0.0f, __fdiv_rn(__fsub_rn(hi_.x, lo_.x), a.ds));
+      if (g.own & 2u) q[1] = make_float2(0.0f, __fdiv_rn(__fsub_rn(hi_.y, lo_.y), a.ds));
+      if (g.own & 4u) q[2] = make_float2(0.0f, __fdiv_rn(__fsub_rn(hi_.z, lo_.z), a.ds));
+      if (g.own & 8u) q[3] = make_float2(0.0f, __fdiv_rn(__fsub_rn(hi_.w, lo_.w), a.ds));
+      if (g.i0 == 0 && (g.own & 1u)) q[W] = make_float2(0.0f, __fdiv_rn(__fsub_rn(mhi, mlo), a.ds));
+    };
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float4 c = x[r];
+      float lf, rt;
+      float4 ev = make_float4(c.y, c.z, c.w, 0.0f);
+      if (MODE == kHalo) {
+        lf = __shfl_up_sync(kFull, c.w, 1);
+        rt = __shfl_down_sync(kFull, c.x, 1);
+      } else {
+        const float lastv = g.rm == 0 ? c.w : (g.rm == 1 ? c.x : (g.rm == 2 ? c.y : c.z));
+        lf = __shfl_sync(kFull, lastv, g.srcw);
+        rt = __shfl_sync(kFull, c.x, g.srce);
+        ev.x = g.rm == 1 ? rt : ev.x;
+        ev.y = g.rm == 2 ? rt : ev.y;
+        ev.z = g.rm == 3 ? rt : ev.z;
+      }
+      ev.w = rt;
+      const float4 nx = r + 1 < R ? x[r + 1 < R ? r + 1 : r] : n4;
+      const float4 n = r + 1 >= g.nvalid ? n4 : nx;
+      if ((g.ownrows >> r) & 1u) {
+        const int j = g.row0 + r;
+        put(j, 0, lf, ev.x, n.x, prev.x);
+        put(j, 1, c.x, ev.y, n.y, prev.y);
+        put(j, 2, c.y, ev.z, n.z, prev.z);
+        put(j, 3, c.z, ev.w, n.w, prev.w);
+        const bool col0 = g.i0 == 0 && (g.own & 1u);
+        if (col0) {  // the mirror column; the Dirichlet rows keep their own value there
+          const float sv = j == 1 ? phi[W] : prev.x, nv = j == nny - 2 ? phi[(size_t)(nny - 1) * nnx + W] : n.x;
+          a.E[(size_t)j * nnx + W] =
+              make_float2(__fdiv_rn(__fsub_rn(lf, ev.x), a.two_ds), __fdiv_rn(__fsub_rn(sv, nv), a.two_ds));
+        }
+        if (j == 1) rim(0, prev, c, col0 ? phi[W] : 0.0f, c.x);
+        if (j == nny - 2) rim(nny - 1, c, n, c.x, col0 ? phi[(size_t)(nny - 1) * nnx + W] : 0.0f);
+      }
+      prev = c;
+    }
+  }
+  // the last CTA to finish writes the report, puts the counters back to zero
+  // and advances the epochs past this solve's
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(&ctl->jdone, 1u) == (unsigned)G - 1u) {
+      __threadfence();
+      ctl->jdone = 0u;
+      if (J.write_stats) {
+        ctl->sweeps = done;
+        ctl->residual = G > 1 && report && !early && nq > 0
+                            ? __uint_as_float((unsigned)ld_word(&J.gmax[((nq - 1) & 3) * 32 + ((J.max_sweeps - 1) % KB)]))
+                            : resv;
+      }
+      unsigned next = ebase + (unsigned)max(e, nq) + 2u;
+      const bool wrap = next > kEpochEnd;  // start over, above the tags left in gmax
+      if (wrap) next = 0u;
+      if (G > 1) {
+        for (int k = 0; k < 4; ++k) J.tbar[k] = 0u;
+        if (wrap)
+          for (int k = 0; k < 128; ++k) J.gmax[k] = 0ull;
+      }
+      ctl->jepoch = next;
+    }
+  }
+}
+
+template <int R, int MODE>
+__global__ void __launch_bounds__(512, 1) k_tile(SimArgs a, JacobiArgs J) {
+  extern __shared__ __align__(16) float tsm[];
+  __shared__ Scratch js;
+  if (threadIdx.x == 0) js.bail = 0;
+  __syncthreads();
+  solve<R, MODE>(a, J, blockIdx.x, tsm, &js);
+}
+
+using Kernel = void (*)(SimArgs, JacobiArgs);
+
+// the kernel of MODE with strips of r rows (1..8)
+template <int MODE>
+inline Kernel pick(int r) {
+  switch (r) {
+    case 1: return k_tile<1, MODE>;
+    case 2: return k_tile<2, MODE>;
+    case 3: return k_tile<3, MODE>;
+    case 4: return k_tile<4, MODE>;
+    case 5: return k_tile<5, MODE>;
+    case 6: return k_tile<6, MODE>;
+    case 7: return k_tile<7, MODE>;
+    default: return k_tile<8, MODE>;
+  }
+}
+
+}  // namespace tile
+}  // namespace cupic
