@@ -538,7 +538,7 @@ struct TileKey {
   }
 };
 std::map<TileKey, TilePlan> g_tiles;
-constexpr int kTileTrials = 16;
+constexpr int kTileTrials = 24;
 
 int tune_tiles(cupic_ctx *c, int dev_max) {
   const int chk = std::max(1, c->p.check_every);

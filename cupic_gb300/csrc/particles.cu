@@ -19,6 +19,7 @@
 #include <utility>
 
 #include "cupic_internal.cuh"
+#include "draws.cuh"
 #include "kernels.h"
 
 namespace cupic {
@@ -210,20 +211,40 @@ __device__ __forceinline__ int settle(const SimArgs &a, const float4 &v, int s, 
 // ---------------------------------------------------------------------------
 // initial plasma (init.cu:159-179, with the project's counter-based draws)
 // ---------------------------------------------------------------------------
-__global__ void k_init_particles(SimArgs a) {
+// the definition, in FP64
+__device__ __noinline__ float4 init_particle_f64(const SimArgs &a, const uint4 r, int j, double sig) {
+  const double x = u01(r.x) * a.Lx_d;
+  const double y = ((double)j + u01(r.y)) * a.ds_d;
+  const double rr = sqrt(-2.0 * dev_log(u01(r.z)));
+  double sn, cs;
+  dev_sincos2pi(u01(r.w), &sn, &cs);
+  return make_float4((float)x, (float)y, (float)(sig * (rr * cs)), (float)(sig * (rr * sn)));
+}
+
+// the same four floats (draws.cuh)
+__device__ __forceinline__ float4 init_particle(const SimArgs &a, const uint4 r, int j, double sig, df lx,
+                                                df ds, df sigf) {
+  bool ok = j < 32768;  // df_int takes 48 bits
+  const df ux = df_scale(df_int(2ull * r.x + 1ull), 0x1p-33f);
+  const df uy = df_scale(df_int(((unsigned long long)(unsigned)j << 33) + 2ull * r.y + 1ull), 0x1p-33f);
+  df sn, cs;
+  df_sincos2pi_u01(r.w, &sn, &cs);
+  const df rr = df_mul(df_sqrt(df_scale(df_log_u01(r.z), -2.0f)), sigf);
+  const float4 p = make_float4(df_round(df_mul(ux, lx), ok), df_round(df_mul(uy, ds), ok),
+                               df_round(df_mul(rr, cs), ok), df_round(df_mul(rr, sn), ok));
+  return ok ? p : init_particle_f64(a, r, j, sig);
+}
+
+__global__ void __launch_bounds__(256) k_init_particles(SimArgs a) {
   const int j = blockIdx.x, sp = blockIdx.y;
   const SpeciesDev &S = a.sp[sp];
   float4 *row = S.parts + S.seg[j];
   const double sig = a.sig[sp];
+  const df lx = df_of(a.Lx_d), ds = df_of(a.ds_d), sigf = df_of(sig);
   for (int k = threadIdx.x; k < a.ppr; k += blockDim.x) {
     const uint4 r = philox4x32_10(
         make_uint4((uint32_t)k, (uint32_t)j, 0u, (uint32_t)((kPurposeInit << 8) | sp)), a.k0, a.k1);
-    const double x = u01(r.x) * a.Lx_d;
-    const double y = ((double)j + u01(r.y)) * a.ds_d;
-    const double rr = sqrt(-2.0 * dev_log(u01(r.z)));
-    double sn, cs;
-    dev_sincos2pi(u01(r.w), &sn, &cs);
-    float4 p = make_float4((float)x, (float)y, (float)(sig * (rr * cs)), (float)(sig * (rr * sn)));
+    float4 p = init_particle(a, r, j, sig, lx, ds, sigf);
     p.x = wrap_x(a, p.x);
     for (int it = 0; it < 16 && row_of(a, p.y) > j; ++it) p.y = nextafterf(p.y, 0.0f);
     for (int it = 0; it < 16 && row_of(a, p.y) < j; ++it) p.y = nextafterf(p.y, a.Ly);
