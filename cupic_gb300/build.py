@@ -19,7 +19,7 @@ LIB = os.path.join(OUT, "libcupic_gpu.so")
 EXE = os.path.join(OUT, "cupic_run")
 REF_LIB = os.path.join(OUT, "libcupic_ref.so")
 SOURCES = ["capi.cu", "particles.cu", "jacobi.cu", "tile.cu", "tile_halo.cu", "tile_ring.cu",
-           "tile_ragged.cu", "io.cu", "noalloc.cu", "refine.cu", "batch.cu",
+           "tile_ragged.cu", "tile_halo_refine.cu", "tile_ring_refine.cu", "tile_ragged_refine.cu", "io.cu", "noalloc.cu", "refine.cu", "batch.cu",
            "files.cpp"]
 MAIN = "cupic_main.cpp"
 REF_API = "ref_api.cpp"

@@ -269,6 +269,7 @@ void fill_constants(cupic_ctx *c) {
 }
 
 JacobiArgs jargs(const cupic_ctx *c, double tol, int mn, int mx, int chk, int field);
+void refine_args(const cupic_ctx *c, JacobiArgs *J, double tol, int mn, int mx, int write_stats);
 
 // ---- Jacobi layout -------------------------------------------------------
 // G CTAs of 512 threads, each holding its B mesh rows plus K halo rows on
@@ -368,9 +369,12 @@ int set_tile_plan(cupic_ctx *c, const TilePlan &t) {
   return alloc_jacobi_scratch(c, t.G, t.words);
 }
 
+// a context's solves may all stop on a tolerance given by the call
+TileForm tile_form(const cupic_ctx *c) { return c->p.refine_every > 0 ? kTileRefine : kTileEarly; }
+
 // whether the context's solves may run as register tiles
 bool tiles_apply(const cupic_ctx *c) {
-  return c->p.refine_every == 0 && !getenv("CUPIC_JACOBI_NOSTRIP") && !getenv("CUPIC_JACOBI_SCALAR");
+  return !c->no_tiles && !getenv("CUPIC_JACOBI_NOSTRIP") && !getenv("CUPIC_JACOBI_SCALAR");
 }
 
 // The fixed rule, used when tuning is off or a layout is forced with
@@ -411,7 +415,7 @@ int plan_jacobi_rule(cupic_ctx *c, int P, long long rows_fit) {
   if (tiles_apply(c))
     for (int nbx = 1; nbx <= G; ++nbx) {
       TilePlan t;
-      if (G % nbx == 0 && tile_plan(c->a.nnx, c->a.nny, nbx, G / nbx, K, 0, true, &t) &&
+      if (G % nbx == 0 && tile_plan(c->a.nnx, c->a.nny, nbx, G / nbx, K, 0, tile_form(c), &t) &&
           set_tile_plan(c, t) == CUPIC_OK)
         return CUPIC_OK;
     }
@@ -531,10 +535,10 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
 // fastest is kept, per device, mesh shape and check interval.  Returns
 // CUPIC_ERR_CAPACITY when no layout holds the mesh.
 struct TileKey {
-  int device, nnx, nny, chk, sweeps, early;
+  int device, nnx, nny, chk, sweeps, early, refine;
   bool operator<(const TileKey &o) const {
-    return std::tie(device, nnx, nny, chk, sweeps, early) <
-           std::tie(o.device, o.nnx, o.nny, o.chk, o.sweeps, o.early);
+    return std::tie(device, nnx, nny, chk, sweeps, early, refine) <
+           std::tie(o.device, o.nnx, o.nny, o.chk, o.sweeps, o.early, o.refine);
   }
 };
 std::map<TileKey, TilePlan> g_tiles;
@@ -544,13 +548,14 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
   const int chk = std::max(1, c->p.check_every);
   const int S = std::max(1, std::min(std::max(c->p.max_sweeps, c->p.init_max_sweeps), 256));
   const int early = c->p.tol > 0.0 && c->p.min_sweeps < c->p.max_sweeps;
-  const TileKey key{c->device, c->a.nnx, c->a.nny, chk, S, early};
+  const int m = c->p.refine_every;
+  const TileKey key{c->device, c->a.nnx, c->a.nny, chk, S, early, m};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tiles.find(key);
     if (it != g_tiles.end()) return set_tile_plan(c, it->second);
   }
-  const std::vector<TilePlan> all = tile_plans(c->a.nnx, c->a.nny, c->num_sms, true, (size_t)dev_max - 1024);
+  const std::vector<TilePlan> all = tile_plans(c->a.nnx, c->a.nny, c->num_sms, tile_form(c), (size_t)dev_max - 1024);
   std::vector<TilePlan> cands;
   size_t words = 0;
   int maxG = 1;
@@ -574,9 +579,11 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
     CU(cudaEventCreate(&e0));
     CU(cudaEventCreate(&e1));
     float best = 1e30f;
+    if (m > 0) CU(cudaMemsetAsync(c->b64, 0, sizeof(double) * (size_t)c->a.nnx * c->a.nny, c->stream));
     for (const TilePlan &t : cands) {
       c->tile = t;
       JacobiArgs J = jargs(c, early ? 1.0 : 0.0, early ? 1 : S, S, chk, 1);
+      if (m > 0) refine_args(c, &J, 0.0, 0, std::min(S, 4 * m), 0);
       J.trial = 1;
       float ms_best = 1e30f;
       bool ok = true;
@@ -651,6 +658,18 @@ JacobiArgs jargs(const cupic_ctx *c, double tol, int mn, int mx, int chk, int fi
   return J;
 }
 
+// the precision form's solve as one launch of register tiles
+void refine_args(const cupic_ctx *c, JacobiArgs *J, double tol, int mn, int mx, int write_stats) {
+  J->max_sweeps = c->p.refine_every;
+  J->write_stats = 0;
+  J->r64_phi = c->phi64;
+  J->r64_b = c->b64;
+  J->r64_tol = tol;
+  J->r64_mn = mn;
+  J->r64_mx = mx;
+  J->r64_stats = write_stats;
+}
+
 // one solve with the context's layout
 cudaError_t launch_solve(const cupic_ctx *c, const JacobiArgs &J) {
   if (J.max_sweeps < 1 && !J.r64_phi && !J.phi) return launch_field(c->a, J.do_field, J.write_stats, c->stream);
@@ -663,7 +682,20 @@ int set_phi_both(cupic_ctx *c, const double *phi) {
   std::vector<float> h(n);
   for (size_t k = 0; k < n; ++k) h[k] = (float)phi[k];
   CU(cudaMemcpy(c->a.phi, h.data(), n * sizeof(float), cudaMemcpyHostToDevice));
-  if (c->phi64) CU(cudaMemcpy(c->phi64, phi, n * sizeof(double), cudaMemcpyHostToDevice));
+  if (c->phi64) {
+    CU(cudaMemcpy(c->phi64, phi, n * sizeof(double), cudaMemcpyHostToDevice));
+    // the precision form's tiles take column 0 for its mirror, column nnx-1,
+    // whose FP64 value otherwise keeps its own start: a potential with two
+    // different columns there is solved by the launches that read both
+    const int nnx = c->a.nnx;
+    bool same = true;
+    for (int j = 0; j < c->a.nny; ++j) same = same && phi[(size_t)j * nnx] == phi[(size_t)j * nnx + nnx - 1];
+    if (!same && c->tile.R) {
+      c->no_tiles = true;
+      destroy_graph(c);
+      return plan_jacobi(c);
+    }
+  }
   return CUPIC_OK;
 }
 
@@ -759,23 +791,39 @@ int refine_solve_device(cupic_ctx *c, double tol, int mn, int mx, int field, int
   return CUPIC_OK;
 }
 
+// The same solve in one launch of register tiles: the source, then every
+// correction, the FP32 potential and the field in k_tile.
+int refine_solve_tiles(cupic_ctx *c, double tol, int mn, int mx, int field, int write_stats, int zero_next) {
+  CU(launch_r64_source(c->a, c->b64, c->stream));
+  JacobiArgs J = jargs(c, 0.0, 0, 0, 1, field);
+  refine_args(c, &J, tol, mn, mx, write_stats);
+  J.zero_next = zero_next;
+  CU(launch_tile(c->a, J, c->tile, c->stream));
+  return CUPIC_OK;
+}
+
 // the solve of a step or stage call, FP32 or in the precision form
 int run_solve(cupic_ctx *c, double tol, int mn, int mx, int chk, int field, int write_stats = 1) {
-  if (c->p.refine_every > 0)
+  if (c->p.refine_every > 0) {
+    if (c->tile.R) return refine_solve_tiles(c, tol, mn, mx, field, write_stats, 0);
     return refine_on_device(c, mx) ? refine_solve_device(c, tol, mn, mx, field, write_stats)
                                    : refine_solve(c, tol, mn, mx, field, write_stats);
+  }
   JacobiArgs J = jargs(c, tol, mn, mx, chk, field);
   J.write_stats = write_stats;
   CU(launch_solve(c, J));
   return CUPIC_OK;
 }
 
-// a step's solve, which also clears the next charge accumulator (the
-// precision form's solve does not: the step clears it separately)
+// a step's solve, which also clears the next charge accumulator (that of
+// refine_solve_device and refine_solve does not: the step clears it separately)
 int run_step_solve(cupic_ctx *c, bool *zeroed) {
   const cupic_params &p = c->p;
   *zeroed = false;
-  if (p.refine_every > 0) return run_solve(c, p.tol, p.min_sweeps, p.max_sweeps, p.check_every, 1);
+  if (p.refine_every > 0 && !c->tile.R)
+    return run_solve(c, p.tol, p.min_sweeps, p.max_sweeps, p.check_every, 1);
+  *zeroed = true;
+  if (p.refine_every > 0) return refine_solve_tiles(c, p.tol, p.min_sweeps, p.max_sweeps, 1, 1, 1);
   JacobiArgs J = jargs(c, p.tol, p.min_sweeps, p.max_sweeps, p.check_every, 1);
   J.zero_next = p.max_sweeps > 0;
   CU(launch_solve(c, J));
@@ -1649,7 +1697,7 @@ int cupic_step(cupic_ctx *c, int32_t nsteps) {
     int rc = deposit_current(c);
     if (rc) return rc;
   }
-  if (c->p.refine_every > 0 && !refine_on_device(c, c->p.max_sweeps)) {
+  if (c->p.refine_every > 0 && !c->tile.R && !refine_on_device(c, c->p.max_sweeps)) {
     // the solve reads its residual norm on the host: no graph, and a step
     // that runs out of room is completed before the next one starts
     for (int i = 0; i < nsteps; ++i) {

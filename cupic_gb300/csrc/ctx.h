@@ -28,6 +28,7 @@ struct cupic_ctx {
   // Jacobi geometry and exchange buffers
   int jG = 1, jB = 1, jK = 1, jP = 0;
   cupic::TilePlan tile{};  // register-tile layout (R == 0: the shared-memory sweep of jacobi.cu)
+  bool no_tiles = false;     // the precision form's potential needs the launches of jacobi.cu
   unsigned long long *jgmax = nullptr;  // [128] maxima of checked sweeps, then [4] counters; zeroed
   bool jNoStrip = false;  // the tuner found the shared-memory sweep faster than register strips
   unsigned *jflags = nullptr;  // [G+1]: per-CTA sweep counters, then the barrier

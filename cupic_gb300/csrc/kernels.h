@@ -55,7 +55,11 @@ cudaError_t launch_jacobi(const SimArgs &a, const JacobiArgs &J, cudaStream_t st
 // the register-tile solve (tile.cuh, tile.cu)
 constexpr int kTileWarps = 16;  // most warps of a CTA
 constexpr int kTileDepth = 16;  // deepest halo
+// a solve of a fixed number of sweeps, one that may stop on its tolerance
+// (and keeps snapshots), the precision form (and keeps its FP64 potential)
+enum TileForm { kTileFixed, kTileEarly, kTileRefine };
 struct TilePlan {
+  TileForm form;
   int R;                   // rows of a strip
   int mode;                // 0 halo, 1 ring, 2 ragged ring
   int nbx, nby, G, K;      // blocks in x and y, their product, halo depth
@@ -65,9 +69,8 @@ struct TilePlan {
   size_t smem, words;      // dynamic shared memory; exchange words
   double cost;             // estimated SM cycles per sweep
 };
-// early: the solve may stop on its tolerance (and then keeps snapshots)
-bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, bool early, TilePlan *out);
-std::vector<TilePlan> tile_plans(int nnx, int nny, int max_ctas, bool early, size_t max_smem);
+bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, TilePlan *out);
+std::vector<TilePlan> tile_plans(int nnx, int nny, int max_ctas, TileForm form, size_t max_smem);
 void tile_args(const TilePlan &t, JacobiArgs *J);
 cudaError_t tile_max_ctas(const TilePlan &t, int num_sms, int *ctas);
 cudaError_t launch_tile(const SimArgs &a, const JacobiArgs &J, const TilePlan &t, cudaStream_t st);

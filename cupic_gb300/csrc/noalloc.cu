@@ -78,14 +78,14 @@ size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 // The register tiles of a mesh: the layout of least estimated cost whose
 // words fit the scratch, on at most max_ctas CTAs; R == 0 when there is none.
 // Layouts depend only on the mesh and the device, and are kept.
-TilePlan tiles_for(int dev, int num_sms, int dev_max, int nnx, int nny, int max_ctas, bool early) {
-  static std::map<std::tuple<int, int, int, int, bool>, TilePlan> kept;
+TilePlan tiles_for(int dev, int num_sms, int dev_max, int nnx, int nny, int max_ctas, TileForm form) {
+  static std::map<std::tuple<int, int, int, int, TileForm>, TilePlan> kept;
   std::lock_guard<std::mutex> lock(g_mu);
-  const auto key = std::make_tuple(dev, nnx, nny, max_ctas, early);
+  const auto key = std::make_tuple(dev, nnx, nny, max_ctas, form);
   const auto it = kept.find(key);
   if (it != kept.end()) return it->second;
   TilePlan pick{};
-  for (const TilePlan &t : tile_plans(nnx, nny, max_ctas, early, (size_t)dev_max - 1024)) {
+  for (const TilePlan &t : tile_plans(nnx, nny, max_ctas, form, (size_t)dev_max - 1024)) {
     int n = 0;
     if (kCtlHeadBytes + sizeof(unsigned long long) * t.words > kStaticScratchBytes || t.G > max_ctas) continue;
     if (tile_max_ctas(t, num_sms, &n) != cudaSuccess) {
@@ -207,9 +207,9 @@ extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t 
   J.gmax = sync;
   J.tbar = reinterpret_cast<unsigned *>(sync + 128);
   // the mesh is one that the scratch holds; most run faster as register tiles
-  const bool early = max_error > 0.0 && min_sweeps < max_sweeps;
+  const TileForm form = max_error > 0.0 && min_sweeps < max_sweeps ? kTileEarly : kTileFixed;
   const TilePlan tile = max_sweeps > 0 ? tiles_for(dev, num_sms, dev_max, a.nnx, a.nny,
-                                                   std::min(forced > 0 ? forced : num_sms, num_sms), early)
+                                                   std::min(forced > 0 ? forced : num_sms, num_sms), form)
                                        : TilePlan{};
   if (tile.R) {
     tile_args(tile, &J);

@@ -10,10 +10,17 @@ namespace cupic {
 const void *tile_kernel_halo(int r);
 const void *tile_kernel_ring(int r);
 const void *tile_kernel_ragged(int r);
+const void *tile_kernel_halo_refine(int r);
+const void *tile_kernel_ring_refine(int r);
+const void *tile_kernel_ragged_refine(int r);
 
 namespace {
 
 const void *tile_kernel(const TilePlan &t) {
+  if (t.form == kTileRefine)
+    return t.mode == 0   ? tile_kernel_halo_refine(t.R)
+           : t.mode == 1 ? tile_kernel_ring_refine(t.R)
+                         : tile_kernel_ragged_refine(t.R);
   return t.mode == 0 ? tile_kernel_halo(t.R) : t.mode == 1 ? tile_kernel_ring(t.R) : tile_kernel_ragged(t.R);
 }
 
@@ -47,9 +54,10 @@ __global__ void k_field(SimArgs a, int do_field, int write_stats) {
 
 // The layout of nbx x nby blocks with halo depth K and strips of R rows (0:
 // the smallest that needs at most kTileWarps warps); false if there is none.
-bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, bool early, TilePlan *out) {
+bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, TilePlan *out) {
   const int W = nnx - 1, M = nny - 2, W4 = (W + 3) / 4;
   TilePlan t{};
+  t.form = form;
   if (nbx < 1 || nby < 1 || K < 1 || nby > M || nbx > W4 || K > kTileDepth) return false;
   if (nby > 1 && K > M / nby) return false;  // a block trades K of its own rows
   if (nbx == 1) {
@@ -100,9 +108,10 @@ bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, bool early, Til
   }
   // strip rows in two parities, edge rows, the exchange image and its tables
   // (even numbers of entries: what follows is 16-byte aligned), two
-  // snapshots of the strips
+  // snapshots of the strips or the FP64 potential
   t.smem = (4 * thr * 4 + 4 * 2 * 128 + (size_t)t.trows * 128) * sizeof(float) +
-           (size_t)(t.tpairs + t.ppairs) * sizeof(uint2) + (early ? 2 * R * thr * sizeof(float4) : 0);
+           (size_t)(t.tpairs + t.ppairs) * sizeof(uint2) + (form == kTileEarly ? 2 * R * thr * sizeof(float4) : 0) +
+           (form == kTileRefine ? ((size_t)(rows + 2) * 128 + 8) * sizeof(double) : 0);
   t.words = t.G == 1 ? 0
                      : (size_t)2 * nby * 2 * K * t.ip + (nbx > 1 ? (size_t)2 * nny * nbx * 2 * K : 0);
   if (t.words >= 1ull << 31) return false;
@@ -115,12 +124,15 @@ bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, bool early, Til
   const double rows_cost = t.R <= 5 ? 18.0 * t.R : 18.0 * t.R * (1.0 + 0.12 * (t.R - 5));
   t.cost = 270.0 + ((t.warps + 3) / 4) * rows_cost;
   if (t.G > 1) t.cost += (2000.0 + (nbx > 1 ? 2000.0 : 0.0) + 800.0 * t.tpairs / thr) / K;
+  // the precision form's FP64 work: about 9 operations a node at 2 a clock,
+  // once a correction (32 sweeps)
+  if (form == kTileRefine) t.cost += 4.5 * 4 * 32 * R * t.warps / 32;
   *out = t;
   return true;
 }
 
 // The layouts worth timing, cheapest estimate first.
-std::vector<TilePlan> tile_plans(int nnx, int nny, int max_ctas, bool early, size_t max_smem) {
+std::vector<TilePlan> tile_plans(int nnx, int nny, int max_ctas, TileForm form, size_t max_smem) {
   const int W = nnx - 1, M = nny - 2, W4 = (W + 3) / 4;
   std::vector<TilePlan> out;
   const int depths[] = {1, 2, 4, 6, 8, 12, 16};
@@ -132,10 +144,10 @@ std::vector<TilePlan> tile_plans(int nnx, int nny, int max_ctas, bool early, siz
       for (int K : depths) {
         if (nbx * nby == 1 && K > 1) continue;
         TilePlan t;
-        if (!tile_plan(nnx, nny, nbx, nby, K, 0, early, &t)) continue;
+        if (!tile_plan(nnx, nny, nbx, nby, K, 0, form, &t)) continue;
         const int R0 = t.R;
         for (int R = R0; R <= std::min(8, R0 + 2); ++R)
-          if (tile_plan(nnx, nny, nbx, nby, K, R, early, &t) && t.smem <= max_smem) out.push_back(t);
+          if (tile_plan(nnx, nny, nbx, nby, K, R, form, &t) && t.smem <= max_smem) out.push_back(t);
       }
     }
   std::sort(out.begin(), out.end(), [](const TilePlan &a, const TilePlan &b) { return a.cost < b.cost; });

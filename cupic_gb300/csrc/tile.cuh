@@ -83,6 +83,7 @@ struct Scratch {
   int dec[2];          // a block's stop decision: index of the stopping sweep, or -1
   float decv[2];       // its residual
   int bail;
+  unsigned long long w64[16], res64[2];  // a correction's max |r| per warp, and over the grid
 };
 
 // one thread's place in its tile
@@ -100,6 +101,29 @@ struct Lane {
 
 __device__ __forceinline__ float node(float b, float w, float e, float n, float s) {
   return __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(b, w), e), n), s));
+}
+
+// A warp's FP64 operation holds the SM's FP64 pipe for about 24 cycles, so the
+// correction's conversions and its product by 4 go through the integer pipe:
+// the same bits (round to nearest even), with the hardware's conversion for
+// what is not normal on both sides.  A 512x2048 correction: 57.1 -> 55.6 us.
+__device__ __forceinline__ float to_float(double v) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+  const unsigned e = (unsigned)(u >> 52) & 0x7ffu;
+  if (e - 897u >= 254u) return __double2float_rn(v);
+  const unsigned t = (unsigned)(((u & 0x7fffffffffffffffull) + 0x0fffffffull + ((u >> 29) & 1ull)) >> 29);
+  return __uint_as_float((t - (896u << 23)) | ((unsigned)(u >> 32) & 0x80000000u));
+}
+__device__ __forceinline__ double to_double(float v) {
+  const unsigned b = __float_as_uint(v), e = (b >> 23) & 0xffu;
+  if (e - 1u >= 254u) return (b << 1) == 0u ? __hiloint2double((int)b, 0) : (double)v;
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+}
+__device__ __forceinline__ double times4(double v) {
+  const int hi = __double2hiint(v);
+  const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
+  if (e - 1u >= 0x7fcu) return 4.0 * v;
+  return __hiloint2double(hi + 0x200000, __double2loint(v));
 }
 
 // One sweep of a strip: v = 1/4 ((((b + west) + east) + north) + south).
@@ -162,7 +186,7 @@ __device__ __forceinline__ float sweep(float4 (&x)[R], const float4 (&b)[R], con
   return md;
 }
 
-template <int R, int MODE>
+template <int R, int MODE, bool REFINE>
 __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, const int c, float *sm,
                                       Scratch *js) {
   Ctl *ctl = a.ctl;
@@ -248,7 +272,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       x[r] = b[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (r < g.nvalid) {
+      if (!REFINE && r < g.nvalid) {
         const int j = g.row0 + r;
         if (!J.phi_zero) x[r] = make_float4(ldphi(j, c0), ldphi(j, c1), ldphi(j, c2), ldphi(j, c3));
         b[r] = make_float4(ldsrc(j, c0), ldsrc(j, c1), ldsrc(j, c2), ldsrc(j, c3));
@@ -260,10 +284,10 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       for (int q = 0; q < 4; ++q) {
         if (south_edge)
           sts4(edge + (2 * q) * 128 + 4 * li,
-               J.phi_zero ? z : make_float4(ldphi(lo - 1, c0), ldphi(lo - 1, c1), ldphi(lo - 1, c2), ldphi(lo - 1, c3)));
+               REFINE || J.phi_zero ? z : make_float4(ldphi(lo - 1, c0), ldphi(lo - 1, c1), ldphi(lo - 1, c2), ldphi(lo - 1, c3)));
         if (north_edge)
           sts4(edge + (2 * q + 1) * 128 + 4 * li,
-               J.phi_zero ? z : make_float4(ldphi(hi + 1, c0), ldphi(hi + 1, c1), ldphi(hi + 1, c2), ldphi(hi + 1, c3)));
+               REFINE || J.phi_zero ? z : make_float4(ldphi(hi + 1, c0), ldphi(hi + 1, c1), ldphi(hi + 1, c2), ldphi(hi + 1, c3)));
       }
     }
     sts4(first + mine, x[0]);
@@ -454,6 +478,251 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       atomicOr(&ctl->step_flags, (uint32_t)CUPIC_FLAG_TIMEOUT);
     }
   };
+
+  // the last CTA to finish puts the counters back to zero and advances the
+  // epochs past this solve's
+  auto finish = [&](int used) {
+    unsigned next = ebase + (unsigned)used + 2u;
+    const bool wrap = next > kEpochEnd;  // start over, above the tags left in gmax
+    if (wrap) next = 0u;
+    if (G > 1) {
+      for (int k = 0; k < 4; ++k) J.tbar[k] = 0u;
+      for (int k = 0; k < (wrap ? 128 : REFINE ? 4 : 0); ++k) J.gmax[k] = 0ull;
+    }
+    ctl->jepoch = next;
+  };
+
+  // ---- the precision form (refine.cu) -----------------------------------
+  // phi64 of the tile, halo included, stays in shared memory: a correction
+  // forms the FP64 residual of every node as its source, runs its sweeps from
+  // zero, trades once more so that the halo holds the neighbours' correction
+  // too, and adds it.  The residual's maximum goes to the grid while the
+  // sweeps run and is looked at before the correction is added; a solve that
+  // had already passed its test drops it.  Same operations, same order, same
+  // bits as one launch per residual, solve and update.  Bound by the FP64
+  // pipe (27 us of a 512x2048 correction's 55.6: six operations a node of the
+  // tile) and the sweeps with their exchanges; a launch per correction, with
+  // a grid barrier and every residual's potential read again, took 96 us.
+  if constexpr (REFINE) {
+    double *const p64 = reinterpret_cast<double *>(ptable + J.ppairs);  // rows lo-1 .. hi+1, [128]
+    double *const q64 = p64 + (g.row0 - lo + 1) * 128 + 4 * li;         // this strip's first row
+    const int cc[4] = {column(0), column(1), column(2), column(3)};
+    double *const phi64 = J.r64_phi;
+    auto load_row = [&](int j) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        p64[(j - lo + 1) * 128 + 4 * li + q] = cc[q] >= 0 ? phi64[(size_t)j * nnx + cc[q]] : 0.0;
+    };
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (r < g.nvalid) load_row(g.row0 + r);
+    if (!idle && south_edge) load_row(lo - 1);
+    if (!idle && north_edge) load_row(hi + 1);
+    // the columns west and east of this lane's, relative to them
+    const int wc = MODE == kHalo ? (li == 0 ? 0 : -1) : (li == 0 ? W - 1 : -1);
+    const int ring0 = -4 * li;  // column 0 of a ring
+    auto east = [&](const double *p, int q) {
+      if (MODE != kHalo && g.me == q) return p[ring0];
+      return p[q + 1];
+    };
+    const int m_ = J.max_sweeps;  // sweeps of a correction
+    const unsigned long long inf64 = 0x7ff0000000000000ull;
+    int e = 0, es = 0, p = 0, done = 0, q = 0;
+    double res = 0.0;
+    __syncthreads();
+    // the grid's maximum of correction n (warp 0)
+    auto wait_res = [&](int n) {
+      if (lane == 0) {
+        bool ok = true;
+        const unsigned target = (unsigned)G * ((unsigned)n / 4u + 1u);
+        for (long long it = 0; ld_acquire(&J.tbar[n & 3]) < target; ++it)
+          if (it >= kSpinLimit || ((it & 255) == 255 && *(volatile int *)&ctl->abort)) {
+            ok = false;
+            break;
+          }
+        js->res64[n & 1] = ld_word(&J.gmax[n & 3]);
+        if (!ok) fail();
+      }
+    };
+    for (;;) {
+      unsigned long long mx = 0ull;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        b[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < g.nvalid) {
+          const double *const z = q64 + r * 128;
+          const double *const src = J.r64_b + (size_t)(g.row0 + r) * nnx;
+          float v[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const double rr = (cc[k] >= 0 ? src[cc[k]] : 0.0) -
+                              (times4(z[k]) - ((((k == 0 ? z[wc] : z[k - 1]) + east(z, k)) + z[k + 128]) + z[k - 128]));
+            v[k] = to_float(rr);
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(rr) & 0x7fffffffffffffffull;
+            if (((g.own >> k) & 1u) && ((g.ownrows >> r) & 1u) && bits <= inf64 && bits > mx) mx = bits;
+          }
+          b[r] = make_float4(v[0], v[1], v[2], v[3]);
+        }
+        x[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(kFull, mx, o));
+      if (lane == 0) js->w64[warp] = mx;
+      __syncthreads();
+      if (warp == 0) {
+        mx = lane < (nthr >> 5) ? js->w64[lane] : 0ull;
+        for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(kFull, mx, o));
+        if (lane == 0) {
+          if (G > 1) {
+            // slot q+2 was last read before anyone could add to slot q
+            if (c == 0) *(volatile unsigned long long *)&J.gmax[(q + 2) & 3] = 0ull;
+            atomicMax(&J.gmax[q & 3], mx);
+            __threadfence();
+            atomicAdd(&J.tbar[q & 3], 1u);
+          } else {
+            js->res64[q & 1] = mx;
+          }
+        }
+        if (G > 1 && done >= J.r64_mx) wait_res(q);
+      }
+      // the correction starts from zero
+      sts4(first + p * par + mine, x[0]);
+      sts4(last + p * par + mine, x[R - 1]);
+      if (!idle && south_edge) sts4(edge + es * 256 + 4 * li, x[0]);
+      if (!idle && north_edge) sts4(edge + es * 256 + 128 + 4 * li, x[0]);
+      __syncthreads();
+      if (js->bail) break;
+      if (G == 1 || done >= J.r64_mx) {
+        res = __longlong_as_double((long long)js->res64[q & 1]);
+        if (done >= J.r64_mx || (done >= J.r64_mn && res < J.r64_tol && !J.trial)) break;
+      }
+      const int todo = min(m_, J.r64_mx - done);
+      for (int sw = 0; sw < todo;) {
+        const int nsw = G > 1 ? min(K, todo - sw) : todo;
+        const float *sA = south_edge ? edge + es * 256 + 4 * li : last + p * par + soff;
+        const float *nA = north_edge || idle ? edge + es * 256 + 128 + 4 * li : first + p * par + noff;
+        const float *sB = south_edge ? sA : last + (p ^ 1) * par + soff;
+        const float *nB = north_edge || idle ? nA : first + (p ^ 1) * par + noff;
+        float *wA = first + p * par + mine, *wB = first + (p ^ 1) * par + mine;
+        const int tolast = 2 * par;
+        auto next = [&]() {
+          sts4(wB, x[0]);
+          sts4(wB + tolast, x[R - 1]);
+          const float *t = sA;
+          sA = sB;
+          sB = t;
+          t = nA;
+          nA = nB;
+          nB = t;
+          float *w_ = wA;
+          wA = wB;
+          wB = w_;
+          __syncthreads();
+        };
+        if (g.full) {
+#pragma unroll 2
+          for (int m = 0; m < nsw; ++m) {
+            sweep<R, MODE, true, false, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0);
+            next();
+          }
+        } else {
+#pragma unroll 2
+          for (int m = 0; m < nsw; ++m) {
+            sweep<R, MODE, false, false, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0);
+            next();
+          }
+        }
+        p ^= nsw & 1;
+        sw += nsw;
+        if (G > 1) {  // also after the last sweep: the halo's correction is added too
+          ++e;
+          show();
+          __syncthreads();
+          publish(e);
+          es = (es + 1) & 3;
+          if (!receive(e, es)) fail();
+          if (sw >= todo && warp == 0) wait_res(q);
+          __syncthreads();
+          take();
+          p ^= 1;
+          sts4(first + p * par + mine, x[0]);
+          sts4(last + p * par + mine, x[R - 1]);
+          __syncthreads();
+          if (js->bail) break;
+        }
+      }
+      if (js->bail) break;
+      if (G > 1) {
+        res = __longlong_as_double((long long)js->res64[q & 1]);
+        if (done >= J.r64_mn && res < J.r64_tol && !J.trial) break;
+      }
+      auto add_row = [&](double *z, const float4 &d) {
+        z[0] += to_double(d.x);
+        z[1] += to_double(d.y);
+        z[2] += to_double(d.z);
+        z[3] += to_double(d.w);
+      };
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (r < g.nvalid) add_row(q64 + r * 128, x[r]);
+      if (!idle && south_edge && by > 0) add_row(p64 + 4 * li, lds4(edge + es * 256 + 4 * li));
+      if (!idle && north_edge && by < nby - 1)
+        add_row(p64 + (hi - lo + 2) * 128 + 4 * li, lds4(edge + es * 256 + 128 + 4 * li));
+      done += todo;
+      ++q;
+      __syncthreads();
+    }
+    // phi64, its FP32 copy and the field (mesh.cu:413-468, rounded once)
+    const double d1 = a.ds_d, d2 = 2.0 * a.ds_d;
+    auto put64 = [&](int j, const double *z, bool rim) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (!((g.own >> k) & 1u)) continue;
+        const size_t o = (size_t)j * nnx + g.i0 + k;
+        const bool col0 = g.i0 == 0 && k == 0;
+        if (!rim) {
+          phi64[o] = z[k];
+          if (col0) phi64[o + W] = z[k];
+        }
+        const float f = __double2float_rn(z[k]);
+        a.phi[o] = f;
+        if (col0) a.phi[o + W] = f;
+        if (J.do_field) {
+          double ex = 0.0, ey;
+          if (j == 0) {
+            ey = (z[k] - z[k + 128]) / d1;
+          } else if (j == nny - 1) {
+            ey = (z[k - 128] - z[k]) / d1;
+          } else {
+            ex = ((k == 0 ? z[wc] : z[k - 1]) - east(z, k)) / d2;
+            ey = (z[k - 128] - z[k + 128]) / d2;
+          }
+          const float2 E = make_float2(__double2float_rn(ex), __double2float_rn(ey));
+          a.E[o] = E;
+          if (col0) a.E[o + W] = E;
+        }
+      }
+    };
+    __syncthreads();
+#pragma unroll 1
+    for (int r = 0; r < R; ++r)
+      if ((g.ownrows >> r) & 1u) put64(g.row0 + r, q64 + r * 128, false);
+    if (!idle && south_edge && by == 0) put64(0, p64 + 4 * li, true);
+    if (!idle && north_edge && by == nby - 1) put64(nny - 1, p64 + (hi - lo + 2) * 128 + 4 * li, true);
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      if (atomicAdd(&ctl->jdone, 1u) == (unsigned)G - 1u) {
+        __threadfence();
+        ctl->jdone = 0u;
+        if (J.r64_stats) {
+          ctl->sweeps = done;
+          ctl->residual = (float)res;
+        }
+        finish(e);
+      }
+    }
+    return;
+  }
 
   // ---- sweeps ----------------------------------------------------------
   // A checked sweep is one that the stop rule looks at; when the solve cannot
@@ -714,8 +983,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       prev = c;
     }
   }
-  // the last CTA to finish writes the report, puts the counters back to zero
-  // and advances the epochs past this solve's
+  // the last CTA to finish also writes the report
   __syncthreads();
   if (tid == 0) {
     __threadfence();
@@ -728,42 +996,34 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
                             ? __uint_as_float((unsigned)ld_word(&J.gmax[((nq - 1) & 3) * 32 + ((J.max_sweeps - 1) % KB)]))
                             : resv;
       }
-      unsigned next = ebase + (unsigned)max(e, nq) + 2u;
-      const bool wrap = next > kEpochEnd;  // start over, above the tags left in gmax
-      if (wrap) next = 0u;
-      if (G > 1) {
-        for (int k = 0; k < 4; ++k) J.tbar[k] = 0u;
-        if (wrap)
-          for (int k = 0; k < 128; ++k) J.gmax[k] = 0ull;
-      }
-      ctl->jepoch = next;
+      finish(max(e, nq));
     }
   }
 }
 
-template <int R, int MODE>
+template <int R, int MODE, bool REFINE>
 __global__ void __launch_bounds__(512, 1) k_tile(SimArgs a, JacobiArgs J) {
   extern __shared__ __align__(16) float tsm[];
   __shared__ Scratch js;
   if (threadIdx.x == 0) js.bail = 0;
   __syncthreads();
-  solve<R, MODE>(a, J, blockIdx.x, tsm, &js);
+  solve<R, MODE, REFINE>(a, J, blockIdx.x, tsm, &js);
 }
 
 using Kernel = void (*)(SimArgs, JacobiArgs);
 
 // the kernel of MODE with strips of r rows (1..8)
-template <int MODE>
+template <int MODE, bool REFINE>
 inline Kernel pick(int r) {
   switch (r) {
-    case 1: return k_tile<1, MODE>;
-    case 2: return k_tile<2, MODE>;
-    case 3: return k_tile<3, MODE>;
-    case 4: return k_tile<4, MODE>;
-    case 5: return k_tile<5, MODE>;
-    case 6: return k_tile<6, MODE>;
-    case 7: return k_tile<7, MODE>;
-    default: return k_tile<8, MODE>;
+    case 1: return k_tile<1, MODE, REFINE>;
+    case 2: return k_tile<2, MODE, REFINE>;
+    case 3: return k_tile<3, MODE, REFINE>;
+    case 4: return k_tile<4, MODE, REFINE>;
+    case 5: return k_tile<5, MODE, REFINE>;
+    case 6: return k_tile<6, MODE, REFINE>;
+    case 7: return k_tile<7, MODE, REFINE>;
+    default: return k_tile<8, MODE, REFINE>;
   }
 }
 

@@ -59,3 +59,50 @@ def test_tile_layouts_match_oracle(gpu_lib, monkeypatch, ncx, ncy, ctas, depth):
         st, so = sim.stats(1)[0], ora.stats()
         assert st["sweeps"] == so["sweeps"] and st["residual"] == so["residual"]
     ora.close()
+
+
+# precision form: (cells in x, cells in y, CTAs, depth, sweeps per correction)
+REFINED = [(3, 5, None, None, 4), (32, 40, 1, 1, 8), (64, 90, 5, 4, 32), (67, 50, 4, 8, 5), (100, 40, 3, 16, 24),
+           (140, 70, 6, 8, 10), (257, 60, 12, 4, 16), (300, 64, None, None, 32)]
+
+
+@pytest.mark.parametrize("ncx,ncy,ctas,depth,every", REFINED)
+def test_refining_tiles_match_oracle(gpu_lib, monkeypatch, ncx, ncy, ctas, depth, every):
+    """The precision form in one launch: FP64 potential, field, sweep counts
+    and residuals equal the oracle's, for stops by the sweep cap, by the
+    tolerance and before the first correction, and for sweeps per correction
+    that are no multiple of the depth."""
+    for name, v in (("CUPIC_JACOBI_CTAS", ctas), ("CUPIC_JACOBI_DEPTH", depth)):
+        if v is None:
+            monkeypatch.delenv(name, raising=False)
+        else:
+            monkeypatch.setenv(name, str(v))
+    p = cg.workload_params("tiny", ncx=ncx, ncy=ncy, refine_every=every, tol=2e-3, min_sweeps=every, max_sweeps=60,
+                           init_tol=1e-2, init_min_sweeps=every, init_max_sweeps=500)
+    ora = Oracle(p, fp64=False)
+    ora.init_plasma()
+    with cg.Sim(p) as sim:
+        sim.init_plasma()
+        np.testing.assert_array_equal(sim.phi64(), ora.phi())
+        for tol, mn, mx in ((0.0, 0, 0), (0.0, 7, 7), (1e9, 0, 50), (5e-2, 10, 300), (1e-3, 10, 97)):
+            sim.poisson_solver(tol, mn, mx, 1)
+            ora.solve(tol, mn, mx, 1)
+            np.testing.assert_array_equal(sim.phi64(), ora.phi(), err_msg=f"tol {tol}, {mn}..{mx} sweeps")
+        for _ in range(3):
+            sim.step(1)
+            ora.step(1)
+            g, o = sim.stats(1)[0], ora.stats()
+            assert g["sweeps"] == o["sweeps"] and g["residual"] == o["residual"] and g["flags"] == 0
+        np.testing.assert_array_equal(sim.phi64(), ora.phi())
+        for g, o in zip(sim.efield(), ora.efield()):
+            np.testing.assert_array_equal(g.astype(np.float64), o)
+        # a mirror column that differs keeps its own FP64 value (launches of jacobi.cu)
+        phi = ora.phi()
+        phi[1:-1, -1] += 1e-3
+        sim.set_phi(phi)
+        ora.set_phi(phi)
+        sim.step(1)
+        ora.step(1)
+        for sp in (0, 1):
+            np.testing.assert_array_equal(sim.particles(sp), ora.particles(sp))
+    ora.close()
