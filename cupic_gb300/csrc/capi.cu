@@ -358,14 +358,16 @@ int set_jacobi_plan(cupic_ctx *c, int G, int B, int K, int P) {
 }
 
 int set_tile_plan(cupic_ctx *c, const TilePlan &t) {
+  int n = 0;
+  if (tile_max_ctas(t, c->num_sms, &n) != cudaSuccess || t.G > n) {
+    cudaGetLastError();
+    return CUPIC_ERR_ARG;
+  }
   c->jG = t.G;
   c->jB = t.B;
   c->jK = t.K;
   c->jP = (c->a.nnx + 3) / 4 * 4;
   c->tile = t;
-  int n = 0;
-  CU(tile_max_ctas(t, c->num_sms, &n));
-  if (t.G > n) return CUPIC_ERR_ARG;
   return alloc_jacobi_scratch(c, t.G, t.words);
 }
 
@@ -568,7 +570,7 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
     cands.push_back(t);
     words = std::max(words, t.words);
     maxG = std::max(maxG, t.G);
-    if ((int)cands.size() >= kTileTrials) break;
+    if ((int)cands.size() >= (getenv("CUPIC_TILE_TRIALS") ? atoi(getenv("CUPIC_TILE_TRIALS")) : kTileTrials)) break;
   }
   if (cands.empty()) return CUPIC_ERR_CAPACITY;
   TilePlan pick = cands.front();
@@ -594,6 +596,9 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
         float ms = 0.0f;
         if (ok && rep > 0 && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess) ms_best = std::min(ms_best, ms);
       }
+      if (getenv("CUPIC_TILE_VERBOSE"))
+        fprintf(stderr, "tile %dx%d: nbx %d nby %d K %d R %d warps %d mode %d: %.1f us (cost %.0f)\n", c->a.nnx, c->a.nny,
+                t.nbx, t.nby, t.K, t.R, t.warps, t.mode, 1e3 * ms_best, t.cost);
       if (!ok) {
         cudaGetLastError();
         continue;

@@ -53,7 +53,8 @@ cudaError_t jacobi_max_ctas(size_t smem, int *per_sm);
 cudaError_t launch_jacobi(const SimArgs &a, const JacobiArgs &J, cudaStream_t st);
 
 // the register-tile solve (tile.cuh, tile.cu)
-constexpr int kTileWarps = 16;  // most warps of a CTA
+constexpr int kTileWarps = 16;  // most warps of a CTA, of 128 registers a thread
+constexpr int kTileRows = 8;    // most rows of a strip
 constexpr int kTileDepth = 16;  // deepest halo
 // a solve of a fixed number of sweeps, one that may stop on its tolerance
 // (and keeps snapshots), the precision form (and keeps its FP64 potential)
@@ -70,7 +71,7 @@ struct TilePlan {
   double cost;             // estimated SM cycles per sweep
 };
 bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, TilePlan *out);
-std::vector<TilePlan> tile_plans(int nnx, int nny, int max_ctas, TileForm form, size_t max_smem);
+std::vector<TilePlan> tile_plans(int nnx, int nny, int num_sms, TileForm form, size_t max_smem);
 void tile_args(const TilePlan &t, JacobiArgs *J);
 cudaError_t tile_max_ctas(const TilePlan &t, int num_sms, int *ctas);
 cudaError_t launch_tile(const SimArgs &a, const JacobiArgs &J, const TilePlan &t, cudaStream_t st);

@@ -85,7 +85,7 @@ TilePlan tiles_for(int dev, int num_sms, int dev_max, int nnx, int nny, int max_
   const auto it = kept.find(key);
   if (it != kept.end()) return it->second;
   TilePlan pick{};
-  for (const TilePlan &t : tile_plans(nnx, nny, max_ctas, form, (size_t)dev_max - 1024)) {
+  for (const TilePlan &t : tile_plans(nnx, nny, num_sms, form, (size_t)dev_max - 1024)) {
     int n = 0;
     if (kCtlHeadBytes + sizeof(unsigned long long) * t.words > kStaticScratchBytes || t.G > max_ctas) continue;
     if (tile_max_ctas(t, num_sms, &n) != cudaSuccess) {

@@ -53,11 +53,12 @@ __global__ void k_field(SimArgs a, int do_field, int write_stats) {
 }  // namespace
 
 // The layout of nbx x nby blocks with halo depth K and strips of R rows (0:
-// the smallest that needs at most kTileWarps warps); false if there is none.
+// the fewest that need at most kTileWarps warps); false if there is none.
 bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, TilePlan *out) {
   const int W = nnx - 1, M = nny - 2, W4 = (W + 3) / 4;
   TilePlan t{};
   t.form = form;
+  if ((long long)M * (nby + 1) >= 1ll << 31) return false;
   if (nbx < 1 || nby < 1 || K < 1 || nby > M || nbx > W4 || K > kTileDepth) return false;
   if (nby > 1 && K > M / nby) return false;  // a block trades K of its own rows
   if (nbx == 1) {
@@ -87,7 +88,7 @@ bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, 
     if (b == 2 && nby > 8 && M % nby == 0) break;  // all inner blocks alike
   }
   if (R == 0) R = (rows + kTileWarps * t.segs - 1) / (kTileWarps * t.segs);
-  if (R < 1 || R > 8) return false;
+  if (R < 1 || R > kTileRows) return false;
   t.R = R;
   t.warps = (rows + R * t.segs - 1) / (R * t.segs);
   if (t.warps > kTileWarps) return false;
@@ -97,33 +98,38 @@ bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, 
   t.K = K;
   t.ip = nbx == 1 ? 4 * W4 : 4 * W4 + 36;
   const size_t thr = 32 * (size_t)t.warps;
+  t.trows = rows;
   if (t.G > 1) {
     const int wide = nbx > 1 ? 4 * ((W4 + nbx - 1) / nbx) + 2 * K : W;
-    t.trows = rows;
     const int own = nbx > 1 ? 4 * ((W4 + nbx - 1) / nbx) : W, side = nbx > 1 ? t.B * K : 0;
     t.tpairs = ((nby > 1 ? 2 : 0) * K * ((wide + 1) / 2) + side + 1) / 2 * 2;
     t.ppairs = (nby > 1 ? 2 : 0) * K * ((own + 1) / 2) + side;
     if (nbx > 1 && nby > 1) t.ppairs += 2 * (W % 2 ? K : K / 2) * 2 * K;  // periodic images
     t.ppairs = (t.ppairs + 1) / 2 * 2;
   }
-  // strip rows in two parities, edge rows, the exchange image and its tables
-  // (even numbers of entries: what follows is 16-byte aligned), two
-  // snapshots of the strips or the FP64 potential
-  t.smem = (4 * thr * 4 + 4 * 2 * 128 + (size_t)t.trows * 128) * sizeof(float) +
+  // strip rows in two parities, edge rows, the tile's image and the tables of
+  // exchange words (even numbers of entries: what follows is 16-byte aligned),
+  // two snapshots of the strips or the charges' image in their place, or the
+  // FP64 potential
+  t.smem = (4 * thr * 4 + 4 * 2 * 128 + (size_t)(rows + 2) * 4 * t.nl + (rows + 3) / 4 * 4) * sizeof(float) +
+           (size_t)(rows + 1) / 2 * 16 +
            (size_t)(t.tpairs + t.ppairs) * sizeof(uint2) + (form == kTileEarly ? 2 * R * thr * sizeof(float4) : 0) +
-           (form == kTileRefine ? ((size_t)(rows + 2) * 128 + 8) * sizeof(double) : 0);
+           (form == kTileFixed ? (size_t)rows * 4 * t.nl * sizeof(long long) : 0) +
+           (form == kTileRefine ? ((size_t)(rows + 2) * 4 * t.nl + 8) * sizeof(double) : 0);
   t.words = t.G == 1 ? 0
                      : (size_t)2 * nby * 2 * K * t.ip + (nbx > 1 ? (size_t)2 * nny * nbx * 2 * K : 0);
   if (t.words >= 1ull << 31) return false;
   // Estimated SM cycles per sweep, from timings at 2 GHz: 270 of latency (the
-  // barrier, the rows read from shared memory, the shuffles) and 18 issue
-  // slots a row for each warp of a scheduler (more above 5 rows, where
-  // registers run short); an exchange takes 2000 cycles, 2000 more with
-  // eight neighbours instead of two, and 800 for each pair of words a thread
-  // waits for, shared by the K sweeps between two of them.
-  const double rows_cost = t.R <= 5 ? 18.0 * t.R : 18.0 * t.R * (1.0 + 0.12 * (t.R - 5));
-  t.cost = 270.0 + ((t.warps + 3) / 4) * rows_cost;
-  if (t.G > 1) t.cost += (2000.0 + (nbx > 1 ? 2000.0 : 0.0) + 800.0 * t.tpairs / thr) / K;
+  // barrier, the shuffles, the two rows a warp takes and sends through shared
+  // memory) and 14 issue slots a row for each warp of a scheduler (more above
+  // 5 rows, where registers run short); an exchange takes 2000 cycles, 1700
+  // more with eight neighbours instead of two, and 700 for each pair of words
+  // a thread waits for, shared by the K sweeps between two of them.
+  // Measured slower, 512x2048, 200 sweeps: strips of 12 rows on 8 warps of 255
+  // registers (half the rows through shared memory) 188 us against 170; two
+  // CTAs to an SM, one sweeping while the other waits, 239 against 175.
+  t.cost = 270.0 + ((t.warps + 3) / 4) * 14.0 * t.R * (t.R <= 5 ? 1.0 : 1.0 + 0.12 * (t.R - 5));
+  if (t.G > 1) t.cost += (2000.0 + (nbx > 1 ? 1700.0 : 0.0) + 700.0 * t.tpairs / thr) / K;
   // the precision form's FP64 work: about 9 operations a node at 2 a clock,
   // once a correction (32 sweeps)
   if (form == kTileRefine) t.cost += 4.5 * 4 * 32 * R * t.warps / 32;
@@ -132,21 +138,21 @@ bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, 
 }
 
 // The layouts worth timing, cheapest estimate first.
-std::vector<TilePlan> tile_plans(int nnx, int nny, int max_ctas, TileForm form, size_t max_smem) {
+std::vector<TilePlan> tile_plans(int nnx, int nny, int num_sms, TileForm form, size_t max_smem) {
   const int W = nnx - 1, M = nny - 2, W4 = (W + 3) / 4;
   std::vector<TilePlan> out;
   const int depths[] = {1, 2, 4, 6, 8, 12, 16};
-  const int grids[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128, max_ctas};
+  const int grids[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128, num_sms};
   for (int nbx = 1; nbx <= std::min(W4, 64); ++nbx)
     for (int g : grids) {
       const int nby = g / nbx;
-      if (nby < 1 || nby > M || (nbx > 1 && g != max_ctas && g % nbx)) continue;
+      if (nby < 1 || nby > M || (nbx > 1 && g < num_sms && g % nbx)) continue;
       for (int K : depths) {
         if (nbx * nby == 1 && K > 1) continue;
         TilePlan t;
         if (!tile_plan(nnx, nny, nbx, nby, K, 0, form, &t)) continue;
         const int R0 = t.R;
-        for (int R = R0; R <= std::min(8, R0 + 2); ++R)
+        for (int R = R0; R <= kTileRows; ++R)
           if (tile_plan(nnx, nny, nbx, nby, K, R, form, &t) && t.smem <= max_smem) out.push_back(t);
       }
     }

@@ -38,6 +38,7 @@
 #include <math.h>
 
 #include "cupic_internal.cuh"
+#include "draws.cuh"
 #include "kernels.h"
 
 namespace cupic {
@@ -99,42 +100,81 @@ struct Lane {
   bool full;         // no lane of the warp has a partial strip
 };
 
+// The strips hold s = 4 phi, the sum of a node before its product by 1/4: the
+// product of a neighbour's sum is exact, so a fused multiply-add rounds as the
+// sum with the neighbour's phi does, and a node takes four operations instead
+// of five.  (phi below 2^-124 in size, whose product by 1/4 would be rounded
+// to a subnormal, is carried exactly instead.)
 __device__ __forceinline__ float node(float b, float w, float e, float n, float s) {
-  return __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(b, w), e), n), s));
+  return __fmaf_rn(0.25f, s, __fmaf_rn(0.25f, n, __fmaf_rn(0.25f, e, __fmaf_rn(0.25f, w, b))));
+}
+__device__ __forceinline__ float times4f(float v) { return __fmul_rn(4.0f, v); }
+__device__ __forceinline__ float quarter(float v) { return __fmul_rn(0.25f, v); }
+__device__ __forceinline__ float4 quarter(const float4 &v) {
+  return make_float4(quarter(v.x), quarter(v.y), quarter(v.z), quarter(v.w));
+}
+
+// The source term of fixed-point charge f, (float)((double)f * cb).  Three FP64
+// operations a node were 13 us of a 512x2048 solve; the product in
+// double-float arithmetic rounds to the same float (draws.cuh) but for a few
+// nodes in a million and charges of 2^16 units and more, which take FP64.
+// (The FP64 fallbacks here and below are calls: inlined, the compiler computes
+// them always and selects.)
+static __device__ __noinline__ float source_f64(long long f, double cb) { return __double2float_rn((double)f * cb); }
+// pow2: cb is a power of two, so the charge's own rounding is the only one.
+__device__ __forceinline__ float source(long long f, double cb, const df &cbf, bool pow2) {
+  const unsigned long long u = f < 0 ? 0ull - (unsigned long long)f : (unsigned long long)f;
+  const df n = df_int(u);
+  bool ok = u < (1ull << 48);
+  float v = __fmul_rn(n.h, cbf.h);
+  if (!pow2) v = df_round(df_mul(n, cbf), ok);
+  if (!ok) return source_f64(f, cb);
+  return f < 0 ? -v : v;
+}
+
+// asynchronous copies of 4 and 8 bytes from global to shared memory
+__device__ __forceinline__ void copy4(void *to, const void *from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(to)), "l"(from) : "memory");
+}
+__device__ __forceinline__ void copy8(void *to, const void *from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(to)), "l"(from) : "memory");
 }
 
 // A warp's FP64 operation holds the SM's FP64 pipe for about 24 cycles, so the
 // correction's conversions and its product by 4 go through the integer pipe:
 // the same bits (round to nearest even), with the hardware's conversion for
 // what is not normal on both sides.  A 512x2048 correction: 57.1 -> 55.6 us.
+static __device__ __noinline__ float to_float_slow(double v) { return __double2float_rn(v); }
+static __device__ __noinline__ double to_double_slow(float v) { return (double)v; }
+static __device__ __noinline__ double times4_slow(double v) { return 4.0 * v; }
 __device__ __forceinline__ float to_float(double v) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(v);
   const unsigned e = (unsigned)(u >> 52) & 0x7ffu;
-  if (e - 897u >= 254u) return __double2float_rn(v);
+  if (e - 897u >= 254u) return u << 1 ? to_float_slow(v) : __uint_as_float((unsigned)(u >> 32));
   const unsigned t = (unsigned)(((u & 0x7fffffffffffffffull) + 0x0fffffffull + ((u >> 29) & 1ull)) >> 29);
   return __uint_as_float((t - (896u << 23)) | ((unsigned)(u >> 32) & 0x80000000u));
 }
 __device__ __forceinline__ double to_double(float v) {
   const unsigned b = __float_as_uint(v), e = (b >> 23) & 0xffu;
-  if (e - 1u >= 254u) return (b << 1) == 0u ? __hiloint2double((int)b, 0) : (double)v;
+  if (e - 1u >= 254u) return (b << 1) == 0u ? __hiloint2double((int)b, 0) : to_double_slow(v);
   return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
 }
 __device__ __forceinline__ double times4(double v) {
   const int hi = __double2hiint(v);
   const unsigned e = ((unsigned)hi >> 20) & 0x7ffu;
-  if (e - 1u >= 0x7fcu) return 4.0 * v;
+  if (e - 1u >= 0x7fcu) return times4_slow(v);
   return __hiloint2double(hi + 0x200000, __double2loint(v));
 }
 
-// One sweep of a strip: v = 1/4 ((((b + west) + east) + north) + south).
+// One sweep of a strip: v = (((b + west) + east) + north) + south on s = 4 phi.
 // FULL: all R rows of the strip are in the tile (the row above the last is
 // then x[R]'s place, taken from n4); otherwise the rows past the strip's end
 // compute values nothing reads.  FIRST: the solve's first sweep, which reads
 // the caller's mirror column (its value may differ from column 0's; every
-// later one equals it).  Returns the max |v - old| over owned nodes (CHECK).
+// later one equals it; used only when some value does differ).  Returns the max |v - old| over owned nodes (CHECK).
 template <int R, int MODE, bool FULL, bool CHECK, bool FIRST>
 __device__ __forceinline__ float sweep(float4 (&x)[R], const float4 (&b)[R], const float4 s4,
-                                       const float4 n4, const Lane &g, const float *mirror, int nnx) {
+                                       const float4 n4, const Lane &g, const float *mirror) {
   float4 prev = s4;
   float md = 0.0f;
 #pragma unroll
@@ -158,7 +198,7 @@ __device__ __forceinline__ float sweep(float4 (&x)[R], const float4 (&b)[R], con
     }
     e.w = rt;
     float mir = 0.0f;
-    if (FIRST && mirror && r < g.nvalid && (g.me >= 0 || g.i0 == 0)) mir = mirror[(size_t)(g.row0 + r) * nnx];
+    if (FIRST && r < g.nvalid) mir = mirror[r];
     if (FIRST && g.me >= 0) {
       e.x = g.me == 0 ? mir : e.x;
       e.y = g.me == 1 ? mir : e.y;
@@ -186,17 +226,55 @@ __device__ __forceinline__ float sweep(float4 (&x)[R], const float4 (&b)[R], con
   return md;
 }
 
+// A strip's rows in shared memory: those below and above it (read), its
+// first and last (written; the last at +to_last), this sweep's (A) and the
+// next one's (B).
+struct Rows {
+  const float *sA, *nA, *sB, *nB;
+  float *wA, *wB;
+  int to_last;
+};
+
+// Sweeps m .. end-1 of a block.  (Measured slower: the strip's outer rows
+// first, an mbarrier arrival and the rows between while the others catch
+// up, 100 cycles more a sweep; the same order with __syncthreads, no gain.)
+template <int R, int MODE, bool FULL, bool CHECK, class Note>
+__device__ __forceinline__ void sweeps(float4 (&x)[R], const float4 (&b)[R], const Lane &g, Rows &w, int &m, int end,
+                                       Note &&note) {
+#pragma unroll 2
+  for (; m < end; ++m) {
+    const float md = sweep<R, MODE, FULL, CHECK, false>(x, b, lds4(w.sA), lds4(w.nA), g, nullptr);
+    if (CHECK) note(md, m);
+    sts4(w.wB, x[0]);
+    sts4(w.wB + w.to_last, x[R - 1]);
+    const float *t = w.sA;
+    w.sA = w.sB;
+    w.sB = t;
+    t = w.nA;
+    w.nA = w.nB;
+    w.nB = t;
+    float *u = w.wA;
+    w.wA = w.wB;
+    w.wB = u;
+    __syncthreads();
+  }
+}
+
 template <int R, int MODE, bool REFINE>
 __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, const int c, float *sm,
                                       Scratch *js) {
   Ctl *ctl = a.ctl;
-  if (halted(ctl)) return;
+  // one round trip for the three words of the control block
+  const bool halt = halted(ctl);
+  const int cur = *reinterpret_cast<volatile int *>(&ctl->cur);
+  const unsigned ebase = *reinterpret_cast<volatile unsigned *>(&ctl->jepoch);
+  if (halt) return;
   const int G = J.G, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
   const int nnx = a.nnx, nny = a.nny, W = nnx - 1, M = nny - 2;
   const int nbx = MODE == kHalo ? J.nbx : 1, nby = J.nby;
   const int K = J.depth;
   const int bx = MODE == kHalo ? c % nbx : 0, by = MODE == kHalo ? c / nbx : c;
-  const int r0 = 1 + (int)(((long long)by * M) / nby), r1 = 1 + (int)(((long long)(by + 1) * M) / nby);
+  const int r0 = 1 + by * M / nby, r1 = 1 + (by + 1) * M / nby;  // (tile_plan bounds nby * M)
   int x0 = 0, x1 = W;
   if (MODE == kHalo) {
     const int W4 = (W + 3) >> 2;
@@ -242,57 +320,110 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   const bool south_edge = g.row0 == lo, north_edge = g.nvalid > 0 && g.row0 + g.nvalid - 1 == hi;
   const bool idle = g.nvalid == 0;
 
-  float *const phi = J.phi ? J.phi : a.phi;
-  const long long *acc = reinterpret_cast<const long long *>(a.rho[ctl->cur]);
-  const unsigned ebase = *reinterpret_cast<volatile unsigned *>(&ctl->jepoch);
-  if (J.zero_next) {  // the accumulator the step's push deposits into, in equal shares
-    unsigned long long *nx = a.rho[ctl->cur ^ 1];
+  float *const phi = a.phi;
+  const long long *acc = reinterpret_cast<const long long *>(a.rho[cur]);
+  // An image of the tile in shared memory, rows lo-1 .. hi+1 of tp columns: the
+  // mesh is read and written through it a warp to a row, coalesced, and halo
+  // nodes pass through it.  The mirror column and the tables of exchange words
+  // follow it, then the snapshots, whose place first holds the charges.
+  const int tp = 4 * nl, rows = hi - lo + 1, nwarp = nthr >> 5;
+  float *const timg0 = edge + 4 * 2 * 128;  // row lo-1
+  float *const timg = timg0 + tp;           // row lo
+  long long *const wcol = reinterpret_cast<long long *>(timg0 + (size_t)(J.trows + 2) * tp);  // the mirror column's
+  float *const mcol = reinterpret_cast<float *>(wcol + (J.trows + 1) / 2 * 2);  // charge, and potential at the start
+  uint2 *const table = reinterpret_cast<uint2 *>(mcol + (J.trows + 3) / 4 * 4);
+  uint2 *const ptable = table + J.tpairs;
+  float4 *const snap = reinterpret_cast<float4 *>(ptable + J.ppairs);
+  // the accumulator the step's push deposits into, cleared in equal shares
+  // (called with loads in flight)
+  auto clear_next = [&]() {
+    if (!J.zero_next) return;
+    unsigned long long *const nx = a.rho[cur ^ 1];
     const long long nodes = (long long)nnx * nny;
-    for (long long k = nodes * c / G + tid; k < nodes * (c + 1) / G; k += nthr) nx[k] = 0ull;
-  }
-
-  // real column of element q of this lane (-1: none)
-  auto column = [&](int q) {
-    int i = g.i0 + q;
-    if (!act) return -1;
-    if (MODE == kHalo) return i < 0 ? i + W : (i >= W ? (i - W < W ? i - W : -1) : i);
-    return i < W ? i : -1;
+    const long long k0 = nodes * c / G, k1 = nodes * (c + 1) / G;
+    const long long e0 = min(k1, (k0 + 1) & ~1ll), e1 = max(e0, k1 & ~1ll);
+    if (tid == 0 && e0 > k0) nx[k0] = 0ull;
+    if (tid == 0 && e1 < k1) nx[e1] = 0ull;
+    for (long long k = e0 + 2 * tid; k < e1; k += 2 * nthr)
+      *reinterpret_cast<ulonglong2 *>(nx + k) = make_ulonglong2(0ull, 0ull);
   };
+  // real column of tile column tc (-1: none)
+  const int nc = x1 - x0 + 2 * KX;
+  auto real = [&](int tc) {
+    const int i = x0 - KX + tc;
+    return tc >= nc ? -1 : (i < 0 ? i + W : (i >= W ? i - W : i));
+  };
+  // The mesh comes in by asynchronous copies, a warp to a row.  These one-time
+  // phases are loops and not unrolled: their instructions are fetched anew in
+  // every solve, and straight-line code of them took longer to fetch than the
+  // data.
   float4 x[R], b[R];
-  {
-    const int c0 = column(0), c1 = column(1), c2 = column(2), c3 = column(3);
-    auto ldphi = [&](int j, int i) { return i >= 0 ? phi[(size_t)j * nnx + i] : 0.0f; };
-    auto ldsrc = [&](int j, int i) {
-      if (i < 0) return 0.0f;
-      const size_t rb = (size_t)j * nnx;
-      if (J.src) return J.src[rb + i];
-      const long long f = i == 0 ? acc[rb] + acc[rb + W] : acc[rb + i];
-      return __double2float_rn((double)f * a.cb);
-    };
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      x[r] = b[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (!REFINE && r < g.nvalid) {
-        const int j = g.row0 + r;
-        if (!J.phi_zero) x[r] = make_float4(ldphi(j, c0), ldphi(j, c1), ldphi(j, c2), ldphi(j, c3));
-        b[r] = make_float4(ldsrc(j, c0), ldsrc(j, c1), ldsrc(j, c2), ldsrc(j, c3));
+  for (int r = 0; r < R; ++r) x[r] = b[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool seam = false;  // the mirror column differs from column 0 somewhere
+  if (!REFINE) {
+    long long *const aimg = reinterpret_cast<long long *>(snap);  // charges of rows lo..hi, then their source terms
+#pragma unroll 1
+    for (int r = warp; r < rows + 2; r += nwarp) {
+      const size_t rb = (size_t)(lo - 1 + r) * nnx;
+      const bool inner = r > 0 && r <= rows;
+#pragma unroll 1
+      for (int tc = lane; tc < nc; tc += 32) {
+        const int i = real(tc);
+        copy4(timg0 + r * tp + tc, phi + rb + i);
+        if (inner) copy8(aimg + (r - 1) * tp + tc, acc + rb + i);
+        if (inner && i == 0) {
+          copy4(mcol + r - 1, phi + rb + W);
+          copy8(wcol + r - 1, acc + rb + W);
+        }
       }
     }
-    if (!idle) {
-      const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    clear_next();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const bool pow2 = (__double_as_longlong(a.cb) & 0xfffffffffffffll) == 0ll;
+    const df cb = df_of(a.cb);
+#pragma unroll 1
+    for (int r = warp; r < rows + 2; r += nwarp) {
+      const bool inner = r > 0 && r <= rows;
+#pragma unroll 2
+      for (int tc = lane; tc < tp; tc += 32) {
+        const int i = real(tc);
+        float *const v = timg0 + r * tp + tc;
+        float p4 = i >= 0 ? times4f(*v) : 0.0f;
+        if (inner) {
+          *v = p4;
+          long long f = i >= 0 ? aimg[(r - 1) * tp + tc] : 0ll;
+          if (i == 0) {  // column 0's charge is folded with the mirror column's
+            f += wcol[r - 1];
+            const float m = times4f(mcol[r - 1]);
+            mcol[r - 1] = m;
+            seam = seam || !(m == p4);
+          }
+          const float s = source(f, a.cb, cb, pow2);
+          *reinterpret_cast<float *>(aimg + (r - 1) * tp + tc) = s;
+        } else {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (south_edge)
-          sts4(edge + (2 * q) * 128 + 4 * li,
-               REFINE || J.phi_zero ? z : make_float4(ldphi(lo - 1, c0), ldphi(lo - 1, c1), ldphi(lo - 1, c2), ldphi(lo - 1, c3)));
-        if (north_edge)
-          sts4(edge + (2 * q + 1) * 128 + 4 * li,
-               REFINE || J.phi_zero ? z : make_float4(ldphi(hi + 1, c0), ldphi(hi + 1, c1), ldphi(hi + 1, c2), ldphi(hi + 1, c3)));
+          for (int q = 0; q < 4; ++q) edge[(2 * q + (r == 0 ? 0 : 1)) * 128 + tc] = p4;
+        }
       }
     }
-    sts4(first + mine, x[0]);
-    sts4(last + mine, x[R - 1]);
+    seam = __syncthreads_or(seam);
+    const float *const q = timg + (g.row0 - lo) * tp + 4 * li;
+    const float4 *const s4 = reinterpret_cast<const float4 *>(aimg + (g.row0 - lo) * tp + 4 * li);
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (r < g.nvalid) {
+        x[r] = lds4(q + r * tp);
+        const float4 u0 = s4[r * (tp / 2)], u1 = s4[r * (tp / 2) + 1];
+        b[r] = make_float4(u0.x, u0.z, u1.x, u1.z);
+      }
+  } else {
+    for (int k = tid; k < 4 * 2 * 128; k += nthr) edge[k] = 0.0f;
+    clear_next();
   }
+  sts4(first + mine, x[0]);
+  sts4(last + mine, x[R - 1]);
 
   // exchange words, two parities of: rows [by][bottom, top][K][ip] by
   // extended column, then (halo tiles) columns [row][bx][left, right][K]
@@ -308,82 +439,55 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   // the periodic images of those within K of column 0 or W.  kEdge marks a
   // place in the edge rows, kOne a single word (odd widths).
   constexpr unsigned kEdge = 1u << 30, kOne = 1u << 31;
-  const int nc = x1 - x0 + 2 * KX, nc2 = (nc + 1) >> 1, h = r1 - r0;
+  const int nc2 = (nc + 1) >> 1, h = r1 - r0;
   const int nlow = by > 0 ? K * nc2 : 0, nhigh = by < nby - 1 ? K * nc2 : 0;
   const int npair = G > 1 ? nlow + nhigh + (MODE == kHalo ? h * K : 0) : 0;
-  float *const timg = edge + 4 * 2 * 128;  // [hi-lo+1][128]: halo nodes of the strips
-  uint2 *const table = reinterpret_cast<uint2 *>(timg + (size_t)J.trows * 128);
-  uint2 *const ptable = table + J.tpairs;
-  float4 *const snap = reinterpret_cast<float4 *>(ptable + J.ppairs);
-  for (int u = tid; u < npair; u += nthr) {
-    uint2 t;
-    int q, j, col;  // word offset, mesh row, tile column of the pair
-    bool one = false;
-    if (u < nlow + nhigh) {
-      const bool low = u < nlow;
-      const int v = low ? u : u - nlow, k = v / nc2;
-      col = 2 * (v - k * nc2);
-      one = col + 1 >= nc;
-      j = low ? r0 - K + k : r1 + k;
-      q = (int)hrow(low ? by - 1 : by + 1, low ? 1 : 0, k) + x0 - KX + col;
-    } else {
-      const int v = u - nlow - nhigh, row = v / K, k = v - row * K;  // K/2 pairs left, K/2 right
-      const bool left = k < (K >> 1);
-      const int kk = 2 * (left ? k : k - (K >> 1));
-      j = r0 + row;
-      col = left ? kk : nc - K + kk;
-      q = (int)(left ? vcol(j, bx == 0 ? nbx - 1 : bx - 1, 1) : vcol(j, bx + 1 == nbx ? 0 : bx + 1, 0)) + kk;
-    }
-    t.x = (unsigned)q;
-    if (j < lo) t.y = kEdge | (unsigned)col;
-    else if (j > hi) t.y = kEdge | (unsigned)(128 + col);
-    else t.y = (unsigned)((j - lo) * 128 + col);
-    if (one) t.y |= kOne;
-    table[u] = t;
-  }
   const int w = x1 - x0, w2 = (w + 1) >> 1;
   const int plow = by > 0 ? K * w2 : 0, phigh = by < nby - 1 ? K * w2 : 0;
-  // the image words of a row: as pairs when W is even, else one by one
+  // the periodic images of a row: as pairs when W is even, else word by word
   const int ni = W & 1 ? K : K >> 1, istep = W & 1 ? 1 : 2;
   const bool im0 = MODE == kHalo && x0 < K, im1 = MODE == kHalo && x1 > W - K;
+  const int per = ((im0 ? 1 : 0) + (im1 ? 1 : 0)) * ni;
   const int nside = MODE == kHalo ? h * K : 0;
-  const int nimg = ((im0 ? 1 : 0) + (im1 ? 1 : 0)) * ni * ((by > 0 ? K : 0) + (by < nby - 1 ? K : 0));
-  const int nout = G > 1 ? plow + phigh + nside + nimg : 0;
-  for (int u = tid; u < nout; u += nthr) {
-    uint2 t;
-    int q, j, i;  // word offset, mesh row, owned column of the first word
-    bool one = false;
-    if (u < plow + phigh) {
-      const bool low = u < plow;
-      const int v = low ? u : u - plow, k = v / w2;
-      i = x0 + 2 * (v - k * w2);
-      one = i + 1 >= x1;
-      j = low ? r0 + k : r1 - K + k;
-      q = (int)hrow(by, low ? 0 : 1, k) + i;
-    } else if (u < plow + phigh + nside) {
-      const int v = u - plow - phigh, row = v / K, k = v - row * K;
-      const bool left = k < (K >> 1);
-      const int kk = 2 * (left ? k : k - (K >> 1));
-      j = r0 + row;
-      i = left ? x0 + kk : x1 - K + kk;
-      q = (int)vcol(j, bx, left ? 0 : 1) + kk;
-    } else {
-      int v = u - plow - phigh - nside;
-      const int per = (im0 ? ni : 0) + (im1 ? ni : 0), row = v / per;
-      v -= row * per;
-      const bool at0 = im0 && v < ni;  // columns 0..K-1 again at W..W+K-1
-      const int k = istep * (at0 ? v : v - (im0 ? ni : 0));
-      i = at0 ? k : W - K + k;
-      one = istep == 1;
-      const bool low = by > 0 && row < K;
-      const int kr = low ? row : row - (by > 0 ? K : 0);
-      j = low ? r0 + kr : r1 - K + kr;
-      q = (int)hrow(by, low ? 0 : 1, kr) + (at0 ? i + W : i - W);
+  const int nout = G > 1 ? plow + phigh + nside + per * ((by > 0 ? K : 0) + (by < nby - 1 ? K : 0)) : 0;
+  if (G > 1) {
+#pragma unroll 1
+    for (int t = warp; t < 2 * K; t += nwarp) {  // row t of the bottom (t < K) and top boundaries
+      const bool low = t < K;
+      const int k = low ? t : t - K;
+      if (low ? by == 0 : by == nby - 1) continue;
+      const int jin = low ? r0 - K + k : r1 + k, jout = low ? r0 + k : r1 - K + k;
+      const unsigned qin = hrow(low ? by - 1 : by + 1, low ? 1 : 0, k) + x0 - KX, qout = hrow(by, low ? 0 : 1, k);
+      const unsigned to = jin < lo ? kEdge : (jin > hi ? kEdge | 128u : (unsigned)((jin - lo) * tp));
+      for (int v = lane; v < nc2; v += 32)
+        table[(low ? 0 : nlow) + k * nc2 + v] =
+            make_uint2(qin + 2 * v, (to + 2 * v) | (2 * v + 1 >= nc ? kOne : 0u));
+      const unsigned from = (unsigned)((jout - lo) * tp + KX);
+      for (int v = lane; v < w2; v += 32)
+        ptable[(low ? 0 : plow) + k * w2 + v] =
+            make_uint2(qout + x0 + 2 * v, (from + 2 * v) | (2 * v + 1 >= w ? kOne : 0u));
+      for (int v = lane; v < per; v += 32) {
+        const bool at0 = im0 && v < ni;  // columns 0..K-1 again at W..W+K-1, W-K..W-1 at -K..-1
+        const int kk = istep * (at0 ? v : v - (im0 ? ni : 0)), i = at0 ? kk : W - K + kk;
+        ptable[plow + phigh + nside + ((low || by == 0 ? 0 : K) + k) * per + v] =
+            make_uint2(qout + (at0 ? i + W : i - W), (from + i - x0) | (istep == 1 ? kOne : 0u));
+      }
     }
-    t.x = (unsigned)q;
-    t.y = (unsigned)((j - lo) * 128 + i - x0 + KX);
-    if (one) t.y |= kOne;
-    ptable[u] = t;
+    if (MODE == kHalo) {
+#pragma unroll 1
+      for (int row = warp; row < h; row += nwarp) {  // K/2 pairs on the left, K/2 on the right
+        const int j = r0 + row, k = lane;
+        if (k < K) {
+          const bool left = k < (K >> 1);
+          const int kk = 2 * (left ? k : k - (K >> 1));
+          const unsigned qin = left ? vcol(j, bx == 0 ? nbx - 1 : bx - 1, 1) : vcol(j, bx + 1 == nbx ? 0 : bx + 1, 0);
+          table[nlow + nhigh + row * K + k] =
+              make_uint2(qin + kk, (unsigned)((j - lo) * tp + (left ? kk : nc - K + kk)));
+          ptable[plow + phigh + row * K + k] =
+              make_uint2(vcol(j, bx, left ? 0 : 1) + kk, (unsigned)((j - lo) * tp + KX + (left ? kk : w - K + kk)));
+        }
+      }
+    }
   }
   // this thread's nodes that go out: rows within K of the block's bottom and
   // top, and every owned row of the lanes within K of its sides
@@ -398,10 +502,10 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   }
   // owned nodes into the image; then, after a barrier, out of it
   auto show = [&]() {
-    float *const q = timg + (g.row0 - lo) * 128 + 4 * li;
+    float *const q = timg + (g.row0 - lo) * tp + 4 * li;
 #pragma unroll
     for (int r = 0; r < R; ++r)
-      if ((outrows >> r) & 1u) sts4(q + r * 128, x[r]);
+      if ((outrows >> r) & 1u) sts4(q + r * tp, x[r]);
   };
   auto publish = [&](int e) {
     const unsigned ep = ebase + (unsigned)e;
@@ -433,14 +537,26 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       uint2 t[NB];
       unsigned long long w[NB][2];
 #pragma unroll
-      for (int q = 0; q < NB; ++q) t[q] = table[min(u0 + q * nthr, npair - 1)];
+      for (int q = 0; q < NB; ++q)  // past the end: the first pair again (no branch around a load)
+        t[q] = table[u0 + q * nthr < npair ? u0 + q * nthr : u0];
+      auto here = [&](int q) {
+        return (unsigned)(w[q][0] >> 32) == ep && ((t[q].y & kOne) || (unsigned)(w[q][1] >> 32) == ep);
+      };
+      // Wait on the first pair alone: the others come from the same blocks, and
+      // polling all of them loads L2 while the blocks are still writing
+      // (512x2048, depth 8: 0.79 us a sweep against 0.74).
+      for (long long it = 0;; ++it) {
+        ld_word2(hw + t[0].x, w[0][0], w[0][1]);
+        if (here(0)) break;
+        if (it >= kSpinLimit || ((it & 255) == 255 && *(volatile int *)&ctl->abort)) return false;
+      }
       for (long long it = 0;; ++it) {
         bool all = true;
 #pragma unroll
-        for (int q = 0; q < NB; ++q) ld_word2(hw + t[q].x, w[q][0], w[q][1]);
+        for (int q = 1; q < NB; ++q)
+          ld_word2(hw + t[q].x, w[q][0], w[q][1]);
 #pragma unroll
-        for (int q = 0; q < NB; ++q)
-          all = all && (unsigned)(w[q][0] >> 32) == ep && ((t[q].y & kOne) || (unsigned)(w[q][1] >> 32) == ep);
+        for (int q = 1; q < NB; ++q) all = all && here(q);
         if (all) break;
         if (it >= kSpinLimit || ((it & 255) == 255 && *(volatile int *)&ctl->abort)) return false;
       }
@@ -456,14 +572,14 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   };
   // this thread's halo nodes from shared memory
   auto take = [&]() {
-    const float *const q = timg + (g.row0 - lo) * 128 + 4 * li;
+    const float *const img = timg + (g.row0 - lo) * tp + 4 * li;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (r >= g.nvalid) continue;
       if (!((g.ownrows >> r) & 1u)) {
-        x[r] = lds4(q + r * 128);
+        x[r] = lds4(img + r * tp);
       } else if (MODE == kHalo && need_side) {
-        const float4 v = lds4(q + r * 128);
+        const float4 v = lds4(img + r * tp);
         x[r].x = (need_side & 1u) ? v.x : x[r].x;
         x[r].y = (need_side & 2u) ? v.y : x[r].y;
         x[r].z = (need_side & 4u) ? v.z : x[r].z;
@@ -479,6 +595,17 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     }
   };
 
+  auto rows_at = [&](int es_, int p_) {
+    Rows w_;
+    w_.sA = south_edge ? edge + es_ * 256 + 4 * li : last + p_ * par + soff;
+    w_.nA = north_edge || idle ? edge + es_ * 256 + 128 + 4 * li : first + p_ * par + noff;
+    w_.sB = south_edge ? w_.sA : last + (p_ ^ 1) * par + soff;
+    w_.nB = north_edge || idle ? w_.nA : first + (p_ ^ 1) * par + noff;
+    w_.wA = first + p_ * par + mine;
+    w_.wB = first + (p_ ^ 1) * par + mine;
+    w_.to_last = 2 * par;
+    return w_;
+  };
   // the last CTA to finish puts the counters back to zero and advances the
   // epochs past this solve's
   auto finish = [&](int used) {
@@ -504,20 +631,27 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   // tile) and the sweeps with their exchanges; a launch per correction, with
   // a grid barrier and every residual's potential read again, took 96 us.
   if constexpr (REFINE) {
-    double *const p64 = reinterpret_cast<double *>(ptable + J.ppairs);  // rows lo-1 .. hi+1, [128]
-    double *const q64 = p64 + (g.row0 - lo + 1) * 128 + 4 * li;         // this strip's first row
-    const int cc[4] = {column(0), column(1), column(2), column(3)};
+    double *const p64 = reinterpret_cast<double *>(ptable + J.ppairs);  // rows lo-1 .. hi+1, [tp]
+    double *const q64 = p64 + (g.row0 - lo + 1) * tp + 4 * li;          // this strip's first row
+    int cc[4];  // real columns of the lane's elements (-1: none)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = g.i0 + q;
+      cc[q] = !act || (MODE != kHalo && i >= W) || i >= x1 + KX ? -1 : (i < 0 ? i + W : (i >= W ? i - W : i));
+    }
     double *const phi64 = J.r64_phi;
-    auto load_row = [&](int j) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        p64[(j - lo + 1) * 128 + 4 * li + q] = cc[q] >= 0 ? phi64[(size_t)j * nnx + cc[q]] : 0.0;
-    };
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (r < g.nvalid) load_row(g.row0 + r);
-    if (!idle && south_edge) load_row(lo - 1);
-    if (!idle && north_edge) load_row(hi + 1);
+#pragma unroll 1
+    for (int r = warp; r < rows + 2; r += nwarp)
+#pragma unroll 1
+      for (int tc = lane; tc < tp; tc += 32) {
+        const int i = real(tc);
+        if (i >= 0)
+          copy8(p64 + r * tp + tc, phi64 + (size_t)(lo - 1 + r) * nnx + i);
+        else
+          p64[r * tp + tc] = 0.0;
+      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     // the columns west and east of this lane's, relative to them
     const int wc = MODE == kHalo ? (li == 0 ? 0 : -1) : (li == 0 ? W - 1 : -1);
     const int ring0 = -4 * li;  // column 0 of a ring
@@ -550,13 +684,13 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       for (int r = 0; r < R; ++r) {
         b[r] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < g.nvalid) {
-          const double *const z = q64 + r * 128;
+          const double *const z = q64 + r * tp;
           const double *const src = J.r64_b + (size_t)(g.row0 + r) * nnx;
           float v[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const double rr = (cc[k] >= 0 ? src[cc[k]] : 0.0) -
-                              (times4(z[k]) - ((((k == 0 ? z[wc] : z[k - 1]) + east(z, k)) + z[k + 128]) + z[k - 128]));
+                              (times4(z[k]) - ((((k == 0 ? z[wc] : z[k - 1]) + east(z, k)) + z[k + tp]) + z[k - tp]));
             v[k] = to_float(rr);
             const unsigned long long bits = (unsigned long long)__double_as_longlong(rr) & 0x7fffffffffffffffull;
             if (((g.own >> k) & 1u) && ((g.ownrows >> r) & 1u) && bits <= inf64 && bits > mx) mx = bits;
@@ -598,39 +732,13 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       const int todo = min(m_, J.r64_mx - done);
       for (int sw = 0; sw < todo;) {
         const int nsw = G > 1 ? min(K, todo - sw) : todo;
-        const float *sA = south_edge ? edge + es * 256 + 4 * li : last + p * par + soff;
-        const float *nA = north_edge || idle ? edge + es * 256 + 128 + 4 * li : first + p * par + noff;
-        const float *sB = south_edge ? sA : last + (p ^ 1) * par + soff;
-        const float *nB = north_edge || idle ? nA : first + (p ^ 1) * par + noff;
-        float *wA = first + p * par + mine, *wB = first + (p ^ 1) * par + mine;
-        const int tolast = 2 * par;
-        auto next = [&]() {
-          sts4(wB, x[0]);
-          sts4(wB + tolast, x[R - 1]);
-          const float *t = sA;
-          sA = sB;
-          sB = t;
-          t = nA;
-          nA = nB;
-          nB = t;
-          float *w_ = wA;
-          wA = wB;
-          wB = w_;
-          __syncthreads();
-        };
-        if (g.full) {
-#pragma unroll 2
-          for (int m = 0; m < nsw; ++m) {
-            sweep<R, MODE, true, false, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0);
-            next();
-          }
-        } else {
-#pragma unroll 2
-          for (int m = 0; m < nsw; ++m) {
-            sweep<R, MODE, false, false, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0);
-            next();
-          }
-        }
+        Rows at = rows_at(es, p);
+        auto none = [](float, int) {};
+        int m = 0;
+        if (g.full)
+          sweeps<R, MODE, true, false>(x, b, g, at, m, nsw, none);
+        else
+          sweeps<R, MODE, false, false>(x, b, g, at, m, nsw, none);
         p ^= nsw & 1;
         sw += nsw;
         if (G > 1) {  // also after the last sweep: the halo's correction is added too
@@ -663,51 +771,53 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       };
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (r < g.nvalid) add_row(q64 + r * 128, x[r]);
-      if (!idle && south_edge && by > 0) add_row(p64 + 4 * li, lds4(edge + es * 256 + 4 * li));
+        if (r < g.nvalid) add_row(q64 + r * tp, quarter(x[r]));
+      if (!idle && south_edge && by > 0) add_row(p64 + 4 * li, quarter(lds4(edge + es * 256 + 4 * li)));
       if (!idle && north_edge && by < nby - 1)
-        add_row(p64 + (hi - lo + 2) * 128 + 4 * li, lds4(edge + es * 256 + 128 + 4 * li));
+        add_row(p64 + (rows + 1) * tp + 4 * li, quarter(lds4(edge + es * 256 + 128 + 4 * li)));
       done += todo;
       ++q;
       __syncthreads();
     }
-    // phi64, its FP32 copy and the field (mesh.cu:413-468, rounded once)
+    // phi64, its FP32 copy and the field (mesh.cu:413-468, rounded once), row
+    // by row; a quotient by a power of two is the product by its inverse
     const double d1 = a.ds_d, d2 = 2.0 * a.ds_d;
-    auto put64 = [&](int j, const double *z, bool rim) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (!((g.own >> k) & 1u)) continue;
-        const size_t o = (size_t)j * nnx + g.i0 + k;
-        const bool col0 = g.i0 == 0 && k == 0;
-        if (!rim) {
-          phi64[o] = z[k];
-          if (col0) phi64[o + W] = z[k];
+    const bool pow2 = (__double_as_longlong(d1) & 0xfffffffffffffll) == 0ll;
+    const double i1 = 1.0 / d1, i2 = 1.0 / d2;
+    auto over = [&](double v, double d, double i) { return pow2 ? v * i : v / d; };
+    __syncthreads();
+    const int ja = by == 0 ? 0 : r0, jb = by == nby - 1 ? nny : r1;
+#pragma unroll 1
+    for (int j = ja + warp; j < jb; j += nwarp) {
+      const double *const z = p64 + (j - lo + 1) * tp;
+#pragma unroll 1
+      for (int i = x0 + lane; i < x1; i += 32) {
+        const int tc = i - x0 + KX;
+        const size_t o = (size_t)j * nnx + i;
+        if (j > 0 && j < nny - 1) {
+          phi64[o] = z[tc];
+          if (i == 0) phi64[o + W] = z[tc];
         }
-        const float f = __double2float_rn(z[k]);
+        const float f = to_float(z[tc]);
         a.phi[o] = f;
-        if (col0) a.phi[o + W] = f;
+        if (i == 0) a.phi[o + W] = f;
         if (J.do_field) {
           double ex = 0.0, ey;
           if (j == 0) {
-            ey = (z[k] - z[k + 128]) / d1;
+            ey = over(z[tc] - z[tc + tp], d1, i1);
           } else if (j == nny - 1) {
-            ey = (z[k - 128] - z[k]) / d1;
+            ey = over(z[tc - tp] - z[tc], d1, i1);
           } else {
-            ex = ((k == 0 ? z[wc] : z[k - 1]) - east(z, k)) / d2;
-            ey = (z[k - 128] - z[k + 128]) / d2;
+            const double wv = z[MODE != kHalo && tc == 0 ? W - 1 : tc - 1], ev = z[MODE != kHalo && tc == W - 1 ? 0 : tc + 1];
+            ex = over(wv - ev, d2, i2);
+            ey = over(z[tc - tp] - z[tc + tp], d2, i2);
           }
-          const float2 E = make_float2(__double2float_rn(ex), __double2float_rn(ey));
+          const float2 E = make_float2(to_float(ex), to_float(ey));
           a.E[o] = E;
-          if (col0) a.E[o + W] = E;
+          if (i == 0) a.E[o + W] = E;
         }
       }
-    };
-    __syncthreads();
-#pragma unroll 1
-    for (int r = 0; r < R; ++r)
-      if ((g.ownrows >> r) & 1u) put64(g.row0 + r, q64 + r * 128, false);
-    if (!idle && south_edge && by == 0) put64(0, p64 + 4 * li, true);
-    if (!idle && north_edge && by == nby - 1) put64(nny - 1, p64 + (hi - lo + 2) * 128 + 4 * li, true);
+    }
     __syncthreads();
     if (tid == 0) {
       __threadfence();
@@ -796,65 +906,30 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       if (start + nsw == J.max_sweeps) mask |= 1u << (nsw - 1);
       if (mask && early) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) snap[((nq & 1) * R + r) * nthr + tid] = x[r];
+        for (int r = 0; r < R; ++r) snap[((G > 1 ? nq & 1 : 0) * R + r) * nthr + tid] = x[r];
       }
     }
-    // smem places of the rows below and above the strip (read) and of its
-    // first and last rows (written), this sweep's (A) and the next one's (B)
-    const float *sA = south_edge ? edge + es * 256 + 4 * li : last + p * par + soff;
-    const float *nA = north_edge || idle ? edge + es * 256 + 128 + 4 * li : first + p * par + noff;
-    const float *sB = south_edge ? sA : last + (p ^ 1) * par + soff;
-    const float *nB = north_edge || idle ? nA : first + (p ^ 1) * par + noff;
-    float *wA = first + p * par + mine, *wB = first + (p ^ 1) * par + mine;
-    const int tolast = 2 * par;
-    // the rest of a sweep: the strip's first and last rows to shared memory
-    auto next = [&]() {
-      sts4(wB, x[0]);
-      sts4(wB + tolast, x[R - 1]);
-      const float *t = sA;
-      sA = sB;
-      sB = t;
-      t = nA;
-      nA = nB;
-      nB = t;
-      float *w = wA;
-      wA = wB;
-      wB = w;
-      __syncthreads();
-    };
+    Rows at = rows_at(es, p);
     auto note = [&](float md, int m) {
-      const unsigned u = __reduce_max_sync(kFull, __float_as_uint(md));
+      const unsigned u = __reduce_max_sync(kFull, __float_as_uint(quarter(md)));
       if (lane == m) keep = u;
     };
     int m = 0;
-    if (start == 0) {
-      note(sweep<R, MODE, false, true, true>(x, b, lds4(sA), lds4(nA), g, J.phi_zero ? nullptr : phi + W, nnx), 0);
-      next();
+    if (seam && start == 0) {  // the first sweep reads the caller's mirror column
+      note(sweep<R, MODE, false, true, true>(x, b, lds4(at.sA), lds4(at.nA), g, mcol + (g.row0 - lo)), 0);
+      sts4(at.wB, x[0]);
+      sts4(at.wB + at.to_last, x[R - 1]);
+      __syncthreads();
+      at = rows_at(es, p ^ 1);
       m = 1;
     }
     const int plain = mask >> m ? m + __ffs(mask >> m) - 1 : nsw;  // sweeps before the next checked one
     if (g.full) {
-#pragma unroll 2
-      for (; m < plain; ++m) {
-        sweep<R, MODE, true, false, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0);
-        next();
-      }
-#pragma unroll 1
-      for (; m < nsw; ++m) {
-        note(sweep<R, MODE, true, true, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0), m);
-        next();
-      }
+      sweeps<R, MODE, true, false>(x, b, g, at, m, plain, note);
+      sweeps<R, MODE, true, true>(x, b, g, at, m, nsw, note);
     } else {
-#pragma unroll 2
-      for (; m < plain; ++m) {
-        sweep<R, MODE, false, false, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0);
-        next();
-      }
-#pragma unroll 1
-      for (; m < nsw; ++m) {
-        note(sweep<R, MODE, false, true, false>(x, b, lds4(sA), lds4(nA), g, nullptr, 0), m);
-        next();
-      }
+      sweeps<R, MODE, false, false>(x, b, g, at, m, plain, note);
+      sweeps<R, MODE, false, true>(x, b, g, at, m, nsw, note);
     }
     p ^= nsw & 1;
     done += nsw;
@@ -898,7 +973,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
         resv = __shfl_sync(kFull, v, k);
         if (warp == 0) js->cm[(nq + 2) & 3][lane] = 0u;
         ++nq;
-        if (pass) stop_at(start, k, (nq - 1) & 1, es0);
+        if (pass) stop_at(start, k, 0, es0);
       } else {
         if (warp == 0) {
           if ((mask >> lane) & 1u)
@@ -918,77 +993,61 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     }
   }
 
-  // ---- results ---------------------------------------------------------
+  // ---- results: the image with its edge rows, then row by row phi and
+  // E = -grad phi (mesh.cu:413-468) of the owned nodes ----------------------
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    if (!((g.ownrows >> r) & 1u)) continue;
-    float *const q = phi + (size_t)(g.row0 + r) * nnx + g.i0;
-    if (g.own & 1u) q[0] = x[r].x;
-    if (g.own & 2u) q[1] = x[r].y;
-    if (g.own & 4u) q[2] = x[r].z;
-    if (g.own & 8u) q[3] = x[r].w;
-    if (g.i0 == 0 && (g.own & 1u)) q[W] = x[r].x;
+  for (int r = 0; r < R; ++r)
+    if (r < g.nvalid) sts4(timg + (g.row0 - lo + r) * tp + 4 * li, quarter(x[r]));
+  for (int k = tid; k < 2 * tp; k += nthr) {
+    const int up = k >= tp ? 1 : 0, tc = k - up * tp;
+    timg0[up * (rows + 1) * tp + tc] = quarter(edge[es * 256 + up * 128 + tc]);
   }
-  if (J.do_field) {  // E = -grad phi (mesh.cu:413-468)
-    const float4 s4 = lds4(south_edge ? edge + es * 256 + 4 * li : last + p * par + soff);
-    const float4 n4 = lds4(north_edge || idle ? edge + es * 256 + 128 + 4 * li : first + p * par + noff);
-    float4 prev = s4;
-    auto put = [&](int j, int q, float wv, float ev, float nv, float sv) {
-      if ((g.own >> q) & 1u)
-        a.E[(size_t)j * nnx + g.i0 + q] =
-            make_float2(__fdiv_rn(__fsub_rn(wv, ev), a.two_ds), __fdiv_rn(__fsub_rn(sv, nv), a.two_ds));
-    };
-    auto rim = [&](int j, const float4 &hi_, const float4 &lo_, float mhi, float mlo) {  // a Dirichlet row
-      float2 *const q = a.E + (size_t)j * nnx + g.i0;
-      if (g.own & 1u) q[0] = make_float2(0.0f, __fdiv_rn(__fsub_rn(hi_.x, lo_.x), a.ds));
-      if (g.own & 2u) q[1] = make_float2(0.0f, __fdiv_rn(__fsub_rn(hi_.y, lo_.y), a.ds));
-      if (g.own & 4u) q[2] = make_float2(0.0f, __fdiv_rn(__fsub_rn(hi_.z, lo_.z), a.ds));
-      if (g.own & 8u) q[3] = make_float2(0.0f, __fdiv_rn(__fsub_rn(hi_.w, lo_.w), a.ds));
-      if (g.i0 == 0 && (g.own & 1u)) q[W] = make_float2(0.0f, __fdiv_rn(__fsub_rn(mhi, mlo), a.ds));
-    };
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const float4 c = x[r];
-      float lf, rt;
-      float4 ev = make_float4(c.y, c.z, c.w, 0.0f);
-      if (MODE == kHalo) {
-        lf = __shfl_up_sync(kFull, c.w, 1);
-        rt = __shfl_down_sync(kFull, c.x, 1);
-      } else {
-        const float lastv = g.rm == 0 ? c.w : (g.rm == 1 ? c.x : (g.rm == 2 ? c.y : c.z));
-        lf = __shfl_sync(kFull, lastv, g.srcw);
-        rt = __shfl_sync(kFull, c.x, g.srce);
-        ev.x = g.rm == 1 ? rt : ev.x;
-        ev.y = g.rm == 2 ? rt : ev.y;
-        ev.z = g.rm == 3 ? rt : ev.z;
-      }
-      ev.w = rt;
-      const float4 nx = r + 1 < R ? x[r + 1 < R ? r + 1 : r] : n4;
-      const float4 n = r + 1 >= g.nvalid ? n4 : nx;
-      if ((g.ownrows >> r) & 1u) {
-        const int j = g.row0 + r;
-        put(j, 0, lf, ev.x, n.x, prev.x);
-        put(j, 1, c.x, ev.y, n.y, prev.y);
-        put(j, 2, c.y, ev.z, n.z, prev.z);
-        put(j, 3, c.z, ev.w, n.w, prev.w);
-        const bool col0 = g.i0 == 0 && (g.own & 1u);
-        if (col0) {  // the mirror column; the Dirichlet rows keep their own value there
-          const float sv = j == 1 ? phi[W] : prev.x, nv = j == nny - 2 ? phi[(size_t)(nny - 1) * nnx + W] : n.x;
-          a.E[(size_t)j * nnx + W] =
-              make_float2(__fdiv_rn(__fsub_rn(lf, ev.x), a.two_ds), __fdiv_rn(__fsub_rn(sv, nv), a.two_ds));
+  __syncthreads();
+  // a quotient by a power of two is the product by its inverse, exactly
+  const bool pow2 = (__float_as_uint(a.ds) & 0x7fffffu) == 0u;
+  const float inv1 = __fdiv_rn(1.0f, a.ds), inv2 = __fdiv_rn(1.0f, a.two_ds);
+  auto over = [&](float v, float d, float i) { return pow2 ? __fmul_rn(v, i) : __fdiv_rn(v, d); };
+#pragma unroll 1
+  for (int j = r0 + warp; j < r1; j += nwarp) {
+    const float *const z = timg + (j - lo) * tp + KX - x0;
+    float *const pr = phi + (size_t)j * nnx;
+    float2 *const er = a.E + (size_t)j * nnx;
+#pragma unroll 2
+    for (int i = x0 + lane; i < x1; i += 32) {
+      const float *const q = z + i;
+      pr[i] = q[0];
+      if (i == 0) pr[W] = q[0];
+      if (J.do_field) {
+        const float wv = q[MODE != kHalo && i == 0 ? W - 1 : -1], ev = q[MODE != kHalo && i == W - 1 ? 1 - W : 1];
+        const float2 E =
+            make_float2(over(__fsub_rn(wv, ev), a.two_ds, inv2), over(__fsub_rn(q[-tp], q[tp]), a.two_ds, inv2));
+        er[i] = E;
+        if (i == 0) {
+          // beside a Dirichlet row, whose mirror column keeps its own value
+          const float sv = j == 1 ? phi[W] : q[-tp], nv = j == nny - 2 ? phi[(size_t)(nny - 1) * nnx + W] : q[tp];
+          er[W] = make_float2(E.x, over(__fsub_rn(sv, nv), a.two_ds, inv2));
         }
-        if (j == 1) rim(0, prev, c, col0 ? phi[W] : 0.0f, c.x);
-        if (j == nny - 2) rim(nny - 1, c, n, c.x, col0 ? phi[(size_t)(nny - 1) * nnx + W] : 0.0f);
       }
-      prev = c;
     }
   }
+  if (J.do_field)
+    for (int side = 0; side < 2; ++side) {  // the Dirichlet rows
+      if (side == 0 ? by > 0 : by < nby - 1) continue;
+      const int j = side == 0 ? 0 : nny - 1;
+      const float *const z = side == 0 ? timg : timg + (rows - 1) * tp;  // the row beside it
+      for (int i = x0 + tid; i < x1 + (x0 == 0 ? 1 : 0); i += nthr) {
+        const int ii = i < x1 ? i : W;  // the mirror column goes with column 0
+        const float d = phi[(size_t)j * nnx + ii], v = z[(i < x1 ? i : 0) - x0 + KX];
+        a.E[(size_t)j * nnx + ii] =
+            make_float2(0.0f, side == 0 ? over(__fsub_rn(d, v), a.ds, inv1) : over(__fsub_rn(v, d), a.ds, inv1));
+      }
+    }
   // the last CTA to finish also writes the report
-  __syncthreads();
+  if (G > 1) __syncthreads();
   if (tid == 0) {
-    __threadfence();
-    if (atomicAdd(&ctl->jdone, 1u) == (unsigned)G - 1u) {
-      __threadfence();
+    if (G > 1) __threadfence();
+    if (G == 1 || atomicAdd(&ctl->jdone, 1u) == (unsigned)G - 1u) {
+      if (G > 1) __threadfence();
       ctl->jdone = 0u;
       if (J.write_stats) {
         ctl->sweeps = done;
@@ -1002,7 +1061,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
 }
 
 template <int R, int MODE, bool REFINE>
-__global__ void __launch_bounds__(512, 1) k_tile(SimArgs a, JacobiArgs J) {
+__global__ void __launch_bounds__(32 * kTileWarps, 1) k_tile(SimArgs a, JacobiArgs J) {
   extern __shared__ __align__(16) float tsm[];
   __shared__ Scratch js;
   if (threadIdx.x == 0) js.bail = 0;
@@ -1012,7 +1071,7 @@ __global__ void __launch_bounds__(512, 1) k_tile(SimArgs a, JacobiArgs J) {
 
 using Kernel = void (*)(SimArgs, JacobiArgs);
 
-// the kernel of MODE with strips of r rows (1..8)
+// the kernel of MODE with strips of r rows (1..kTileRows)
 template <int MODE, bool REFINE>
 inline Kernel pick(int r) {
   switch (r) {
