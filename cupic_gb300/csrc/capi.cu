@@ -570,7 +570,7 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
     cands.push_back(t);
     words = std::max(words, t.words);
     maxG = std::max(maxG, t.G);
-    if ((int)cands.size() >= (getenv("CUPIC_TILE_TRIALS") ? atoi(getenv("CUPIC_TILE_TRIALS")) : kTileTrials)) break;
+    if ((int)cands.size() >= kTileTrials) break;
   }
   if (cands.empty()) return CUPIC_ERR_CAPACITY;
   TilePlan pick = cands.front();
@@ -596,9 +596,6 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
         float ms = 0.0f;
         if (ok && rep > 0 && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess) ms_best = std::min(ms_best, ms);
       }
-      if (getenv("CUPIC_TILE_VERBOSE"))
-        fprintf(stderr, "tile %dx%d: nbx %d nby %d K %d R %d warps %d mode %d: %.1f us (cost %.0f)\n", c->a.nnx, c->a.nny,
-                t.nbx, t.nby, t.K, t.R, t.warps, t.mode, 1e3 * ms_best, t.cost);
       if (!ok) {
         cudaGetLastError();
         continue;

@@ -27,12 +27,12 @@
 //
 // What bounds it: the latency of a sweep on a small tile (350 cycles with one
 // row a thread: barrier, shared-memory rows, shuffles) and instruction issue
-// on a large one (18 a row and warp), plus the exchange (2900 cycles with two
-// neighbours, 5500-7300 with eight) every K sweeps.  Against the
+// on a large one (14 a row and warp), plus the exchange (2900 cycles with two
+// neighbours, 5000-6500 with eight) every K sweeps.  Against the
 // shared-memory sweep and register strips of jacobi.cu, 200 sweeps in a step:
-// 512x2048 0.334 -> 0.182 ms, 256x1024 0.191 -> 0.115, 301x700 (rows of no
-// multiple of 4) 0.325 -> 0.110, 32x128 0.127 -> 0.052 ms; with a check after
-// each of 2000 sweeps, 64x256 5.0 -> 0.95 ms.
+// 512x2048 0.334 -> 0.163 ms, 256x1024 0.191 -> 0.104, 301x700 (rows of no
+// multiple of 4) 0.325 -> 0.102, 32x128 0.127 -> 0.050 ms; with a check after
+// each of 2000 sweeps, 64x256 5.0 -> 0.85 ms.
 #pragma once
 
 #include <math.h>
@@ -143,7 +143,7 @@ __device__ __forceinline__ void copy8(void *to, const void *from) {
 // A warp's FP64 operation holds the SM's FP64 pipe for about 24 cycles, so the
 // correction's conversions and its product by 4 go through the integer pipe:
 // the same bits (round to nearest even), with the hardware's conversion for
-// what is not normal on both sides.  A 512x2048 correction: 57.1 -> 55.6 us.
+// what is not normal on both sides.
 static __device__ __noinline__ float to_float_slow(double v) { return __double2float_rn(v); }
 static __device__ __noinline__ double to_double_slow(float v) { return (double)v; }
 static __device__ __noinline__ double times4_slow(double v) { return 4.0 * v; }
@@ -627,9 +627,10 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   // sweeps run and is looked at before the correction is added; a solve that
   // had already passed its test drops it.  Same operations, same order, same
   // bits as one launch per residual, solve and update.  Bound by the FP64
-  // pipe (27 us of a 512x2048 correction's 55.6: six operations a node of the
-  // tile) and the sweeps with their exchanges; a launch per correction, with
-  // a grid barrier and every residual's potential read again, took 96 us.
+  // pipe (six operations a node of the tile) and the sweeps with their
+  // exchanges: a 512x2048 correction of 32 sweeps takes 52 us; a launch per
+  // correction, with a grid barrier and every residual's potential read
+  // again, took 96.
   if constexpr (REFINE) {
     double *const p64 = reinterpret_cast<double *>(ptable + J.ppairs);  // rows lo-1 .. hi+1, [tp]
     double *const q64 = p64 + (g.row0 - lo + 1) * tp + 4 * li;          // this strip's first row
@@ -655,10 +656,6 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     // the columns west and east of this lane's, relative to them
     const int wc = MODE == kHalo ? (li == 0 ? 0 : -1) : (li == 0 ? W - 1 : -1);
     const int ring0 = -4 * li;  // column 0 of a ring
-    auto east = [&](const double *p, int q) {
-      if (MODE != kHalo && g.me == q) return p[ring0];
-      return p[q + 1];
-    };
     const int m_ = J.max_sweeps;  // sweeps of a correction
     const unsigned long long inf64 = 0x7ff0000000000000ull;
     int e = 0, es = 0, p = 0, done = 0, q = 0;
@@ -686,11 +683,26 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
         if (r < g.nvalid) {
           const double *const z = q64 + r * tp;
           const double *const src = J.r64_b + (size_t)(g.row0 + r) * nnx;
+          // the strip's columns in 16-byte loads
+          auto row4 = [](const double *q, double (&d)[4]) {
+            const double2 u = *reinterpret_cast<const double2 *>(q), v_ = *reinterpret_cast<const double2 *>(q + 2);
+            d[0] = u.x;
+            d[1] = u.y;
+            d[2] = v_.x;
+            d[3] = v_.y;
+          };
+          double zc[4], zn[4], zs[4];
+          row4(z, zc);
+          row4(z + tp, zn);
+          row4(z - tp, zs);
+          const double zw = z[wc], ze = z[MODE != kHalo && g.me == 3 ? ring0 : 4], z0 = MODE == kRingRagged ? z[ring0] : 0.0;
           float v[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            const double rr = (cc[k] >= 0 ? src[cc[k]] : 0.0) -
-                              (times4(z[k]) - ((((k == 0 ? z[wc] : z[k - 1]) + east(z, k)) + z[k + tp]) + z[k - tp]));
+            const double wv = k == 0 ? zw : zc[k > 0 ? k - 1 : 0];
+            double ev = k == 3 ? ze : zc[k < 3 ? k + 1 : 3];
+            if (MODE == kRingRagged && g.me == k) ev = z0;
+            const double rr = (cc[k] >= 0 ? src[cc[k]] : 0.0) - (times4(zc[k]) - (((wv + ev) + zn[k]) + zs[k]));
             v[k] = to_float(rr);
             const unsigned long long bits = (unsigned long long)__double_as_longlong(rr) & 0x7fffffffffffffffull;
             if (((g.own >> k) & 1u) && ((g.ownrows >> r) & 1u) && bits <= inf64 && bits > mx) mx = bits;
@@ -764,10 +776,13 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
         if (done >= J.r64_mn && res < J.r64_tol && !J.trial) break;
       }
       auto add_row = [&](double *z, const float4 &d) {
-        z[0] += to_double(d.x);
-        z[1] += to_double(d.y);
-        z[2] += to_double(d.z);
-        z[3] += to_double(d.w);
+        double2 u = *reinterpret_cast<double2 *>(z), v = *reinterpret_cast<double2 *>(z + 2);
+        u.x += to_double(d.x);
+        u.y += to_double(d.y);
+        v.x += to_double(d.z);
+        v.y += to_double(d.w);
+        *reinterpret_cast<double2 *>(z) = u;
+        *reinterpret_cast<double2 *>(z + 2) = v;
       };
 #pragma unroll
       for (int r = 0; r < R; ++r)
