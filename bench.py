@@ -29,6 +29,7 @@ divides by the slowest rank's time.
 """
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -41,21 +42,21 @@ sys.path.insert(0, ROOT)
 METRIC = "particle-steps/s full PIC cycle"
 UNIT = "particle-steps/s"
 STATS_BYTES = 96
-# kernels launched per step: jacobi (which also clears the next charge),
-# push, room check, arrive, inject sched/gen/append, finalize
-KERNELS_PER_STEP = 8
+# kernels launched per step: solve (which also clears the next charge), push,
+# inject sched and gen, and the step's end (room check, arrivals, append,
+# bookkeeping)
+KERNELS_PER_STEP = 5
+FEW_DRAWS = 128  # draws per step and species up to which sched and gen are one kernel
 
 
 def kernels_per_step(p):
-    """Kernels one step launches.  The precision form replaces the solve by
-    the FP64 source, one Jacobi launch per correction up to the sweep cap
-    (each with the residual, the stop test and the update fused in; the
-    ones after the stop test return at once), a last test launch and the
-    field; its step also clears the next charge with its own kernel."""
-    if p.refine_every <= 0:
-        return KERNELS_PER_STEP
-    corrections = -(-max(p.max_sweeps, 0) // p.refine_every)
-    return (KERNELS_PER_STEP - 1) + 1 + 1 + corrections + 1 + 1
+    """Kernels one step launches.  The precision form adds the FP64 source
+    (its corrections, stop tests, FP32 potential and field are in the
+    solve's launch)."""
+    n = KERNELS_PER_STEP + (1 if p.refine_every > 0 else 0)
+    flux = [p.n * p.ds * p.ncx * p.ds * math.sqrt(kt / m) / math.sqrt(2.0 * math.pi)
+            for m, kt in ((p.me, p.kte), (p.mi, p.kti))]
+    return n - 1 if max(flux) * p.dt <= FEW_DRAWS else n
 
 # algorithmic bytes per unit of work (FP32 SoA, 16 B state per particle)
 PUSH_BYTES_PER_PARTICLE = 32      # 16 B read + 16 B write

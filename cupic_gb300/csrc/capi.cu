@@ -895,6 +895,13 @@ int enqueue_after_solve(cupic_ctx *c, bool zeroed, const cudaEvent_t *marks = nu
   CU(launch_push_deposit(c->a, c->stream));
   CU(mark(2));
   CU(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+  if (tail_applies(c->a)) {
+    CU(launch_tail(c->a, c->num_sms, c->stream));
+    CU(mark(3));
+    CU(mark(4));
+    CU(mark(5));
+    return CUPIC_OK;
+  }
   CU(launch_room(c->a, c->stream));
   CU(launch_arrive(c->a, c->stream));
   CU(mark(3));

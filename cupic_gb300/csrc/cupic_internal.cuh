@@ -41,7 +41,7 @@ struct Ctl {
   uint32_t idle;          // never written: the bounded-wait self-test waits on it
   int32_t refine_done;    // precision-form solve: the stop test passed, later corrections idle
   uint32_t jdone;         // CTAs of the running solve that have finished (the last one resets it)
-  uint32_t pad;
+  uint32_t tail_done;     // of the two CTAs that end a step, those that are done (the later resets it)
   cupic_step_stats ring[kStatsRing];
 };
 

@@ -673,6 +673,35 @@ __device__ __forceinline__ void arrive_row(const SimArgs &a, const int d, const 
 
 __global__ void k_arrive(SimArgs a) { arrive_row(a, blockIdx.x, blockIdx.y); }
 
+// the same by one warp; inj: particles that the append adds to the row
+__device__ __forceinline__ void arrive_warp(const SimArgs &a, const int d, const int sp, const int lane, const int inj = 0) {
+  const SpeciesDev &S = a.sp[sp];
+  const int ns = S.nstay[d];
+  const int nb = d > 0 ? S.nup[d - 1] : 0;
+  const int na = d + 1 < a.ncy ? S.ndown[d + 1] : 0;
+  const int capd = S.cap[d];
+  float4 *row = S.parts + S.seg[d];
+  auto copy = [&](const float4 *from, int n, int at) {
+    constexpr int kU = 4;  // loads of a lane in flight
+    const int m = min(n, capd - at);
+    for (int k = lane; k < m; k += 32 * kU) {
+      float4 v[kU];
+#pragma unroll
+      for (int u = 0; u < kU; ++u) v[u] = from[min(k + 32 * u, m - 1)];
+#pragma unroll
+      for (int u = 0; u < kU; ++u)
+        if (k + 32 * u < m) row[at + k + 32 * u] = v[u];
+    }
+  };
+  copy(S.stage_up + (size_t)max(d - 1, 0) * S.stage_cap, nb, ns);
+  copy(S.stage_down + (size_t)(d + 1) * S.stage_cap, na, ns + nb);
+  if (lane == 0) {
+    const int tot = ns + nb + na;
+    if (tot > capd) raise_flags(a.ctl, CUPIC_FLAG_CAPACITY);
+    S.cnt[d] = min(tot + inj, capd);
+  }
+}
+
 // many contexts: one warp per (row, species) task t = 2 * work index +
 // species, eight per block -- most rows of a batch move few particles, so a
 // block per row would be mostly set-up
@@ -684,28 +713,7 @@ __global__ void __launch_bounds__(32 * kArriveWarps)
   const int2 w = work[t >> 1];
   const SimArgs &a = inst[w.x];
   if (halted(a.ctl)) return;
-  const int d = w.y, sp = t & 1;
-  const SpeciesDev &S = a.sp[sp];
-  const int ns = S.nstay[d];
-  const int nb = d > 0 ? S.nup[d - 1] : 0;
-  const int na = d + 1 < a.ncy ? S.ndown[d + 1] : 0;
-  const int capd = S.cap[d];
-  float4 *row = S.parts + S.seg[d];
-  if (nb) {
-    const float4 *up = S.stage_up + (size_t)(d - 1) * S.stage_cap;
-    for (int k = lane; k < nb; k += 32)
-      if (ns + k < capd) row[ns + k] = up[k];
-  }
-  if (na) {
-    const float4 *dn = S.stage_down + (size_t)(d + 1) * S.stage_cap;
-    for (int k = lane; k < na; k += 32)
-      if (ns + nb + k < capd) row[ns + nb + k] = dn[k];
-  }
-  if (lane == 0) {
-    const int tot = ns + nb + na;
-    if (tot > capd) raise_flags(a.ctl, CUPIC_FLAG_CAPACITY);
-    S.cnt[d] = min(tot, capd);
-  }
+  arrive_warp(a, w.y, t & 1, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -812,11 +820,9 @@ __global__ void k_inject_sched_batch(const SimArgs *__restrict__ inst, int n) {
   if (t < 2 * n) inject_sched(inst[t >> 1], t & 1);
 }
 
-__device__ __forceinline__ void inject_gen(const SimArgs &a, const int sp, const int k) {
+// draw k of species sp, injected at time tin
+__device__ __forceinline__ void inject_one(const SimArgs &a, const int sp, const int k, const double tin) {
   const Ctl *ctl = a.ctl;
-  if (halted(ctl)) return;
-  const int ne = ctl->inj_gen[sp];
-  if (k >= ne) return;
   const SpeciesDev &S = a.sp[sp];
   const double t = ctl->t, fpt = t + a.dt_d, fvt = t + 0.5 * a.dt_d;
   const double sig = a.sig[sp], qm = a.qm[sp];
@@ -835,7 +841,6 @@ __device__ __forceinline__ void inject_gen(const SimArgs &a, const int sp, const
   const float2 e0 = a.E[top + ic], e1 = a.E[top + ic + 1];
   const double epx = (1.0 - fx) * (double)e0.x + fx * (double)e1.x;
   const double epy = (1.0 - fx) * (double)e0.y + fx * (double)e1.y;
-  const double tin = S.inj_tin[k];
   const double dp = fpt - tin, dv = fvt - tin;
   x = x + dp * vx;
   const double y = a.Ly_d + dp * vy;
@@ -849,6 +854,44 @@ __device__ __forceinline__ void inject_gen(const SimArgs &a, const int sp, const
   S.inj_d[k] = c.dest;
 }
 
+__device__ __forceinline__ void inject_gen(const SimArgs &a, const int sp, const int k) {
+  if (halted(a.ctl)) return;
+  if (k < a.ctl->inj_gen[sp]) inject_one(a, sp, k, a.sp[sp].inj_tin[k]);
+}
+
+// Schedule and draws of a few particles a step in one launch, a block per
+// species: every thread accumulates its own draw's time, one dtin at a time
+// as the schedule does.  Behind the schedule's launch the draws of a 32x128
+// mesh held up the step 7 us longer than the push beside them.
+constexpr int kDrawBlock = 128;
+__global__ void __launch_bounds__(kDrawBlock) k_inject_few(SimArgs a) {
+  Ctl *ctl = a.ctl;
+  if (halted(ctl)) return;
+  const int sp = blockIdx.x;
+  const SpeciesDev &S = a.sp[sp];
+  const double dtin = a.dtin[sp], t = ctl->t, fpt = t + a.dt_d;
+  const double tin0 = ctl->tin_set[sp] ? ctl->tin[sp] : t + dtin;
+  int in = 0;
+  if (tin0 < fpt) in = 1 + (int)((fpt - tin0) / dtin);
+  const int ne = in < S.inj_cap ? in : S.inj_cap;
+  __syncthreads();  // every thread has read the clocks
+  if (threadIdx.x == 0) {
+    double tin = tin0;
+    for (int k = 0; k < in; ++k) tin += dtin;
+    ctl->tin[sp] = tin;
+    ctl->tin_set[sp] = 1;
+    ctl->inj_count[sp] = in;
+    ctl->inj_gen[sp] = ne;
+    if (in > ne) atomicOr(&ctl->step_flags, (uint32_t)CUPIC_FLAG_CAPACITY);
+  }
+  double tin = tin0;
+  int done = 0;
+  for (int k = threadIdx.x; k < ne; k += kDrawBlock) {
+    for (; done < k; ++done) tin += dtin;
+    inject_one(a, sp, k, tin);
+  }
+}
+
 __global__ void k_inject_gen(SimArgs a) {
   inject_gen(a, blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -858,23 +901,26 @@ __global__ void k_inject_gen_batch(const SimArgs *__restrict__ inst) {
   inject_gen(inst[blockIdx.z], blockIdx.y, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// TAIL (k_tail): running is zero, a row's count is what it will hold when the
+// arrivals are in, and the counts are kept by others
+template <int NT, bool TAIL = false>
 __device__ __forceinline__ void inject_append(const SimArgs &a, const int sp, int *running) {
   // running: [ncy] injected per destination row
-  constexpr int NW = kInjBlock / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const SpeciesDev &S = a.sp[sp];
   Ctl *ctl = a.ctl;
-  if (halted(ctl)) return;
+  if (!TAIL && halted(ctl)) return;
   __shared__ unsigned s_rem;
   if (tid == 0) s_rem = 0;
-  for (int k = tid; k < a.ncy; k += kInjBlock) running[k] = 0;
+  if (!TAIL)
+    for (int k = tid; k < a.ncy; k += NT) running[k] = 0;
   __syncthreads();
   const int ne = ctl->inj_gen[sp];
   const long long q = sp == 0 ? -1 : 1;
   unsigned long long *rho_next = a.rho[ctl->cur ^ 1];
   uint32_t fl = 0;
   unsigned nrem = 0;
-  for (int base = 0; base < ne; base += kInjBlock) {
+  for (int base = 0; base < ne; base += NT) {
     const int k = base + tid;
     int d = kRowRemoved;
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -889,7 +935,8 @@ __device__ __forceinline__ void inject_append(const SimArgs &a, const int sp, in
     const int leader = __ffs(grp) - 1;
     const int rank = __popc(grp & ((1u << lane) - 1u));
     int basev = 0;
-    for (int w = 0; w < NW; ++w) {
+    const int nw = (min(ne - base, NT) + 31) / 32;  // warps with draws
+    for (int w = 0; w < nw; ++w) {
       if (warp == w && d >= 0 && lane == leader) {
         basev = running[d];
         running[d] = basev + __popc(grp);
@@ -898,7 +945,10 @@ __device__ __forceinline__ void inject_append(const SimArgs &a, const int sp, in
     }
     const int b0 = __shfl_sync(kFull, basev, leader);
     if (d >= 0) {
-      const int pos = S.cnt[d] + b0 + rank;
+      const int have = TAIL ? S.nstay[d] + (d > 0 ? S.nup[d > 0 ? d - 1 : 0] : 0) +
+                                  (d + 1 < a.ncy ? S.ndown[d + 1 < a.ncy ? d + 1 : d] : 0)
+                            : S.cnt[d];
+      const int pos = have + b0 + rank;
       if (pos < S.cap[d]) {
         S.parts[S.seg[d] + pos] = p;
         const CicFixed c = cic_fixed(a, p.x, p.y);
@@ -916,26 +966,71 @@ __device__ __forceinline__ void inject_append(const SimArgs &a, const int sp, in
   if (lane == 0 && wr) atomicAdd(&s_rem, wr);
   fl = __reduce_or_sync(kFull, fl);
   if (lane == 0) raise_flags(ctl, fl);
+  if (TAIL) return;
   __syncthreads();
-  for (int k = tid; k < a.ncy; k += kInjBlock)
+  for (int k = tid; k < a.ncy; k += NT)
     if (running[k]) S.cnt[k] = min(S.cnt[k] + running[k], S.cap[k]);
   if (tid == 0 && s_rem) atomicAdd(&ctl->removed[sp], (unsigned long long)s_rem);
 }
 
 __global__ void __launch_bounds__(kInjBlock) k_inject_append(SimArgs a) {
   extern __shared__ int running[];
-  inject_append(a, blockIdx.x, running);
+  inject_append<kInjBlock>(a, blockIdx.x, running);
 }
 
 // grid (species, instance)
 __global__ void __launch_bounds__(kInjBlock) k_inject_append_batch(const SimArgs *__restrict__ inst) {
   extern __shared__ int running[];
-  inject_append(inst[blockIdx.y], blockIdx.x, running);
+  inject_append<kInjBlock>(inst[blockIdx.y], blockIdx.x, running);
 }
 
 // ---------------------------------------------------------------------------
 // end of step: stats ring entry, clocks, charge buffer flip
 // ---------------------------------------------------------------------------
+// one thread: live particles, and injected ones beyond the domain that the
+// append did not count
+__device__ __forceinline__ void end_step(const SimArgs &a, unsigned long long live0, unsigned long long live1,
+                                         unsigned rem0, unsigned rem1) {
+  Ctl *ctl = a.ctl;
+  // every field is read before the first store: the ring entry lies in
+  // the same block, so interleaved loads and stores would each wait for
+  // the one before (one L2 round trip per field)
+  const int64_t step = ctl->step;
+  const double t = ctl->t;
+  const unsigned long long ab0 = ctl->absorbed[0], ab1 = ctl->absorbed[1];
+  const unsigned long long rm0 = ctl->removed[0] + rem0, rm1 = ctl->removed[1] + rem1;
+  const int32_t in0 = ctl->inj_count[0], in1 = ctl->inj_count[1];
+  const int32_t sweeps = ctl->sweeps;
+  const float residual = ctl->residual;
+  const uint32_t sfl = ctl->step_flags, fl = ctl->flags;
+  const int32_t cur = ctl->cur;
+  cupic_step_stats st{};
+  st.step = step;
+  st.t = t;
+  st.absorbed[0] = (int64_t)ab0;
+  st.absorbed[1] = (int64_t)ab1;
+  st.removed[0] = (int64_t)rm0;
+  st.removed[1] = (int64_t)rm1;
+  st.injected[0] = in0;
+  st.injected[1] = in1;
+  st.live[0] = (int64_t)live0;
+  st.live[1] = (int64_t)live1;
+  st.sweeps = sweeps;
+  st.residual = residual;
+  st.flags = sfl;
+  ctl->ring[step % kStatsRing] = st;
+  for (int sp = 0; sp < 2; ++sp) {
+    ctl->absorbed[sp] = 0ull;
+    ctl->removed[sp] = 0ull;
+    ctl->inj_count[sp] = 0;
+  }
+  ctl->flags = fl | sfl;
+  ctl->step_flags = 0u;
+  ctl->t = t + a.dt_d;
+  ctl->step = step + 1;
+  ctl->cur = cur ^ 1;
+}
+
 __device__ __forceinline__ void finalize(const SimArgs &a) {
   Ctl *ctl = a.ctl;
   if (halted(ctl)) {  // the host completes the halted step and reruns the ones counted here
@@ -961,48 +1056,93 @@ __device__ __forceinline__ void finalize(const SimArgs &a) {
     atomicAdd(&live[1], v1);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    // every field is read before the first store: the ring entry lies in
-    // the same block, so interleaved loads and stores would each wait for
-    // the one before (one L2 round trip per field)
-    const int64_t step = ctl->step;
-    const double t = ctl->t;
-    const unsigned long long ab0 = ctl->absorbed[0], ab1 = ctl->absorbed[1];
-    const unsigned long long rm0 = ctl->removed[0], rm1 = ctl->removed[1];
-    const int32_t in0 = ctl->inj_count[0], in1 = ctl->inj_count[1];
-    const int32_t sweeps = ctl->sweeps;
-    const float residual = ctl->residual;
-    const uint32_t sfl = ctl->step_flags, fl = ctl->flags;
-    const int32_t cur = ctl->cur;
-    cupic_step_stats st{};
-    st.step = step;
-    st.t = t;
-    st.absorbed[0] = (int64_t)ab0;
-    st.absorbed[1] = (int64_t)ab1;
-    st.removed[0] = (int64_t)rm0;
-    st.removed[1] = (int64_t)rm1;
-    st.injected[0] = in0;
-    st.injected[1] = in1;
-    st.live[0] = (int64_t)live[0];
-    st.live[1] = (int64_t)live[1];
-    st.sweeps = sweeps;
-    st.residual = residual;
-    st.flags = sfl;
-    ctl->ring[step % kStatsRing] = st;
-    for (int sp = 0; sp < 2; ++sp) {
-      ctl->absorbed[sp] = 0ull;
-      ctl->removed[sp] = 0ull;
-      ctl->inj_count[sp] = 0;
-    }
-    ctl->flags = fl | sfl;
-    ctl->step_flags = 0u;
-    ctl->t = t + a.dt_d;
-    ctl->step = step + 1;
-    ctl->cur = cur ^ 1;
-  }
+  if (threadIdx.x == 0) end_step(a, live[0], live[1], 0u, 0u);
 }
 
 __global__ void k_finalize(SimArgs a) { finalize(a); }
+
+// ---------------------------------------------------------------------------
+// The end of a step in one launch: room check, arrivals, append and
+// bookkeeping, which four launches did one after another (32x128: 20 us of
+// the step, each a chain of L2 round trips).  Every CTA makes the room check
+// for itself from what the push and the draws left, so no CTA waits for
+// another: a warp to a (row, species) copies the arrivals, two CTAs append one
+// species' draws each (their places follow from the row counts), and the
+// later of these two does the bookkeeping with the totals of its own check.
+// ---------------------------------------------------------------------------
+constexpr int kTailBlock = 512;
+__global__ void __launch_bounds__(kTailBlock, 2) k_tail(SimArgs a) {
+  extern __shared__ int tail_rows[];  // draws per row of both species [2][ncy], append's running counts [ncy]
+  __shared__ unsigned long long s_live[2];
+  __shared__ unsigned s_rem[2];
+  __shared__ int s_last;
+  Ctl *ctl = a.ctl;
+  const int tid = threadIdx.x, lane = tid & 31, ncy = a.ncy, rank = blockIdx.x;
+  // the row this warp copies first: its counts come with the control words
+  const int nw = kTailBlock / 32, t0 = (rank - 2) * nw + (tid >> 5), tstep = ((int)gridDim.x - 2) * nw;
+  const bool halt = halted(ctl);
+  const int ne[2] = {ctl->inj_gen[0], ctl->inj_gen[1]};
+  for (int k = tid; k < 3 * ncy; k += kTailBlock) tail_rows[k] = 0;
+  if (tid < 2) {
+    s_live[tid] = 0ull;
+    s_rem[tid] = 0u;
+  }
+  if (halt) {  // as finalize(): the host reruns the steps counted here
+    if (rank == 0 && tid == 0) ctl->skipped += 1;
+    return;
+  }
+  __syncthreads();
+  for (int sp = 0; sp < 2; ++sp)
+    for (int k = tid; k < ne[sp]; k += kTailBlock) {
+      const int d = a.sp[sp].inj_d[k];
+      if (d >= 0 && d < ncy)
+        atomicAdd(&tail_rows[sp * ncy + d], 1);
+      else if (d < 0)
+        atomicAdd(&s_rem[sp], 1u);
+    }
+  __syncthreads();
+  int over = 0;
+  unsigned long long live[2] = {0ull, 0ull};
+  for (int d = tid; d < ncy; d += kTailBlock)
+#pragma unroll
+    for (int sp = 0; sp < 2; ++sp) {
+      const SpeciesDev &S = a.sp[sp];
+      const int up = S.nup[d > 0 ? d - 1 : 0], dn = S.ndown[d + 1 < ncy ? d + 1 : d];
+      const long long need = (long long)S.nstay[d] + (d > 0 ? up : 0) + (d + 1 < ncy ? dn : 0) + tail_rows[sp * ncy + d];
+      over |= need > (long long)S.cap[d];
+      live[sp] += (unsigned long long)need;
+    }
+  if (__syncthreads_or(over)) {
+    // every CTA finds the same; one that reads the flag first returns above
+    if (rank == 0 && tid == 0) {
+      ctl->skipped += 1;
+      atomicExch(&ctl->halt, 1);
+    }
+    return;
+  }
+  if (rank >= 2) {
+    for (int t = t0; t < 2 * ncy; t += tstep) arrive_warp(a, t >> 1, t & 1, lane, tail_rows[(t & 1) * ncy + (t >> 1)]);
+    return;
+  }
+  for (int o = 16; o > 0; o >>= 1)
+    for (int sp = 0; sp < 2; ++sp) live[sp] += __shfl_down_sync(kFull, live[sp], o);
+  if (lane == 0) {
+    atomicAdd(&s_live[0], live[0]);
+    atomicAdd(&s_live[1], live[1]);
+  }
+  inject_append<kTailBlock, true>(a, rank, tail_rows + 2 * ncy);
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(&ctl->tail_done, 1u) == 1u;
+  }
+  __syncthreads();
+  if (s_last && tid == 0) {
+    __threadfence();
+    ctl->tail_done = 0u;
+    end_step(a, s_live[0], s_live[1], s_rem[0], s_rem[1]);
+  }
+}
 
 __global__ void k_finalize_batch(const SimArgs *__restrict__ inst) { finalize(inst[blockIdx.x]); }
 
@@ -1099,11 +1239,25 @@ cudaError_t launch_arrive(const SimArgs &a, cudaStream_t st) {
 // The draws depend only on the clocks and the step's field, so a step can
 // run them beside the push; the append needs the push's row counts.
 cudaError_t launch_inject_draw(const SimArgs &a, cudaStream_t st) {
+  if (a.dt_d <= kDrawBlock * a.dtin[0] && a.dt_d <= kDrawBlock * a.dtin[1]) {
+    k_inject_few<<<2, kDrawBlock, 0, st>>>(a);
+    return cudaGetLastError();
+  }
   const int cap = max(a.sp[0].inj_cap, a.sp[1].inj_cap);
   k_inject_sched<<<1, 32, 0, st>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   k_inject_gen<<<dim3((cap + 127) / 128, 2), 128, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+// The step's end in one launch, where a CTA's shared memory holds the counts of
+// all rows; a warp for every (row, species), two CTAs to an SM at most.
+bool tail_applies(const SimArgs &a) { return 3 * a.ncy * sizeof(int) <= 48 * 1024; }
+
+cudaError_t launch_tail(const SimArgs &a, int num_sms, cudaStream_t st) {
+  const int nw = kTailBlock / 32, ctas = min(2 + (2 * a.ncy + nw - 1) / nw, 2 * num_sms);
+  k_tail<<<max(ctas, 3), kTailBlock, 3 * a.ncy * sizeof(int), st>>>(a);
   return cudaGetLastError();
 }
 
