@@ -90,8 +90,9 @@ struct JacobiArgs {
   int32_t G;              // CTAs (cooperative)
   // register tiles (tile.cuh): rows of a strip (0: the shared-memory sweep of
   // jacobi.cu), tile mode, blocks in x and y (G = nbx * nby), lanes of a
-  // strip, strips per warp, warps, exchange row pitch in words
-  int32_t tile, mode, nbx, nby, nl, segs, warps, ip;
+  // strip, strips per warp, warps, exchange row pitch in words, and whether the
+  // CTAs are one cluster that trades through shared memory
+  int32_t tile, mode, nbx, nby, nl, segs, warps, ip, near;
   int32_t trows, tpairs, ppairs;  // rows of the exchange image, entries of the tables of words in and out
   uint32_t pwords;        // exchange words of one parity
   int32_t trial;          // 1: a timing run, checked but never stopped

@@ -99,7 +99,10 @@ bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, 
   t.ip = nbx == 1 ? 4 * W4 : 4 * W4 + 36;
   const size_t thr = 32 * (size_t)t.warps;
   t.trows = rows;
-  if (t.G > 1) {
+  t.near = nbx == 1 && nby > 1 && nby <= kTileCluster;
+  if (t.near) {
+    t.tpairs = 2 * K * 4 * t.nl;  // the rows that arrive, two exchanges in turn
+  } else if (t.G > 1) {
     const int wide = nbx > 1 ? 4 * ((W4 + nbx - 1) / nbx) + 2 * K : W;
     const int own = nbx > 1 ? 4 * ((W4 + nbx - 1) / nbx) : W, side = nbx > 1 ? t.B * K : 0;
     t.tpairs = ((nby > 1 ? 2 : 0) * K * ((wide + 1) / 2) + side + 1) / 2 * 2;
@@ -116,20 +119,28 @@ bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, 
            (size_t)(t.tpairs + t.ppairs) * sizeof(uint2) + (form == kTileEarly ? 2 * R * thr * sizeof(float4) : 0) +
            (form == kTileFixed ? (size_t)rows * 4 * t.nl * sizeof(long long) : 0) +
            (form == kTileRefine ? ((size_t)(rows + 2) * 4 * t.nl + 8) * sizeof(double) : 0);
-  t.words = t.G == 1 ? 0
+  t.words = t.G == 1 || t.near ? 0
                      : (size_t)2 * nby * 2 * K * t.ip + (nbx > 1 ? (size_t)2 * nny * nbx * 2 * K : 0);
   if (t.words >= 1ull << 31) return false;
-  // Estimated SM cycles per sweep, from timings at 2 GHz: 270 of latency (the
-  // barrier, the shuffles, the two rows a warp takes and sends through shared
-  // memory) and 14 issue slots a row for each warp of a scheduler (more above
-  // 5 rows, where registers run short); an exchange takes 2000 cycles, 1700
-  // more with eight neighbours instead of two, and 700 for each pair of words
-  // a thread waits for, shared by the K sweeps between two of them.
+  // Estimated SM cycles per sweep, fitted to the times of 2900 layouts of 12
+  // meshes (33x129 .. 513x2049, 200 sweeps, at 2 GHz; the cheapest estimate is
+  // within 8% of the fastest layout timed on all but two of them): the
+  // barrier and the two rows that every warp takes and sends through shared
+  // memory, 16 issue slots a row for each warp of a scheduler (more above 5
+  // rows, where registers run short, and for the selects of a ragged ring),
+  // the stop test, and the share of an exchange: 640 cycles in a cluster,
+  // 1160 by way of L2, more for each warp that issues it and for each pair of
+  // words a thread waits for.
   // Measured slower, 512x2048, 200 sweeps: strips of 12 rows on 8 warps of 255
   // registers (half the rows through shared memory) 188 us against 170; two
   // CTAs to an SM, one sweeping while the other waits, 239 against 175.
-  t.cost = 270.0 + ((t.warps + 3) / 4) * 14.0 * t.R * (t.R <= 5 ? 1.0 : 1.0 + 0.12 * (t.R - 5));
-  if (t.G > 1) t.cost += (2000.0 + (nbx > 1 ? 1700.0 : 0.0) + 700.0 * t.tpairs / thr) / K;
+  const double per = (t.warps + 3) / 4 * R;  // rows of a scheduler
+  t.cost = 55.0 * R + 5.0 * t.warps + per * (16.0 + 6.5 * std::max(0, R - 5) + (t.mode == 2 ? 30.0 : 0.0));
+  if (form == kTileEarly) t.cost += 127.0 + 3.0 * t.warps + (t.near ? 500.0 / K : 0.0);
+  if (t.near)
+    t.cost += (640.0 + 52.0 * t.warps) / K;
+  else if (t.G > 1)
+    t.cost += (1160.0 + 130.0 * t.warps + 240.0 * t.tpairs / thr) / K;
   // the precision form's FP64 work: about 9 operations a node at 2 a clock,
   // once a correction (32 sweeps)
   if (form == kTileRefine) t.cost += 4.5 * 4 * 32 * R * t.warps / 32;
@@ -172,33 +183,55 @@ void tile_args(const TilePlan &t, JacobiArgs *J) {
   J->segs = t.segs;
   J->warps = t.warps;
   J->ip = t.ip;
+  J->near = t.near;
   J->trows = t.trows;
   J->tpairs = t.tpairs;
   J->ppairs = t.ppairs;
   J->pwords = (uint32_t)(t.words / 2);
 }
 
+// the launch of a layout: a cluster, or a cooperative grid where CTAs wait for
+// one another without one
+static void tile_launch(const TilePlan &t, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr) {
+  cfg->gridDim = dim3(t.G);
+  cfg->blockDim = dim3(32 * t.warps);
+  cfg->dynamicSmemBytes = t.smem;
+  if (t.near) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = t.G;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  } else {
+    attr->id = cudaLaunchAttributeCooperative;
+    attr->val.cooperative = 1;
+  }
+  cfg->attrs = attr;
+  cfg->numAttrs = t.G > 1 ? 1 : 0;
+}
+
 // CTAs of this layout that the device holds at once
 cudaError_t tile_max_ctas(const TilePlan &t, int num_sms, int *ctas) {
   const void *fn = tile_kernel(t);
   cudaError_t e = raise_dyn_smem(fn, t.smem);
-  int per_sm = 0;
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * t.warps, t.smem);
-  *ctas = per_sm * num_sms;
+  int n = 0;
+  if (e == cudaSuccess && t.near) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    tile_launch(t, &cfg, attr);
+    if (t.G > 8) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, fn, &cfg);
+    *ctas = n * t.G;
+  } else {
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, 32 * t.warps, t.smem);
+    *ctas = n * num_sms;
+  }
   return e;
 }
 
 cudaError_t launch_tile(const SimArgs &a, const JacobiArgs &J, const TilePlan &t, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(t.G);
-  cfg.blockDim = dim3(32 * t.warps);
-  cfg.dynamicSmemBytes = t.smem;
-  cfg.stream = st;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = t.G > 1 ? 1 : 0;
+  tile_launch(t, &cfg, attr);
+  cfg.stream = st;
   SimArgs sa = a;
   JacobiArgs ja = J;
   void *args[] = {&sa, &ja};

@@ -14,25 +14,27 @@
 //   nbx > 1 (halo)    K (a multiple of 4) halo columns on each side, updated
 //                     redundantly like the halo rows, so no lane needs more
 //                     than its two neighbours, for every W.
-// Every K sweeps the blocks trade the K nodes inside each boundary as 64-bit
-// words {value, epoch} (one L2 round trip, no flag and no fence), written
-// from and read into registers.  Every value is computed with the same
-// operands in the same order on every layout, so all layouts give the same
-// bits.
+// Every K sweeps the blocks trade the K nodes inside each boundary.  Rings of
+// up to kTileCluster CTAs are one cluster: a row's columns go from registers
+// into the neighbour's shared memory, whose barrier counts their bytes.  Other
+// grids trade by way of L2, as 64-bit words {value, epoch} (one round trip, no
+// flag and no fence).  Every value is computed with the same operands in the
+// same order on every layout, so all layouts give the same bits.
 //
 // Convergence checks never wait in the sweep loop: the maxima of a block of
 // K sweeps are combined over the grid while the next block runs, and when
 // a sweep turns out to have passed the stop test the state at the start of
 // its block (kept in shared memory) is restored and swept up to it.
 //
-// What bounds it: the latency of a sweep on a small tile (350 cycles with one
-// row a thread: barrier, shared-memory rows, shuffles) and instruction issue
-// on a large one (14 a row and warp), plus the exchange (2900 cycles with two
-// neighbours, 5000-6500 with eight) every K sweeps.  Against the
+// What bounds it: the latency of a sweep on a small tile (170 cycles with one
+// row a thread on 8 warps, 280 on 15: barrier, shared-memory rows, shuffles)
+// and instruction issue on a large one (16 a row and warp), plus the exchange
+// every K sweeps (1000 cycles in a cluster, 3000-5000 by way of L2, where the
+// instructions of 16 warps weigh as much as the round trip).  Against the
 // shared-memory sweep and register strips of jacobi.cu, 200 sweeps in a step:
-// 512x2048 0.334 -> 0.163 ms, 256x1024 0.191 -> 0.104, 301x700 (rows of no
-// multiple of 4) 0.325 -> 0.102, 32x128 0.127 -> 0.050 ms; with a check after
-// each of 2000 sweeps, 64x256 5.0 -> 0.85 ms.
+// 512x2048 0.334 -> 0.163 ms, 256x1024 0.191 -> 0.093, 301x700 (rows of no
+// multiple of 4) 0.325 -> 0.096, 32x128 0.127 -> 0.039; with a check after
+// each of 2000 sweeps, 64x256 5.0 -> 0.61 ms.
 #pragma once
 
 #include <math.h>
@@ -75,8 +77,47 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
   return v;
 }
 
+// Rings of a cluster: a row's columns go straight into the neighbour's shared
+// memory, whose barrier counts the bytes.
+__device__ __forceinline__ unsigned cluster_addr(unsigned addr, int rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_cluster(unsigned to, const float4 &v, unsigned bar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
+      "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ bool cluster_wait(unsigned bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0u;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_join() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ float4 lds4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 __device__ __forceinline__ void sts4(float *p, const float4 &v) { *reinterpret_cast<float4 *>(p) = v; }
+
+// Waits: look() until it is true for every lane.  The lanes leave a wait
+// together, by a vote, so that the warp is whole when it comes to the block's
+// next barrier.  False if the wait gave up or another CTA did.
+template <class Look>
+__device__ __forceinline__ bool wait_for(const Ctl *ctl, Look &&look) {
+  for (long long it = 0;; ++it) {
+    if (__all_sync(kFull, look())) return true;
+    if ((it & 255) == 255) {
+      const bool quit = it >= kSpinLimit || *(const volatile int *)&ctl->abort;
+      if (__any_sync(kFull, quit)) return false;
+    }
+  }
+}
 
 // static shared scratch
 struct Scratch {
@@ -84,6 +125,7 @@ struct Scratch {
   int dec[2];          // a block's stop decision: index of the stopping sweep, or -1
   float decv[2];       // its residual
   int bail;
+  uint64_t arrived[2];  // a cluster's exchanges, odd and even ones
   unsigned long long w64[16], res64[2];  // a correction's max |r| per warp, and over the grid
 };
 
@@ -238,15 +280,22 @@ struct Rows {
 // Sweeps m .. end-1 of a block.  (Measured slower: the strip's outer rows
 // first, an mbarrier arrival and the rows between while the others catch
 // up, 100 cycles more a sweep; the same order with __syncthreads, no gain.)
-template <int R, int MODE, bool FULL, bool CHECK, class Note>
+// CHECK: a sweep's maximum goes through the warp's reduction while the next
+// sweep waits for its rows, and to the lane of its number in keep after that;
+// md holds the last one's (reduced before the stores and the barrier, it
+// added 260 cycles to a sweep).
+template <int R, int MODE, bool FULL, bool CHECK>
 __device__ __forceinline__ void sweeps(float4 (&x)[R], const float4 (&b)[R], const Lane &g, Rows &w, int &m, int end,
-                                       Note &&note) {
+                                       float &md, unsigned &keep) {
 #pragma unroll 2
   for (; m < end; ++m) {
-    const float md = sweep<R, MODE, FULL, CHECK, false>(x, b, lds4(w.sA), lds4(w.nA), g, nullptr);
-    if (CHECK) note(md, m);
+    const float4 s4 = lds4(w.sA), n4 = lds4(w.nA);
+    unsigned v = 0u;
+    if (CHECK) v = __reduce_max_sync(kFull, __float_as_uint(md));
+    md = sweep<R, MODE, FULL, CHECK, false>(x, b, s4, n4, g, nullptr);
     sts4(w.wB, x[0]);
-    sts4(w.wB + w.to_last, x[R - 1]);
+    if (R > 1) sts4(w.wB + w.to_last, x[R - 1]);
+    if (CHECK && (int)(threadIdx.x & 31) == m - 1) keep = v;
     const float *t = w.sA;
     w.sA = w.sB;
     w.sB = t;
@@ -269,6 +318,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   const int cur = *reinterpret_cast<volatile int *>(&ctl->cur);
   const unsigned ebase = *reinterpret_cast<volatile unsigned *>(&ctl->jepoch);
   if (halt) return;
+  const bool near = MODE != kHalo && J.near;
   const int G = J.G, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
   const int nnx = a.nnx, nny = a.nny, W = nnx - 1, M = nny - 2;
   const int nbx = MODE == kHalo ? J.nbx : 1, nby = J.nby;
@@ -286,6 +336,16 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   const int lo = nby > 1 ? max(1, r0 - (K - 1)) : 1, hi = nby > 1 ? min(nny - 2, r1 + K - 2) : nny - 2;
   // lane -> strip
   const int nl = J.nl, segs = J.segs;
+  const uint32_t near_bytes = ((by > 0 ? 1 : 0) + (by < nby - 1 ? 1 : 0)) * 16u * K * nl;
+  if (near) {
+    if (tid == 0) {
+      for (int k = 0; k < 2; ++k) mbar_init(&js->arrived[k], 1);
+      fence_mbar_init();
+      for (int k = 0; k < 2; ++k) mbar_arrive_expect_tx(&js->arrived[k], near_bytes);
+    }
+    __syncwarp();
+    cluster_arrive();
+  }
   const int seg = segs == 1 ? 0 : lane / nl, li = segs == 1 ? lane : lane - seg * nl;
   const bool act = segs == 1 ? lane < nl : seg < segs;
   Lane g;
@@ -312,7 +372,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   // edge rows of 4 blocks of sweeps in turn, then (below) the received halo
   // nodes, the table of halo words and two snapshots of the strips
   const int par = nthr * 4;
-  float *const first = sm, *const last = sm + 2 * par;
+  float *const first = sm, *const last = R > 1 ? sm + 2 * par : sm;  // one row is both
   float *const edge = sm + 4 * par;  // [4][south, north][128]
   const int mine = tid * 4;
   const int soff = seg > 0 ? mine - 4 * nl : (warp - 1) * 128 + 4 * ((segs - 1) * nl + li);
@@ -420,10 +480,12 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       }
   } else {
     for (int k = tid; k < 4 * 2 * 128; k += nthr) edge[k] = 0.0f;
+    for (int k = tid; k < (rows + 2) * tp; k += nthr) timg0[k] = 0.0f;
     clear_next();
   }
   sts4(first + mine, x[0]);
-  sts4(last + mine, x[R - 1]);
+  if (R > 1) sts4(last + mine, x[R - 1]);
+  if (near) cluster_join();
 
   // exchange words, two parities of: rows [by][bottom, top][K][ip] by
   // extended column, then (halo tiles) columns [row][bx][left, right][K]
@@ -450,7 +512,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   const int per = ((im0 ? 1 : 0) + (im1 ? 1 : 0)) * ni;
   const int nside = MODE == kHalo ? h * K : 0;
   const int nout = G > 1 ? plow + phigh + nside + per * ((by > 0 ? K : 0) + (by < nby - 1 ? K : 0)) : 0;
-  if (G > 1) {
+  if (G > 1 && !near) {
 #pragma unroll 1
     for (int t = warp; t < 2 * K; t += nwarp) {  // row t of the bottom (t < K) and top boundaries
       const bool low = t < K;
@@ -511,8 +573,9 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     const unsigned ep = ebase + (unsigned)e;
     unsigned long long *const hw = J.halo + ((e & 1) ? pwords : 0u);
 #pragma unroll 4
-    for (int u = tid; u < nout; u += nthr) {
-      const uint2 t = ptable[u];
+    for (int v0 = tid - lane; v0 < nout; v0 += nthr) {  // the same for a warp's lanes
+      if (v0 + lane >= nout) continue;
+      const uint2 t = ptable[v0 + lane];
       const float *from = timg + (t.y & ~kOne);
       if (t.y & kOne)
         st_word(hw + t.x, from[0], ep);
@@ -520,20 +583,14 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
         st_word2(hw + t.x, from[0], from[1], ep);
     }
   };
-  // elements of this lane beside the owned columns
-  unsigned need_side = 0u;
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int i = g.i0 + q;
-    if (MODE == kHalo && act && ((i < x0 && i >= x0 - KX) || (i >= x1 && i < x1 + KX))) need_side |= 1u << q;
-  }
   // waits for the words of exchange e and puts them in shared memory; false
   // if the wait gave up
   auto receive = [&](int e, int to_edge) -> bool {
     const unsigned ep = ebase + (unsigned)e;
     const unsigned long long *const hw = J.halo + ((e & 1) ? pwords : 0u);
     constexpr int NB = 4;  // pairs of a thread in flight
-    for (int u0 = tid; u0 < npair; u0 += NB * nthr) {
+    for (int v0 = tid - lane; v0 < npair; v0 += NB * nthr) {  // the same for a warp's lanes
+      const int u0 = min(v0 + lane, npair - 1);
       uint2 t[NB];
       unsigned long long w[NB][2];
 #pragma unroll
@@ -545,21 +602,20 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       // Wait on the first pair alone: the others come from the same blocks, and
       // polling all of them loads L2 while the blocks are still writing
       // (512x2048, depth 8: 0.79 us a sweep against 0.74).
-      for (long long it = 0;; ++it) {
-        ld_word2(hw + t[0].x, w[0][0], w[0][1]);
-        if (here(0)) break;
-        if (it >= kSpinLimit || ((it & 255) == 255 && *(volatile int *)&ctl->abort)) return false;
-      }
-      for (long long it = 0;; ++it) {
-        bool all = true;
+      if (!wait_for(ctl, [&]() {
+            ld_word2(hw + t[0].x, w[0][0], w[0][1]);
+            return here(0);
+          }))
+        return false;
+      if (!wait_for(ctl, [&]() {
+            bool all = true;
 #pragma unroll
-        for (int q = 1; q < NB; ++q)
-          ld_word2(hw + t[q].x, w[q][0], w[q][1]);
+            for (int q = 1; q < NB; ++q) ld_word2(hw + t[q].x, w[q][0], w[q][1]);
 #pragma unroll
-        for (int q = 1; q < NB; ++q) all = all && here(q);
-        if (all) break;
-        if (it >= kSpinLimit || ((it & 255) == 255 && *(volatile int *)&ctl->abort)) return false;
-      }
+            for (int q = 1; q < NB; ++q) all = all && here(q);
+            return all;
+          }))
+        return false;
 #pragma unroll
       for (int q = 0; q < NB; ++q) {
         float *to = (t[q].y & kEdge) ? edge + to_edge * 256 : timg;
@@ -570,22 +626,72 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     }
     return true;
   };
-  // this thread's halo nodes from shared memory
+  // this thread's rows with halo nodes from the image, which holds the owned
+  // nodes beside them as well (show)
+  unsigned inrows = 0u;
+  const bool beside = MODE == kHalo && act && g.own != 15u && g.i0 < x1 + KX;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (r < g.nvalid && (beside || !((g.ownrows >> r) & 1u))) inrows |= 1u << r;
   auto take = [&]() {
     const float *const img = timg + (g.row0 - lo) * tp + 4 * li;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (r >= g.nvalid) continue;
-      if (!((g.ownrows >> r) & 1u)) {
-        x[r] = lds4(img + r * tp);
-      } else if (MODE == kHalo && need_side) {
-        const float4 v = lds4(img + r * tp);
-        x[r].x = (need_side & 1u) ? v.x : x[r].x;
-        x[r].y = (need_side & 2u) ? v.y : x[r].y;
-        x[r].z = (need_side & 4u) ? v.z : x[r].z;
-        x[r].w = (need_side & 8u) ? v.w : x[r].w;
-      }
+    for (int r = 0; r < R; ++r)
+      if ((inrows >> r) & 1u) x[r] = lds4(img + r * tp);
+  };
+  // The same exchange inside a cluster: the rows [2][bottom, top][K][tp] that
+  // the neighbours write, in place of the tables.  A neighbour sends exchange
+  // e+2 once it has exchange e+1 of this CTA, which takes e before that.
+  float *const got = reinterpret_cast<float *>(table);
+  const bool dn = by > 0, up = by < nby - 1;
+  const unsigned gpar = 8u * K * tp;  // bytes of one exchange's rows
+  // where this strip's first row goes and comes from, and its rows (bits 0-7:
+  // to the block below, 8-15: above; 16-23: those from above in a strip that
+  // also has rows from below)
+  const unsigned dto = near ? cluster_addr(smem_addr(got), max(by - 1, 0)) + 16u * li + 4u * (K + g.row0 - r0) * tp : 0u;
+  const unsigned uto =
+      near ? cluster_addr(smem_addr(got), min(by + 1, nby - 1)) + 16u * li + 4u * (K + g.row0 - r1) * tp : 0u;
+  const float *const zin = got + 4 * li + (K + g.row0 - (g.row0 < r0 ? r0 : r1)) * tp;
+  unsigned trades = 0u;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int j = g.row0 + r;
+    if ((outrows >> r) & 1u) {
+      if (dn && j < r0 + K) trades |= 1u << r;
+      if (up && j >= r1 - K) trades |= 0x100u << r;
     }
+    if (j >= r1 && g.row0 < r0) trades |= 0x10000u << r;
+  }
+  const bool eslow = !idle && south_edge && dn, eshigh = !idle && north_edge && up;
+  auto send = [&](int e) {
+    const unsigned o = (e & 1) ? gpar : 0u;
+    const unsigned bar = smem_addr(&js->arrived[e & 1]);
+    if (trades & 0xffu) {
+      const unsigned nb = cluster_addr(bar, by - 1);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if ((trades >> r) & 1u) st_cluster(dto + o + 4u * r * tp, x[r], nb);
+    }
+    if (trades & 0xff00u) {
+      const unsigned nb = cluster_addr(bar, by + 1);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if ((trades >> (8 + r)) & 1u) st_cluster(uto + o + 4u * r * tp, x[r], nb);
+    }
+  };
+  auto await = [&](int e) -> bool {
+    const unsigned bar = smem_addr(&js->arrived[e & 1]), parity = ((unsigned)(e - 1) >> 1) & 1u;
+    if (!wait_for(ctl, [&]() { return cluster_wait(bar, parity); })) return false;
+    if (tid == 0) mbar_arrive_expect_tx(&js->arrived[e & 1], near_bytes);  // for exchange e+2
+    return true;
+  };
+  auto take_rows = [&](int e, int to_edge) {
+    const int o = (e & 1) ? 2 * K * tp : 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if ((inrows >> r) & 1u) x[r] = lds4(zin + o + (r - ((trades >> (16 + r)) & 1u ? h : 0)) * tp);
+    if (eslow) sts4(edge + to_edge * 256 + 4 * li, lds4(got + o + 4 * li));
+    if (eshigh) sts4(edge + to_edge * 256 + 128 + 4 * li, lds4(got + o + (2 * K - 1) * tp + 4 * li));
   };
   auto fail = [&]() {
     js->bail = 1;
@@ -593,6 +699,31 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       atomicExch(&ctl->abort, 1);
       atomicOr(&ctl->step_flags, (uint32_t)CUPIC_FLAG_TIMEOUT);
     }
+  };
+
+  // an exchange up to the arrival of the neighbours' nodes, and (after a
+  // barrier, outside a cluster) their way into the strips; between() reads
+  // what the grid has found while the nodes are on their way
+  auto trade_out = [&](int &e, int &es, auto &&between) {
+    ++e;
+    es = (es + 1) & 3;
+    if (near) {
+      send(e);
+      between();
+      if (!await(e)) fail();
+    } else {
+      show();
+      __syncthreads();
+      publish(e);
+      between();
+      if (!receive(e, es)) fail();
+    }
+  };
+  auto trade_in = [&](int e, int es) {
+    if (near)
+      take_rows(e, es);
+    else
+      take();
   };
 
   auto rows_at = [&](int es_, int p_) {
@@ -663,17 +794,11 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     __syncthreads();
     // the grid's maximum of correction n (warp 0)
     auto wait_res = [&](int n) {
-      if (lane == 0) {
-        bool ok = true;
-        const unsigned target = (unsigned)G * ((unsigned)n / 4u + 1u);
-        for (long long it = 0; ld_acquire(&J.tbar[n & 3]) < target; ++it)
-          if (it >= kSpinLimit || ((it & 255) == 255 && *(volatile int *)&ctl->abort)) {
-            ok = false;
-            break;
-          }
-        js->res64[n & 1] = ld_word(&J.gmax[n & 3]);
-        if (!ok) fail();
-      }
+      const unsigned target = (unsigned)G * ((unsigned)n / 4u + 1u);
+      const bool ok = wait_for(ctl, [&]() { return ld_acquire(&J.tbar[n & 3]) >= target; });
+      const unsigned long long most = ld_word(&J.gmax[n & 3]);
+      if (lane == 0) js->res64[n & 1] = most;
+      if (!ok) fail();
     };
     for (;;) {
       unsigned long long mx = 0ull;
@@ -732,7 +857,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       }
       // the correction starts from zero
       sts4(first + p * par + mine, x[0]);
-      sts4(last + p * par + mine, x[R - 1]);
+      if (R > 1) sts4(last + p * par + mine, x[R - 1]);
       if (!idle && south_edge) sts4(edge + es * 256 + 4 * li, x[0]);
       if (!idle && north_edge) sts4(edge + es * 256 + 128 + 4 * li, x[0]);
       __syncthreads();
@@ -745,27 +870,24 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       for (int sw = 0; sw < todo;) {
         const int nsw = G > 1 ? min(K, todo - sw) : todo;
         Rows at = rows_at(es, p);
-        auto none = [](float, int) {};
         int m = 0;
+        float md = 0.0f;
+        unsigned keep = 0u;
         if (g.full)
-          sweeps<R, MODE, true, false>(x, b, g, at, m, nsw, none);
+          sweeps<R, MODE, true, false>(x, b, g, at, m, nsw, md, keep);
         else
-          sweeps<R, MODE, false, false>(x, b, g, at, m, nsw, none);
+          sweeps<R, MODE, false, false>(x, b, g, at, m, nsw, md, keep);
         p ^= nsw & 1;
         sw += nsw;
         if (G > 1) {  // also after the last sweep: the halo's correction is added too
-          ++e;
-          show();
-          __syncthreads();
-          publish(e);
-          es = (es + 1) & 3;
-          if (!receive(e, es)) fail();
-          if (sw >= todo && warp == 0) wait_res(q);
-          __syncthreads();
-          take();
+          trade_out(e, es, [&]() {
+            if (sw >= todo && warp == 0) wait_res(q);
+          });
+          if (!near) __syncthreads();
+          trade_in(e, es);
           p ^= 1;
           sts4(first + p * par + mine, x[0]);
-          sts4(last + p * par + mine, x[R - 1]);
+          if (R > 1) sts4(last + p * par + mine, x[R - 1]);
           __syncthreads();
           if (js->bail) break;
         }
@@ -866,15 +988,8 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   // the stop decision on checked block q, taken by warp 0 once every CTA's
   // maxima are in (usually long before it asks)
   auto decide = [&](int q, unsigned mask) {
-    bool ok = true;
     const unsigned target = (unsigned)G * ((unsigned)q / 4u + 1u);
-    if (lane == 0)
-      for (long long it = 0; ld_acquire(&J.tbar[q & 3]) < target; ++it)
-        if (it >= kSpinLimit || ((it & 255) == 255 && *(volatile int *)&ctl->abort)) {
-          ok = false;
-          break;
-        }
-    ok = __shfl_sync(kFull, ok, 0);
+    const bool ok = wait_for(ctl, [&]() { return ld_acquire(&J.tbar[q & 3]) >= target; });
     const bool mineck = (mask >> lane) & 1u;
     const float v = mineck ? __uint_as_float((unsigned)ld_word(&J.gmax[(q & 3) * 32 + lane])) : 0.0f;
     const unsigned pass = __ballot_sync(kFull, mineck && (double)v < J.tol && !J.trial);
@@ -895,9 +1010,10 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     maxs = start + k + 1;
     checks = false;
     sts4(first + p * par + mine, x[0]);
-    sts4(last + p * par + mine, x[R - 1]);
+    if (R > 1) sts4(last + p * par + mine, x[R - 1]);
     __syncthreads();
   };
+  const bool owns = __any_sync(kFull, g.ownrows != 0u);
   for (int k = tid; k < 128; k += nthr) js->cm[k >> 5][k & 31] = 0u;
   __syncthreads();
   for (;;) {
@@ -912,12 +1028,46 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       if (k < 0) break;
       stop_at(pstart, k, (nq - 1) & 1, pes);
     }
+    // Whole blocks without a checked sweep, and not the last ones: what the
+    // general path below decides costs some 600 cycles a block (512x2048, depth
+    // 8: 0.72 -> 0.62 us a sweep; 256x1024, depth 4: 0.69 -> 0.56).
+    if (G > 1 && !pend && !(seam && done == 0)) {
+      int next = maxs;  // the next checked or last sweep
+      if (checks && early) {
+        const unsigned s = (unsigned)max(done + 1, J.min_sweeps), ev = (unsigned)J.check_every;
+        next = (int)min((unsigned)next, ev == 1u ? s : (s + ev - 1u) / ev * ev);
+      }
+      for (int n = (next - 1 - done) / K; n > 0; --n) {
+        Rows at = rows_at(es, p);
+        int m = 0;
+        float md = 0.0f;
+        unsigned keep = 0u;
+        if (g.full)
+          sweeps<R, MODE, true, false>(x, b, g, at, m, K, md, keep);
+        else
+          sweeps<R, MODE, false, false>(x, b, g, at, m, K, md, keep);
+        p ^= (K & 1) ^ 1;
+        done += K;
+        trade_out(e, es, []() {});
+        if (!near) __syncthreads();
+        trade_in(e, es);
+        sts4(first + p * par + mine, x[0]);
+        if (R > 1) sts4(last + p * par + mine, x[R - 1]);
+        __syncthreads();
+        if (js->bail) break;
+      }
+      if (js->bail) break;
+    }
     const int nsw = min(KB, maxs - done), start = done, es0 = es;
     unsigned mask = 0u, keep = 0u;
     if (checks) {
-      if (early)
+      if (early && J.check_every == 1) {
+        const int s = max(J.min_sweeps - start - 1, 0);
+        if (s < nsw) mask = (kFull >> (32 - nsw)) & (kFull << s);
+      } else if (early) {
         for (int s = (start / J.check_every + 1) * J.check_every; s <= start + nsw; s += J.check_every)
           if (s >= J.min_sweeps) mask |= 1u << (s - start - 1);
+      }
       if (start + nsw == J.max_sweeps) mask |= 1u << (nsw - 1);
       if (mask && early) {
 #pragma unroll
@@ -925,49 +1075,51 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       }
     }
     Rows at = rows_at(es, p);
-    auto note = [&](float md, int m) {
-      const unsigned u = __reduce_max_sync(kFull, __float_as_uint(quarter(md)));
-      if (lane == m) keep = u;
-    };
     int m = 0;
+    float md = 0.0f;  // four times a sweep's maximum
     if (seam && start == 0) {  // the first sweep reads the caller's mirror column
-      note(sweep<R, MODE, false, true, true>(x, b, lds4(at.sA), lds4(at.nA), g, mcol + (g.row0 - lo)), 0);
+      md = sweep<R, MODE, false, true, true>(x, b, lds4(at.sA), lds4(at.nA), g, mcol + (g.row0 - lo));
+      const unsigned u = __reduce_max_sync(kFull, __float_as_uint(md));
+      if (lane == 0) keep = u;
       sts4(at.wB, x[0]);
-      sts4(at.wB + at.to_last, x[R - 1]);
+      if (R > 1) sts4(at.wB + at.to_last, x[R - 1]);
       __syncthreads();
       at = rows_at(es, p ^ 1);
       m = 1;
     }
-    const int plain = mask >> m ? m + __ffs(mask >> m) - 1 : nsw;  // sweeps before the next checked one
+    // sweeps before the next checked one; rows of a halo alone are not looked at
+    const int plain = mask >> m && owns ? m + __ffs(mask >> m) - 1 : nsw;
     if (g.full) {
-      sweeps<R, MODE, true, false>(x, b, g, at, m, plain, note);
-      sweeps<R, MODE, true, true>(x, b, g, at, m, nsw, note);
+      sweeps<R, MODE, true, false>(x, b, g, at, m, plain, md, keep);
+      sweeps<R, MODE, true, true>(x, b, g, at, m, nsw, md, keep);
     } else {
-      sweeps<R, MODE, false, false>(x, b, g, at, m, plain, note);
-      sweeps<R, MODE, false, true>(x, b, g, at, m, nsw, note);
+      sweeps<R, MODE, false, false>(x, b, g, at, m, plain, md, keep);
+      sweeps<R, MODE, false, true>(x, b, g, at, m, nsw, md, keep);
     }
     p ^= nsw & 1;
     done += nsw;
-    if ((mask >> lane) & 1u) atomicMax(&js->cm[nq & 3][lane], keep);
+    if (mask && owns) {
+      const unsigned u = __reduce_max_sync(kFull, __float_as_uint(md));
+      if (lane == nsw - 1) keep = u;
+    }
+    if ((mask >> lane) & 1u) atomicMax(&js->cm[nq & 3][lane], __float_as_uint(quarter(__uint_as_float(keep))));
     // the last exchange serves the field; a solve of less than K sweeps
     // trades once too, so that no CTA stores its rows before its neighbours
     // have loaded them
     const bool trade = G > 1 && ((nsw == K && (done < maxs || J.do_field)) || (done >= maxs && e == 0));
+    auto look = [&]() {
+      if (pend && warp == 0) decide(nq - 1, pmask);
+    };
+    if (trade)
+      trade_out(e, es, look);
+    else
+      look();
+    if (!near || !trade) __syncthreads();
     if (trade) {
-      ++e;
-      show();
-      __syncthreads();
-      publish(e);
-      es = (es + 1) & 3;
-      if (!receive(e, es)) fail();
-    }
-    if (pend && warp == 0) decide(nq - 1, pmask);
-    __syncthreads();
-    if (trade) {
-      take();
+      trade_in(e, es);
       p ^= 1;
       sts4(first + p * par + mine, x[0]);
-      sts4(last + p * par + mine, x[R - 1]);
+      if (R > 1) sts4(last + p * par + mine, x[R - 1]);
       __syncthreads();
     }
     if (js->bail) break;
@@ -1082,6 +1234,16 @@ __global__ void __launch_bounds__(32 * kTileWarps, 1) k_tile(SimArgs a, JacobiAr
   if (threadIdx.x == 0) js.bail = 0;
   __syncthreads();
   solve<R, MODE, REFINE>(a, J, blockIdx.x, tsm, &js);
+  if (MODE != kHalo && J.near) {
+    // A CTA whose wait gave up stays until its neighbours have stopped sending;
+    // without that, all that was sent here has been taken.
+    __syncthreads();
+    if (js.bail) {
+      cluster_arrive();
+      cluster_join();
+      __nanosleep(100000);
+    }
+  }
 }
 
 using Kernel = void (*)(SimArgs, JacobiArgs);
