@@ -32,8 +32,8 @@
 // every K sweeps (1000 cycles in a cluster, 3000-5000 by way of L2, where the
 // instructions of 16 warps weigh as much as the round trip).  Against the
 // shared-memory sweep and register strips of jacobi.cu, 200 sweeps in a step:
-// 512x2048 0.334 -> 0.163 ms, 256x1024 0.191 -> 0.093, 301x700 (rows of no
-// multiple of 4) 0.325 -> 0.096, 32x128 0.127 -> 0.039; with a check after
+// 512x2048 0.334 -> 0.154 ms, 256x1024 0.191 -> 0.092, 301x700 (rows of no
+// multiple of 4) 0.325 -> 0.093, 32x128 0.127 -> 0.038; with a check after
 // each of 2000 sweeps, 64x256 5.0 -> 0.61 ms.
 #pragma once
 
@@ -240,7 +240,7 @@ __device__ __forceinline__ float sweep(float4 (&x)[R], const float4 (&b)[R], con
     }
     e.w = rt;
     float mir = 0.0f;
-    if (FIRST && r < g.nvalid) mir = mirror[r];
+    if (FIRST && r < g.nvalid) mir = times4f(mirror[r]);
     if (FIRST && g.me >= 0) {
       e.x = g.me == 0 ? mir : e.x;
       e.y = g.me == 1 ? mir : e.y;
@@ -413,10 +413,13 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     const int i = x0 - KX + tc;
     return tc >= nc ? -1 : (i < 0 ? i + W : (i >= W ? i - W : i));
   };
-  // The mesh comes in by asynchronous copies, a warp to a row.  These one-time
-  // phases are loops and not unrolled: their instructions are fetched anew in
-  // every solve, and straight-line code of them took longer to fetch than the
-  // data.
+  // The mesh comes in by asynchronous copies, a warp to a row, each lane down
+  // one column at a time (its place in the mesh worked out once), and the
+  // source terms are formed by the strips' own threads, four at a time: going
+  // through the tile element by element took 150 instructions an element and
+  // 10 us of a 512x2048 solve of 163.  These one-time phases are loops and
+  // not unrolled: their instructions are fetched anew in every solve, and
+  // straight-line code of them took longer to fetch than the data.
   float4 x[R], b[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) x[r] = b[r] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -424,59 +427,69 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   if (!REFINE) {
     long long *const aimg = reinterpret_cast<long long *>(snap);  // charges of rows lo..hi, then their source terms
 #pragma unroll 1
-    for (int r = warp; r < rows + 2; r += nwarp) {
-      const size_t rb = (size_t)(lo - 1 + r) * nnx;
-      const bool inner = r > 0 && r <= rows;
-#pragma unroll 1
-      for (int tc = lane; tc < nc; tc += 32) {
-        const int i = real(tc);
-        copy4(timg0 + r * tp + tc, phi + rb + i);
-        if (inner) copy8(aimg + (r - 1) * tp + tc, acc + rb + i);
-        if (inner && i == 0) {
-          copy4(mcol + r - 1, phi + rb + W);
-          copy8(wcol + r - 1, acc + rb + W);
+    for (int tc = lane; tc < tp; tc += 32) {  // a lane's column, down the warp's rows
+      const int i = real(tc);
+      const size_t step = (size_t)nwarp * nnx;
+      const float *from = phi + (size_t)(lo - 1 + warp) * nnx + max(i, 0);
+      const long long *cfrom = acc + (size_t)(lo - 1 + warp) * nnx + max(i, 0);
+#pragma unroll 2
+      for (int r = warp; r < rows + 2; r += nwarp) {
+        float *const to = timg0 + r * tp + tc;
+        const bool inner = r > 0 && r <= rows;
+        if (i >= 0) {
+          copy4(to, from);
+          if (inner) copy8(aimg + (r - 1) * tp + tc, cfrom);
+        } else {
+          *to = 0.0f;
+          if (inner) aimg[(r - 1) * tp + tc] = 0ll;
         }
+        from += step;
+        cfrom += step;
       }
+    }
+    for (int r = tid; r < rows; r += nthr) {  // the mirror column
+      copy4(mcol + r, phi + (size_t)(lo + r) * nnx + W);
+      copy8(wcol + r, acc + (size_t)(lo + r) * nnx + W);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     clear_next();
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
     const bool pow2 = (__double_as_longlong(a.cb) & 0xfffffffffffffll) == 0ll;
     const df cb = df_of(a.cb);
-#pragma unroll 1
-    for (int r = warp; r < rows + 2; r += nwarp) {
-      const bool inner = r > 0 && r <= rows;
-#pragma unroll 2
-      for (int tc = lane; tc < tp; tc += 32) {
-        const int i = real(tc);
-        float *const v = timg0 + r * tp + tc;
-        float p4 = i >= 0 ? times4f(*v) : 0.0f;
-        if (inner) {
-          *v = p4;
-          long long f = i >= 0 ? aimg[(r - 1) * tp + tc] : 0ll;
-          if (i == 0) {  // column 0's charge is folded with the mirror column's
-            f += wcol[r - 1];
-            const float m = times4f(mcol[r - 1]);
-            mcol[r - 1] = m;
-            seam = seam || !(m == p4);
-          }
-          const float s = source(f, a.cb, cb, pow2);
-          *reinterpret_cast<float *>(aimg + (r - 1) * tp + tc) = s;
-        } else {
+    for (int k = tid; k < 2 * tp; k += nthr) {
+      const int up = k >= tp ? 1 : 0, tc = k - up * tp;
+      const float p4 = times4f(timg0[up * (rows + 1) * tp + tc]);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) edge[(2 * q + (r == 0 ? 0 : 1)) * 128 + tc] = p4;
-        }
+      for (int q = 0; q < 4; ++q) edge[(2 * q + up) * 128 + tc] = p4;
+    }
+    // the strip's source terms, in the place of its charges; column 0 (or its
+    // image past column W-1) is folded with the mirror column
+    const int z = !act ? -1 : (g.i0 == 0 ? 0 : (MODE == kHalo && W >= g.i0 && W < g.i0 + 4 ? W - g.i0 : -1));
+#pragma unroll 1
+    for (int r = 0; r < g.nvalid; ++r) {
+      const int j = g.row0 - lo + r;
+      long long *const ar = aimg + j * tp + 4 * li;
+      longlong2 u = *reinterpret_cast<const longlong2 *>(ar), v = *reinterpret_cast<const longlong2 *>(ar + 2);
+      if (z >= 0) {
+        const long long m = wcol[j];
+        u.x += z == 0 ? m : 0ll;
+        u.y += z == 1 ? m : 0ll;
+        v.x += z == 2 ? m : 0ll;
+        v.y += z == 3 ? m : 0ll;
+        seam = seam || !(times4f(mcol[j]) == times4f(timg[j * tp + 4 * li + z]));
       }
+      sts4(reinterpret_cast<float *>(ar), make_float4(source(u.x, a.cb, cb, pow2), source(u.y, a.cb, cb, pow2),
+                                                      source(v.x, a.cb, cb, pow2), source(v.y, a.cb, cb, pow2)));
     }
     seam = __syncthreads_or(seam);
-    const float *const q = timg + (g.row0 - lo) * tp + 4 * li;
-    const float4 *const s4 = reinterpret_cast<const float4 *>(aimg + (g.row0 - lo) * tp + 4 * li);
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (r < g.nvalid) {
-        x[r] = lds4(q + r * tp);
-        const float4 u0 = s4[r * (tp / 2)], u1 = s4[r * (tp / 2) + 1];
-        b[r] = make_float4(u0.x, u0.z, u1.x, u1.z);
+        const int j = g.row0 - lo + r;
+        const float4 v = lds4(timg + j * tp + 4 * li);
+        x[r] = make_float4(times4f(v.x), times4f(v.y), times4f(v.z), times4f(v.w));
+        b[r] = lds4(reinterpret_cast<const float *>(aimg + j * tp + 4 * li));
       }
   } else {
     for (int k = tid; k < 4 * 2 * 128; k += nthr) edge[k] = 0.0f;
