@@ -47,8 +47,8 @@ struct cupic_ctx {
   // scratch of the host-format particle transfers, grown on demand and kept
   void *io_buf = nullptr;
   size_t io_cap = 0;
-  // graph of one step
-  cudaGraphExec_t graph = nullptr;
+  // graphs of one step and of kStepsPerGraph (captured by the first long run)
+  cudaGraphExec_t graph = nullptr, graph_many = nullptr;
   bool graph_ok = false;
   bool initialized = false;
   bool rho_valid = false;
