@@ -102,6 +102,7 @@ bool tile_plan(int nnx, int nny, int nbx, int nby, int K, int R, TileForm form, 
   t.near = nbx == 1 && nby > 1 && nby <= kTileCluster;
   if (t.near) {
     t.tpairs = 2 * K * 4 * t.nl;  // the rows that arrive, two exchanges in turn
+    if (form == kTileEarly) t.tpairs += 2 * t.G * 32 / 2;  // and the maxima of checked blocks
   } else if (t.G > 1) {
     const int wide = nbx > 1 ? 4 * ((W4 + nbx - 1) / nbx) + 2 * K : W;
     const int own = nbx > 1 ? 4 * ((W4 + nbx - 1) / nbx) : W, side = nbx > 1 ? t.B * K : 0;

@@ -34,7 +34,7 @@
 // shared-memory sweep and register strips of jacobi.cu, 200 sweeps in a step:
 // 512x2048 0.334 -> 0.154 ms, 256x1024 0.191 -> 0.092, 301x700 (rows of no
 // multiple of 4) 0.325 -> 0.093, 32x128 0.127 -> 0.038; with a check after
-// each of 2000 sweeps, 64x256 5.0 -> 0.61 ms.
+// each of 2000 sweeps, 64x256 5.0 -> 0.54 ms.
 #pragma once
 
 #include <math.h>
@@ -126,6 +126,7 @@ struct Scratch {
   float decv[2];       // its residual
   int bail;
   uint64_t arrived[2];  // a cluster's exchanges, odd and even ones
+  uint64_t voted[2];    // the maxima of its checked blocks, likewise
   unsigned long long w64[16], res64[2];  // a correction's max |r| per warp, and over the grid
 };
 
@@ -255,10 +256,11 @@ __device__ __forceinline__ float sweep(float4 (&x)[R], const float4 (&b)[R], con
     v.z = node(b[r].z, c.y, e.z, n.z, prev.z);
     v.w = node(b[r].w, c.z, e.w, n.w, prev.w);
     if (CHECK) {
-      float d = (g.own & 1u) ? fabsf(__fsub_rn(v.x, c.x)) : 0.0f;
-      d = (g.own & 2u) ? fmaxf(d, fabsf(__fsub_rn(v.y, c.y))) : d;
-      d = (g.own & 4u) ? fmaxf(d, fabsf(__fsub_rn(v.z, c.z))) : d;
-      d = (g.own & 8u) ? fmaxf(d, fabsf(__fsub_rn(v.w, c.w))) : d;
+      constexpr bool kAll = MODE == kRing;  // a lane with rows owns all its columns
+      float d = kAll || (g.own & 1u) ? fabsf(__fsub_rn(v.x, c.x)) : 0.0f;
+      d = kAll || (g.own & 2u) ? fmaxf(d, fabsf(__fsub_rn(v.y, c.y))) : d;
+      d = kAll || (g.own & 4u) ? fmaxf(d, fabsf(__fsub_rn(v.z, c.z))) : d;
+      d = kAll || (g.own & 8u) ? fmaxf(d, fabsf(__fsub_rn(v.w, c.w))) : d;
       if (FIRST && g.i0 == 0 && (g.own & 1u)) d = fmaxf(d, fabsf(__fsub_rn(v.x, mir)));
       md = (g.ownrows >> r) & 1u ? fmaxf(md, d) : md;
     }
@@ -339,9 +341,15 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   const uint32_t near_bytes = ((by > 0 ? 1 : 0) + (by < nby - 1 ? 1 : 0)) * 16u * K * nl;
   if (near) {
     if (tid == 0) {
-      for (int k = 0; k < 2; ++k) mbar_init(&js->arrived[k], 1);
+      for (int k = 0; k < 2; ++k) {
+        mbar_init(&js->arrived[k], 1);
+        mbar_init(&js->voted[k], 1);
+      }
       fence_mbar_init();
-      for (int k = 0; k < 2; ++k) mbar_arrive_expect_tx(&js->arrived[k], near_bytes);
+      for (int k = 0; k < 2; ++k) {
+        mbar_arrive_expect_tx(&js->arrived[k], near_bytes);
+        mbar_arrive_expect_tx(&js->voted[k], 128u * G);
+      }
     }
     __syncwarp();
     cluster_arrive();
@@ -656,6 +664,8 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   // the neighbours write, in place of the tables.  A neighbour sends exchange
   // e+2 once it has exchange e+1 of this CTA, which takes e before that.
   float *const got = reinterpret_cast<float *>(table);
+  // and after them the maxima of checked blocks [2][CTA][sweep], from every CTA
+  float *const votes = got + 4 * K * tp;
   const bool dn = by > 0, up = by < nby - 1;
   const unsigned gpar = 8u * K * tp;  // bytes of one exchange's rows
   // where this strip's first row goes and comes from, and its rows (bits 0-7:
@@ -999,12 +1009,23 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   int pstart = 0, pes = 0;
   unsigned pmask = 0u;
   // the stop decision on checked block q, taken by warp 0 once every CTA's
-  // maxima are in (usually long before it asks)
+  // maxima are in (usually long before it asks).  In a cluster every CTA has
+  // sent them here: reading a counter and then the maxima from L2 took two
+  // round trips a block (64x256, 2000 checked sweeps: 610 -> 543 us).
   auto decide = [&](int q, unsigned mask) {
-    const unsigned target = (unsigned)G * ((unsigned)q / 4u + 1u);
-    const bool ok = wait_for(ctl, [&]() { return ld_acquire(&J.tbar[q & 3]) >= target; });
     const bool mineck = (mask >> lane) & 1u;
-    const float v = mineck ? __uint_as_float((unsigned)ld_word(&J.gmax[(q & 3) * 32 + lane])) : 0.0f;
+    bool ok;
+    float v = 0.0f;
+    if (near) {
+      const unsigned bar = smem_addr(&js->voted[q & 1]), parity = ((unsigned)q >> 1) & 1u;
+      ok = wait_for(ctl, [&]() { return cluster_wait(bar, parity); });
+      for (int k = 0; k < G; ++k) v = fmaxf(v, votes[((q & 1) * G + k) * 32 + lane]);
+      if (lane == 0) mbar_arrive_expect_tx(&js->voted[q & 1], 128u * G);  // for block q+2, sent after this CTA's q+1
+    } else {
+      const unsigned target = (unsigned)G * ((unsigned)q / 4u + 1u);
+      ok = wait_for(ctl, [&]() { return ld_acquire(&J.tbar[q & 3]) >= target; });
+      if (mineck) v = __uint_as_float((unsigned)ld_word(&J.gmax[(q & 3) * 32 + lane]));
+    }
     const unsigned pass = __ballot_sync(kFull, mineck && (double)v < J.tol && !J.trial);
     const int k = pass ? __ffs(pass) - 1 : 31 - __clz(mask);
     const float vk = __shfl_sync(kFull, v, k);
@@ -1155,7 +1176,15 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
         ++nq;
         if (pass) stop_at(start, k, 0, es0);
       } else {
-        if (warp == 0) {
+        if (near && early) {
+          if (warp == 0) {  // eight lanes to a CTA
+            const float4 u = lds4(reinterpret_cast<const float *>(js->cm[nq & 3]) + 4 * (lane & 7));
+            const unsigned to = smem_addr(votes + ((nq & 1) * G + c) * 32) + 16u * (lane & 7), bar = smem_addr(&js->voted[nq & 1]);
+            for (int k = lane >> 3; k < G; k += 4) st_cluster(cluster_addr(to, k), u, cluster_addr(bar, k));
+            __syncwarp();
+            js->cm[(nq + 2) & 3][lane] = 0u;
+          }
+        } else if (warp == 0) {
           if ((mask >> lane) & 1u)
             atomicMax(&J.gmax[(nq & 3) * 32 + lane],
                       ((unsigned long long)(ebase + (unsigned)nq + 1u) << 32) | js->cm[nq & 3][lane]);
