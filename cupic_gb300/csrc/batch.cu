@@ -182,12 +182,14 @@ int layout_solve(cupic_batch *b, const Knobs &kn) {
   const int T = per_sm * b->num_sms;
   // With few members the fewest CTAs that hold a mesh leave most of the GPU
   // idle: a member takes up to its share of the CTAs by work, but no more
-  // than its own tuned single-context layout.  More CTAs hold fewer rows
-  // each, so the shared memory per CTA does not grow.
+  // than its own tuned single-context layout, and no CTA less than 6 rows
+  // (that layout may divide the rows' columns too; 128x512 alone on 152 CTAs of
+  // 4 rows 0.216 ms a step, on 85 0.194).  More CTAs hold fewer rows each, so the
+  // shared memory per CTA does not grow.
   const double wsum = std::accumulate(work.begin(), work.end(), 0.0);
   for (int i = 0; i < n; ++i) {
     const int share = (int)(T * work[i] / wsum);
-    const int want = std::min(b->members[i]->jG, share);
+    const int want = std::min({b->members[i]->jG, (inst[i].nny - 2) / 6, share});
     Plan q;
     if (want > plan[i].G && plan_on(inst[i], want, fit[i], kn.depth, &q) && q.smem <= smem) plan[i] = q;
   }
