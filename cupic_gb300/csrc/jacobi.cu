@@ -1,5 +1,7 @@
 // jacobi.cu -- Poisson solve (5-point Jacobi, periodic in x, Dirichlet in y)
-// with the field derivation fused into the end of the last sweep
+// with the field derivation fused into the end of the last sweep, for what
+// register tiles (tile.cuh) do not take: meshes that no layout of tiles holds,
+// the precision form from two different columns 0 and nnx-1, and batches
 // (reference: jacobi_iteration mesh.cu:297-381, its host loop
 // mesh.cu:55-120, field_derivation mesh.cu:385-472).
 //

@@ -10,10 +10,14 @@
 //                   reference runs fast_grid_to_particle, leap_frog_step,
 //                   pDefragDown/Up, pRebracketing, bmHandler, pCyclicCC and
 //                   fast_particle_to_grid as separate passes)
-//   k_arrive        appends the movers from the rows below and above
-//   k_inject        draws the injected flux of the step (cc.cu:179-256),
-//                   appends it to the rows it falls in, deposits it
-//   k_finalize      per-step counters, clock advance, charge buffer flip
+//   k_inject_few    draws the injected flux of the step (cc.cu:179-256);
+//                   k_inject_sched and k_inject_gen where it is large
+//   k_tail          room check, the movers appended to the rows above and
+//                   below, the injected particles appended and deposited,
+//                   per-step counters, clock advance, charge buffer flip;
+//                   k_room, k_arrive, k_inject_append and k_finalize do these
+//                   one by one above 4096 rows, in the stage API, when the host
+//                   completes a halted step, and (as _batch) in batches
 #include <map>
 #include <mutex>
 #include <utility>

@@ -185,8 +185,9 @@ int cupic_get_time(struct cupic_ctx *ctx, int64_t *step, double *t, double *tin_
 int cupic_init_mesh(struct cupic_ctx *ctx);
 /* The parameters the context was created with. */
 int cupic_get_params(struct cupic_ctx *ctx, cupic_params *p);
-/* The Jacobi solver's layout: CTAs of the cooperative grid, mesh rows each
- * CTA owns, and the halo depth (sweeps between neighbour exchanges). */
+/* The Jacobi solver's layout: CTAs of its launch (a cluster or a cooperative
+ * grid, which may divide the columns as well as the rows), the most mesh rows
+ * a CTA owns, and the halo depth (sweeps between neighbour exchanges). */
 int cupic_get_solver_plan(struct cupic_ctx *ctx, int32_t *ctas, int32_t *rows_per_cta,
                           int32_t *depth);
 
@@ -207,7 +208,8 @@ int cupic_particle_mover(struct cupic_ctx *ctx);
 int cupic_cc(struct cupic_ctx *ctx, double t);
 
 /* nsteps full cycles (solve, field, push, bin, absorb, inject) with the
- * clock advancing by dt per step, replayed from a captured CUDA graph.
+ * clock advancing by dt per step, replayed from a captured CUDA graph (runs
+ * of 64 steps and more from one of several steps).
  * Returns once the steps are enqueued.  A step whose particles do not fit
  * their rows (checked on the device after the push) idles the rest of the
  * run; the next call that waits grows those rows, completes that step and
@@ -223,7 +225,9 @@ enum {
   CUPIC_PHASE_PUSH = 2,   /* push + wrap + binning + deposition (particles.cu, cc.cu, mesh.cu) */
   CUPIC_PHASE_ARRIVE = 3, /* movers appended to their new rows (cc.cu:640-772); the draws
                              of the injected flux run on a side stream beside the push,
-                             and this phase includes the wait for them and the room check */
+                             and this phase includes the wait for them and the room check.
+                             Up to 4096 rows the append and the bookkeeping are part of the
+                             same launch, and the two phases below take no time of their own */
   CUPIC_PHASE_INJECT = 4, /* append of the injected particles (cc.cu:134-272) */
   CUPIC_PHASE_FINAL = 5,  /* per-step counters and clock */
   CUPIC_NPHASE = 6
