@@ -43,20 +43,22 @@ METRIC = "particle-steps/s full PIC cycle"
 UNIT = "particle-steps/s"
 STATS_BYTES = 96
 # kernels launched per step: solve (which also clears the next charge), push,
-# inject sched and gen, and the step's end (room check, arrivals, append,
-# bookkeeping)
+# inject sched and gen (few draws: draws and kick), and the step's end (room
+# check, arrivals, append, bookkeeping)
 KERNELS_PER_STEP = 5
-FEW_DRAWS = 128  # draws per step and species up to which sched and gen are one kernel
+FEW_DRAWS = 128  # draws per step and species up to which they are made beside the solve
+SMS = 152
 
 
-def kernels_per_step(p):
-    """Kernels one step launches.  The precision form adds the FP64 source
+def kernels_per_step(p, ctas):
+    """Kernels one step launches.  Few draws are one kernel where the solve's
+    CTAs leave no room beside it.  The precision form adds the FP64 source
     (its corrections, stop tests, FP32 potential and field are in the
     solve's launch)."""
     n = KERNELS_PER_STEP + (1 if p.refine_every > 0 else 0)
     flux = [p.n * p.ds * p.ncx * p.ds * math.sqrt(kt / m) / math.sqrt(2.0 * math.pi)
             for m, kt in ((p.me, p.kte), (p.mi, p.kti))]
-    return n - 1 if max(flux) * p.dt <= FEW_DRAWS else n
+    return n - 1 if max(flux) * p.dt <= FEW_DRAWS and ctas + 2 > SMS else n
 
 # algorithmic bytes per unit of work (FP32 SoA, 16 B state per particle)
 PUSH_BYTES_PER_PARTICLE = 32      # 16 B read + 16 B write
@@ -458,7 +460,7 @@ def run_cupic(args, world, rank, local):
                        "parallelism": "replicas" if world > 1 else "single GPU",
                        "jacobi_plan": plan},
             "e2e": e2e,
-            "gpu_launches": kernels_per_step(p) * args.steps,
+            "gpu_launches": kernels_per_step(p, plan["ctas"]) * args.steps,
             "roofline": dominant,
             "roofline_other": other,
             "phases_ms_per_step": {k: v / args.steps for k, v in phases.items()},

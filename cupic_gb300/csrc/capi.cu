@@ -164,6 +164,7 @@ void free_species(cupic_ctx *c, SpeciesDev &S) {
   dfree(c, S.stage_up);
   dfree(c, S.stage_down);
   dfree(c, S.inj_tin);
+  dfree(c, S.inj_v);
   dfree(c, S.inj_p);
   dfree(c, S.inj_d);
   memset(&S, 0, sizeof(S));
@@ -204,6 +205,7 @@ int layout_species(cupic_ctx *c, int sp, const std::vector<int32_t> &capv) {
   CU(dalloc(c, &S.stage_up, (size_t)ncy * S.stage_cap));
   CU(dalloc(c, &S.stage_down, (size_t)ncy * S.stage_cap));
   CU(dalloc(c, &S.inj_tin, (size_t)S.inj_cap));
+  CU(dalloc(c, &S.inj_v, (size_t)3 * S.inj_cap));
   CU(dalloc(c, &S.inj_p, (size_t)S.inj_cap));
   CU(dalloc(c, &S.inj_d, (size_t)S.inj_cap));
   const bool uniform = std::all_of(capv.begin(), capv.end(), [&](int32_t v) { return v == capv[0]; });
@@ -878,19 +880,19 @@ int finish(cupic_ctx *c) {
   return flag_status(f);
 }
 
-// One step: solve + field, then the injection draws on the side stream while
-// the main stream clears the next charge, pushes and appends the movers;
+// After the solve: the injection draws (drawn: only the field's kick of draws
+// made beside the solve) on the side stream while the main stream clears the next charge, pushes and appends the movers;
 // the injected particles are appended once both branches are done.
 // marks: null, or CUPIC_NPHASE events recorded on the main stream after the
 // solve, the clearing, the push, the arrivals (with the wait for the draws
 // and the room check), the append and the bookkeeping -- the phases of
 // cupic_step_timed.
-int enqueue_after_solve(cupic_ctx *c, bool zeroed, const cudaEvent_t *marks = nullptr) {
+int enqueue_after_solve(cupic_ctx *c, bool zeroed, bool drawn, const cudaEvent_t *marks = nullptr) {
   auto mark = [&](int k) { return marks ? cudaEventRecord(marks[k], c->stream) : cudaSuccess; };
   CU(mark(0));
   CU(cudaEventRecord(c->ev_fork, c->stream));
   CU(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-  CU(launch_inject_draw(c->a, c->side));
+  CU(drawn ? launch_inject_kick(c->a, c->side) : launch_inject_draw(c->a, c->side));
   CU(cudaEventRecord(c->ev_join, c->side));
   if (!zeroed) CU(launch_zero_next_rho(c->a, c->stream));
   CU(mark(1));
@@ -915,10 +917,19 @@ int enqueue_after_solve(cupic_ctx *c, bool zeroed, const cudaEvent_t *marks = nu
 }
 
 int enqueue_step(cupic_ctx *c, const cudaEvent_t *marks = nullptr) {
+  // Few draws are made beside the solve, where it leaves them two SMs (each of
+  // its CTAs fills one): beside the push of a small mesh they were what the end
+  // of the step waited for (32x128: 53.5 -> 48.6 us a step).
+  const bool drawn = few_draws(c->a) && c->tile.R && c->tile.G + 2 <= c->num_sms;
+  if (drawn) {
+    CU(cudaEventRecord(c->ev_fork, c->stream));
+    CU(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
+    CU(launch_draw_few(c->a, c->side));
+  }
   bool zeroed = false;
   int rc = run_step_solve(c, &zeroed);
   if (rc) return rc;
-  return enqueue_after_solve(c, zeroed, marks);
+  return enqueue_after_solve(c, zeroed, drawn, marks);
 }
 
 // the graph of `steps` steps; null where they cannot be captured
@@ -939,7 +950,7 @@ int capture_steps(cupic_ctx *c, int steps, cudaGraphExec_t *exec) {
 }
 
 // One graph launch takes 2.5 us of the stream between two steps, so a run of
-// kLongRun steps or more goes in graphs of kStepsPerGraph (32x128 55.7 -> 50.7
+// kLongRun steps or more goes in graphs of kStepsPerGraph (32x128 55.7 -> 53.0
 // us a step, 256x1024 212.4 -> 209.3, 301x700 251.0 -> 247.8).  They cost
 // 130 us to capture, once, which a run of 60 steps just earns back.
 constexpr int kStepsPerGraph = 8, kLongRun = 64;

@@ -23,6 +23,11 @@ cudaError_t launch_leapfrog_start(const SimArgs &a, cudaStream_t st);
 cudaError_t launch_push_deposit(const SimArgs &a, cudaStream_t st);
 cudaError_t launch_arrive(const SimArgs &a, cudaStream_t st);
 cudaError_t launch_inject_draw(const SimArgs &a, cudaStream_t st);
+// the same in two parts where a step draws few particles: all that needs no
+// field, and the field's kick
+bool few_draws(const SimArgs &a);
+cudaError_t launch_draw_few(const SimArgs &a, cudaStream_t st);
+cudaError_t launch_inject_kick(const SimArgs &a, cudaStream_t st);
 cudaError_t launch_inject_append(const SimArgs &a, cudaStream_t st);
 cudaError_t launch_finalize(const SimArgs &a, cudaStream_t st);
 // room check, arrivals, append and bookkeeping in one launch

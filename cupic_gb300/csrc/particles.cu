@@ -10,8 +10,10 @@
 //                   reference runs fast_grid_to_particle, leap_frog_step,
 //                   pDefragDown/Up, pRebracketing, bmHandler, pCyclicCC and
 //                   fast_particle_to_grid as separate passes)
-//   k_inject_few    draws the injected flux of the step (cc.cu:179-256);
-//                   k_inject_sched and k_inject_gen where it is large
+//   k_draw_few      draws the injected flux of the step (cc.cu:179-256) beside
+//   k_inject_kick   the solve, and moves it in the step's field beside the push
+//                   (k_inject_few: both, where the solve takes all SMs;
+//                   k_inject_sched and k_inject_gen where the flux is large)
 //   k_tail          room check, the movers appended to the rows above and
 //                   below, the injected particles appended and deposited,
 //                   per-step counters, clock advance, charge buffer flip;
@@ -824,22 +826,27 @@ __global__ void k_inject_sched_batch(const SimArgs *__restrict__ inst, int n) {
   if (t < 2 * n) inject_sched(inst[t >> 1], t & 1);
 }
 
-// draw k of species sp, injected at time tin
-__device__ __forceinline__ void inject_one(const SimArgs &a, const int sp, const int k, const double tin) {
-  const Ctl *ctl = a.ctl;
-  const SpeciesDev &S = a.sp[sp];
-  const double t = ctl->t, fpt = t + a.dt_d, fvt = t + 0.5 * a.dt_d;
-  const double sig = a.sig[sp], qm = a.qm[sp];
-  const int64_t step = ctl->step;
-  const size_t top = (size_t)(a.nny - 1) * a.nnx;
+// draw k of species sp: its place and velocity before the field's kick
+__device__ __forceinline__ void draw_one(const SimArgs &a, const int sp, const int k, double &x, double &vx, double &vy) {
+  const double sig = a.sig[sp];
+  const int64_t step = a.ctl->step;
   const uint4 r = philox4x32_10(make_uint4((uint32_t)k, (uint32_t)step, (uint32_t)((uint64_t)step >> 32),
                                            (uint32_t)((kPurposeInject << 8) | sp)),
                                 a.k0, a.k1);
-  double x = u01(r.x) * a.Lx_d;
+  x = u01(r.x) * a.Lx_d;
   double sn, cs;
   dev_sincos2pi(u01(r.z), &sn, &cs);
-  double vx = sig * (sqrt(-2.0 * dev_log(u01(r.y))) * cs);
-  double vy = -(sig * sqrt(-2.0 * dev_log(u01(r.w))));
+  vx = sig * (sqrt(-2.0 * dev_log(u01(r.y))) * cs);
+  vy = -(sig * sqrt(-2.0 * dev_log(u01(r.w))));
+}
+
+// its move in the step's field from the time of its injection on
+__device__ __forceinline__ void kick_one(const SimArgs &a, const int sp, const int k, const double tin, double x, double vx,
+                                         double vy) {
+  const SpeciesDev &S = a.sp[sp];
+  const double t = a.ctl->t, fpt = t + a.dt_d, fvt = t + 0.5 * a.dt_d;
+  const double qm = a.qm[sp];
+  const size_t top = (size_t)(a.nny - 1) * a.nnx;
   const int ic = cfloord(x * a.inv_ds_d, 0, a.ncx - 1);
   const double fx = clamp01d(x * a.inv_ds_d - (double)ic);
   const float2 e0 = a.E[top + ic], e1 = a.E[top + ic + 1];
@@ -858,6 +865,13 @@ __device__ __forceinline__ void inject_one(const SimArgs &a, const int sp, const
   S.inj_d[k] = c.dest;
 }
 
+// draw k of species sp, injected at time tin
+__device__ __forceinline__ void inject_one(const SimArgs &a, const int sp, const int k, const double tin) {
+  double x, vx, vy;
+  draw_one(a, sp, k, x, vx, vy);
+  kick_one(a, sp, k, tin, x, vx, vy);
+}
+
 __device__ __forceinline__ void inject_gen(const SimArgs &a, const int sp, const int k) {
   if (halted(a.ctl)) return;
   if (k < a.ctl->inj_gen[sp]) inject_one(a, sp, k, a.sp[sp].inj_tin[k]);
@@ -867,8 +881,11 @@ __device__ __forceinline__ void inject_gen(const SimArgs &a, const int sp, const
 // species: every thread accumulates its own draw's time, one dtin at a time
 // as the schedule does.  Behind the schedule's launch the draws of a 32x128
 // mesh held up the step 7 us longer than the push beside them.
+// KICK: in the step's field at once; else (k_draw_few) left for k_inject_kick,
+// and the kernel runs beside the solve.
 constexpr int kDrawBlock = 128;
-__global__ void __launch_bounds__(kDrawBlock) k_inject_few(SimArgs a) {
+template <bool KICK>
+__device__ __forceinline__ void inject_few(const SimArgs &a) {
   Ctl *ctl = a.ctl;
   if (halted(ctl)) return;
   const int sp = blockIdx.x;
@@ -892,7 +909,24 @@ __global__ void __launch_bounds__(kDrawBlock) k_inject_few(SimArgs a) {
   int done = 0;
   for (int k = threadIdx.x; k < ne; k += kDrawBlock) {
     for (; done < k; ++done) tin += dtin;
-    inject_one(a, sp, k, tin);
+    if (KICK) {
+      inject_one(a, sp, k, tin);
+    } else {
+      double *const v = S.inj_v + 3 * k;
+      draw_one(a, sp, k, v[0], v[1], v[2]);
+      S.inj_tin[k] = tin;
+    }
+  }
+}
+__global__ void __launch_bounds__(kDrawBlock) k_inject_few(SimArgs a) { inject_few<true>(a); }
+__global__ void __launch_bounds__(kDrawBlock) k_draw_few(SimArgs a) { inject_few<false>(a); }
+
+__global__ void __launch_bounds__(kDrawBlock) k_inject_kick(SimArgs a) {
+  if (halted(a.ctl)) return;
+  const SpeciesDev &S = a.sp[blockIdx.x];
+  for (int k = threadIdx.x; k < a.ctl->inj_gen[blockIdx.x]; k += kDrawBlock) {
+    const double *const v = S.inj_v + 3 * k;
+    kick_one(a, blockIdx.x, k, S.inj_tin[k], v[0], v[1], v[2]);
   }
 }
 
@@ -1240,10 +1274,22 @@ cudaError_t launch_arrive(const SimArgs &a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+bool few_draws(const SimArgs &a) { return a.dt_d <= kDrawBlock * a.dtin[0] && a.dt_d <= kDrawBlock * a.dtin[1]; }
+
+cudaError_t launch_draw_few(const SimArgs &a, cudaStream_t st) {
+  k_draw_few<<<2, kDrawBlock, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_inject_kick(const SimArgs &a, cudaStream_t st) {
+  k_inject_kick<<<2, kDrawBlock, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
 // The draws depend only on the clocks and the step's field, so a step can
 // run them beside the push; the append needs the push's row counts.
 cudaError_t launch_inject_draw(const SimArgs &a, cudaStream_t st) {
-  if (a.dt_d <= kDrawBlock * a.dtin[0] && a.dt_d <= kDrawBlock * a.dtin[1]) {
+  if (few_draws(a)) {
     k_inject_few<<<2, kDrawBlock, 0, st>>>(a);
     return cudaGetLastError();
   }
