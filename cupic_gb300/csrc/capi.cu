@@ -573,7 +573,7 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
     cands.push_back(t);
     words = std::max(words, t.words);
     maxG = std::max(maxG, t.G);
-    if ((int)cands.size() >= (getenv("TN")?atoi(getenv("TN")):kTileTrials)) break;
+    if ((int)cands.size() >= kTileTrials) break;
   }
   if (cands.empty()) return CUPIC_ERR_CAPACITY;
   TilePlan pick = cands.front();
@@ -603,7 +603,6 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
         cudaGetLastError();
         continue;
       }
-      if (getenv("TDUMP")) printf("T %d %d nbx %d nby %d K %d R %d w %d m %d near %d cost %.0f cyc %.0f\n", c->a.nnx, c->a.nny, t.nbx,t.nby,t.K,t.R,t.warps,t.mode,t.near,t.cost, (ms_best*1e-3-15e-6)/S*2.07e9);
       if (ms_best < best) {
         best = ms_best;
         pick = t;
