@@ -610,8 +610,9 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    // a solve that gave up waiting leaves a flag: clear what the trials raised
+    // a solve that gave up waiting leaves two flags: clear what the trials raised
     CU(cudaMemsetAsync(&c->ctl->step_flags, 0, sizeof(uint32_t), c->stream));
+    CU(cudaMemsetAsync(&c->ctl->abort, 0, sizeof(c->ctl->abort), c->stream));
     CU(cudaStreamSynchronize(c->stream));
   }
   {
