@@ -24,15 +24,22 @@ using namespace cupic;
 cudaError_t cupic::raise_dyn_smem(const void *kernel, size_t bytes) {
   static std::mutex mu;
   static std::map<std::pair<const void *, int>, size_t> cur;
-  if (bytes <= 48 * 1024) return cudaSuccess;  // below the default limit
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> lock(mu);
-  size_t &have = cur[std::make_pair(kernel, dev)];
-  if (bytes <= have) return cudaSuccess;
+  const auto key = std::make_pair(kernel, dev);
+  auto it = cur.find(key);
+  if (it == cur.end()) {
+    // by default 48 KB, of which the kernel's static shared memory is a part
+    cudaFuncAttributes at;
+    e = cudaFuncGetAttributes(&at, kernel);
+    if (e != cudaSuccess) return e;
+    it = cur.emplace(key, (size_t)at.maxDynamicSharedSizeBytes).first;
+  }
+  if (bytes <= it->second) return cudaSuccess;
   e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e == cudaSuccess) have = bytes;
+  if (e == cudaSuccess) it->second = bytes;
   return e;
 }
 

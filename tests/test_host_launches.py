@@ -1,0 +1,69 @@
+"""The library's host code without a GPU: its objects linked with a runtime that
+looks at launches instead of running them (fake_cuda/runtime.cu).  Layouts,
+tuner trials and scratch of the solves are held against the buffers that the
+launches get, and a solve leaves marks where it would write."""
+import ctypes
+import glob
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+import cupic_gb300 as cg
+from cupic_gb300 import build
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+MARK = 7.0
+
+
+@pytest.fixture(scope="session")
+def fake_path(tmp_path_factory):
+    build.build()
+    out = tmp_path_factory.mktemp("fake")
+    obj, lib = str(out / "runtime.o"), str(out / "libcupic_fake.so")
+    subprocess.run([build.nvcc()] + build.common_flags() + ["-I", build.CSRC, "-D__CUDA_DEVICE_RUNTIME_API_H__", "-c",
+                   os.path.join(HERE, "fake_cuda", "runtime.cu"), "-o", obj], check=True)
+    objs = [os.path.join(build.OUT, os.path.splitext(s)[0] + ".o") for s in build.SOURCES]
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", lib, obj] + objs + ["-lpthread"], check=True)
+    return lib
+
+
+@pytest.fixture
+def fake(fake_path, monkeypatch):
+    """cupic_gb300 on a library of its own on that runtime (nothing tuned yet)."""
+    copy = fake_path + f".{len(glob.glob(fake_path + '*'))}"
+    shutil.copyfile(fake_path, copy)  # one handle each
+    for name in ("CTAS", "DEPTH", "TUNE", "NOSTRIP", "SCALAR"):
+        monkeypatch.delenv("CUPIC_JACOBI_" + name, raising=False)
+    monkeypatch.setattr(cg, "_LIB", None)
+    monkeypatch.setattr(cg, "library_path", lambda: copy)
+    L = cg.load_library()
+    L.fake_allocated.restype = ctypes.c_uint64
+    L.fake_raise.restype = ctypes.c_uint64
+    L.fake_raise.argtypes = [ctypes.c_uint64]
+    return L
+
+
+def faults(L):
+    text = ctypes.create_string_buffer(1 << 16)
+    L.fake_faults(text, len(text))
+    return text.value.decode().splitlines()
+
+
+def params(ncx, ncy, **over):
+    return cg.workload_params("tiny", ncx=ncx, ncy=ncy, n=2.0, **over)
+
+
+def test_raised_shared_memory_counts_the_static_part(fake):
+    """48 KB without an opt-in are static and dynamic shared memory together: a
+    kernel's dynamic part is raised from there on, not from 48 KB on, and never
+    lowered again."""
+    for n in (1000, 48 * 1024 - 720, 48 * 1024 - 719, 48 * 1024, 100000):
+        assert fake.fake_raise(n) >= n
+    # rows of 200 cells take 48,768 bytes of the push, beside its static 640
+    with cg.Sim(params(200, 40)) as sim:
+        sim.init_plasma()
+        sim.step(2)
+    assert faults(fake) == []
