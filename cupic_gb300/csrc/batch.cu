@@ -189,7 +189,7 @@ int layout_solve(cupic_batch *b, const Knobs &kn) {
   const double wsum = std::accumulate(work.begin(), work.end(), 0.0);
   for (int i = 0; i < n; ++i) {
     const int share = (int)(T * work[i] / wsum);
-    const int want = std::min({b->members[i]->jG, (inst[i].nny - 2) / 6, share});
+    const int want = std::min({b->members[i]->lay.G, (inst[i].nny - 2) / 6, share});
     Plan q;
     if (want > plan[i].G && plan_on(inst[i], want, fit[i], kn.depth, &q) && q.smem <= smem) plan[i] = q;
   }

@@ -278,7 +278,7 @@ void fill_constants(cupic_ctx *c) {
   a.k1 = (uint32_t)(p.seed >> 32);
 }
 
-JacobiArgs jargs(const cupic_ctx *c, double tol, int mn, int mx, int chk, int field);
+JacobiArgs jargs(const cupic_ctx *c, const SolveLayout &l, double tol, int mn, int mx, int chk, int field);
 void refine_args(const cupic_ctx *c, JacobiArgs *J, double tol, int mn, int mx, int write_stats);
 
 // ---- Jacobi layout -------------------------------------------------------
@@ -310,24 +310,40 @@ int jacobi_rows(const cupic_ctx *c, int G, int K, int P, long long rows_fit) {
   return B;
 }
 
-// exchange words, residual slots and counters of a layout, zeroed
-int alloc_jacobi_scratch(cupic_ctx *c, int G, size_t words) {
-  dfree(c, c->jflags);
-  dfree(c, c->jres);
-  dfree(c, c->jhalo);
-  dfree(c, c->jgmax);
-  c->jflags = nullptr;
-  c->jres = nullptr;
-  c->jhalo = nullptr;
-  c->jgmax = nullptr;
-  CU(dalloc(c, &c->jflags, (size_t)G + 1));
-  CU(dalloc(c, &c->jres, (size_t)2 * G));
-  CU(dalloc(c, &c->jhalo, words));
-  CU(dalloc(c, &c->jgmax, (size_t)130));
-  c->jhalo_words = words;
-  // epoch 0 is never valid; the solves on the context's stream follow the clearing
-  CU(cudaMemsetAsync(c->jhalo, 0, sizeof(unsigned long long) * words, c->stream));
-  CU(cudaMemsetAsync(c->jgmax, 0, sizeof(unsigned long long) * 130, c->stream));
+void free_solve_scratch(cupic_ctx *c, SolveLayout *l) {
+  dfree(c, l->flags);
+  dfree(c, l->res);
+  dfree(c, l->halo);
+  dfree(c, l->gmax);
+  l->flags = nullptr;
+  l->res = nullptr;
+  l->halo = nullptr;
+  l->gmax = nullptr;
+}
+
+// exchange words, residual slots and counters for layouts of up to G CTAs,
+// zeroed (epoch 0 is never valid; the solves on the context's stream follow
+// the clearing)
+int alloc_solve_scratch(cupic_ctx *c, SolveLayout *l, int G, size_t words) {
+  cudaError_t e = dalloc(c, &l->flags, (size_t)G + 1);
+  if (e == cudaSuccess) e = dalloc(c, &l->res, (size_t)2 * G);
+  if (e == cudaSuccess) e = dalloc(c, &l->halo, words);
+  if (e == cudaSuccess) e = dalloc(c, &l->gmax, (size_t)130);
+  if (e == cudaSuccess) e = cudaMemsetAsync(l->halo, 0, sizeof(unsigned long long) * words, c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(l->gmax, 0, sizeof(unsigned long long) * 130, c->stream);
+  l->halo_words = words;
+  if (e == cudaSuccess) return CUPIC_OK;
+  free_solve_scratch(c, l);
+  return cuda_status(e);
+}
+
+// makes l, with scratch of its own, the context's layout; the one before stays
+// when that scratch cannot be had
+int use_layout(cupic_ctx *c, SolveLayout l, size_t words) {
+  const int rc = alloc_solve_scratch(c, &l, l.G, words);
+  if (rc) return rc;
+  free_solve_scratch(c, &c->lay);
+  c->lay = l;
   c->epoch_use = 0;
   return CUPIC_OK;
 }
@@ -342,8 +358,8 @@ int alloc_jacobi_scratch(cupic_ctx *c, int G, size_t words) {
 // exchanges: an upper bound of those the enqueued solves can make.
 constexpr int64_t kEpochGuard = 1ll << 30;
 int epoch_guard(cupic_ctx *c, int64_t exchanges) {
-  if (c->jhalo && c->epoch_use + exchanges > kEpochGuard) {
-    CU(cudaMemsetAsync(c->jhalo, 0, sizeof(unsigned long long) * c->jhalo_words, c->stream));
+  if (c->lay.halo && c->epoch_use + exchanges > kEpochGuard) {
+    CU(cudaMemsetAsync(c->lay.halo, 0, sizeof(unsigned long long) * c->lay.halo_words, c->stream));
     c->epoch_use = 0;
   }
   c->epoch_use += exchanges;
@@ -357,14 +373,33 @@ int64_t solves_of(const cupic_ctx *c, int mx) {
   return std::max(mx, 0) + 4 * launches;
 }
 
-int set_jacobi_plan(cupic_ctx *c, int G, int B, int K, int P) {
-  c->jG = G;
-  c->jB = B;
-  c->jK = G > 1 ? K : 1;
-  c->jP = P;
-  c->tile.R = 0;
-  CU(jacobi_set_smem(jacobi_smem_bytes(B, c->jK, P)));
-  return alloc_jacobi_scratch(c, G, (size_t)4 * G * c->jK * P);
+// a layout of jacobi.cu, without scratch
+SolveLayout jacobi_layout(int G, int B, int K, int P, bool nostrip) {
+  SolveLayout l;
+  l.G = G;
+  l.B = B;
+  l.K = G > 1 ? K : 1;
+  l.P = P;
+  l.nostrip = nostrip;
+  return l;
+}
+
+size_t jacobi_words(const SolveLayout &l) { return (size_t)4 * l.G * l.K * l.P; }
+
+int set_jacobi_plan(cupic_ctx *c, const SolveLayout &l) {
+  CU(jacobi_set_smem(jacobi_smem_bytes(l.B, l.K, l.P)));
+  return use_layout(c, l, jacobi_words(l));
+}
+
+// a layout of register tiles, without scratch
+SolveLayout tile_layout(const cupic_ctx *c, const TilePlan &t) {
+  SolveLayout l;
+  l.G = t.G;
+  l.B = t.B;
+  l.K = t.K;
+  l.P = (c->a.nnx + 3) / 4 * 4;
+  l.tile = t;
+  return l;
 }
 
 int set_tile_plan(cupic_ctx *c, const TilePlan &t) {
@@ -373,12 +408,7 @@ int set_tile_plan(cupic_ctx *c, const TilePlan &t) {
     cudaGetLastError();
     return CUPIC_ERR_ARG;
   }
-  c->jG = t.G;
-  c->jB = t.B;
-  c->jK = t.K;
-  c->jP = (c->a.nnx + 3) / 4 * 4;
-  c->tile = t;
-  return alloc_jacobi_scratch(c, t.G, t.words);
+  return use_layout(c, tile_layout(c, t), t.words);
 }
 
 // a context's solves may all stop on a tolerance given by the call
@@ -431,7 +461,7 @@ int plan_jacobi_rule(cupic_ctx *c, int P, long long rows_fit) {
           set_tile_plan(c, t) == CUPIC_OK)
         return CUPIC_OK;
     }
-  return set_jacobi_plan(c, G, B, K, P);
+  return set_jacobi_plan(c, jacobi_layout(G, B, K, P, false));
 }
 
 // Autotuner: times every feasible (CTAs, depth) layout on this context's own
@@ -451,6 +481,16 @@ struct TunePick {
 };
 std::map<TuneKey, TunePick> g_tuned;
 
+// a trial's layout in the scratch of all trials
+SolveLayout on_scratch(SolveLayout l, const SolveLayout &scratch) {
+  l.flags = scratch.flags;
+  l.res = scratch.res;
+  l.halo = scratch.halo;
+  l.halo_words = scratch.halo_words;
+  l.gmax = scratch.gmax;
+  return l;
+}
+
 int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
   const int M = c->a.nny - 2;
   const int chk = std::max(1, c->p.check_every);
@@ -462,18 +502,16 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
     if (it != g_tuned.end()) {
       const int G = it->second.G, K = it->second.K;
       const int B = jacobi_rows(c, G, K, P, rows_fit);
-      c->jNoStrip = it->second.nostrip;
-      if (B) return set_jacobi_plan(c, G, B, K, P);
+      if (B) return set_jacobi_plan(c, jacobi_layout(G, B, K, P, it->second.nostrip));
     }
   }
   // every layout is timed with the sweep form it would get, and again with
   // the shared-memory sweep where that form is register strips
-  struct Cand { int G, B, K; bool nostrip; };
-  std::vector<Cand> cands;
+  std::vector<SolveLayout> cands;
   const int ns = c->num_sms;
   const int gs[] = {1, 2, 4, 8, 16, 24, ns / 4, ns / 2, ns};
   int maxG = 1;
-  long long maxGK = 1;
+  size_t words = 0;
   for (int G : gs) {
     if (G < 1 || G > M) continue;
     if (!cands.empty() && cands.back().G == G) continue;
@@ -485,30 +523,27 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
       if (!cands.empty() && cands.back().G == G && cands.back().K >= K) continue;  // no repeats
       const int B = jacobi_rows(c, G, K, P, rows_fit);
       if (!B) continue;
-      cands.push_back({G, B, K, false});
-      if (jacobi_strip_rows(c->a.nnx, B + 2 * (G > 1 ? K : 1) - 2) > 0) cands.push_back({G, B, K, true});
+      cands.push_back(jacobi_layout(G, B, K, P, false));
       maxG = std::max(maxG, G);
-      maxGK = std::max(maxGK, (long long)G * K);
+      words = std::max(words, jacobi_words(cands.back()));
+      if (jacobi_strip_rows(c->a.nnx, B + 2 * (G > 1 ? K : 1) - 2) > 0)
+        cands.push_back(jacobi_layout(G, B, K, P, true));
     }
   }
   if (cands.empty()) return plan_jacobi_rule(c, P, rows_fit);
-  int rc = alloc_jacobi_scratch(c, maxG, (size_t)4 * maxGK * P);
+  SolveLayout scratch;
+  int rc = alloc_solve_scratch(c, &scratch, maxG, words);
   if (rc) return rc;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
   float best = 1e30f;
-  Cand pick = cands.front();
-  for (const Cand &cd : cands) {
-    c->jG = cd.G;
-    c->jB = cd.B;
-    c->jK = cd.G > 1 ? cd.K : 1;
-    c->jP = P;
-    c->jNoStrip = cd.nostrip;
+  SolveLayout pick = cands.front();
+  for (const SolveLayout &cd : cands) {
     // write_stats keeps the residual checks of the real solve (a solve with
     // no tolerance that reports nothing skips them); the stats it writes
     // are overwritten by the first real solve
-    JacobiArgs J = jargs(c, 0.0, S, S, chk, 1);
+    JacobiArgs J = jargs(c, on_scratch(cd, scratch), 0.0, S, S, chk, 1);
     J.write_stats = 1;
     float t = 1e30f;
     bool ok = true;
@@ -534,12 +569,12 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
   // a solve that gave up waiting leaves a flag: clear what the trials raised
   CU(cudaMemsetAsync(&c->ctl->step_flags, 0, sizeof(uint32_t), c->stream));
   CU(cudaStreamSynchronize(c->stream));
+  free_solve_scratch(c, &scratch);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tuned[key] = {pick.G, pick.K, pick.nostrip};
   }
-  c->jNoStrip = pick.nostrip;
-  return set_jacobi_plan(c, pick.G, pick.B, pick.K, P);
+  return set_jacobi_plan(c, pick);
 }
 
 // Register tiles: the layouts with the lowest estimated cost are timed on
@@ -585,7 +620,8 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
   if (cands.empty()) return CUPIC_ERR_CAPACITY;
   TilePlan pick = cands.front();
   if (cands.size() > 1) {
-    const int rc = alloc_jacobi_scratch(c, maxG, words);
+    SolveLayout scratch;
+    const int rc = alloc_solve_scratch(c, &scratch, maxG, words);
     if (rc) return rc;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     CU(cudaEventCreate(&e0));
@@ -593,8 +629,7 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
     float best = 1e30f;
     if (m > 0) CU(cudaMemsetAsync(c->b64, 0, sizeof(double) * (size_t)c->a.nnx * c->a.nny, c->stream));
     for (const TilePlan &t : cands) {
-      c->tile = t;
-      JacobiArgs J = jargs(c, early ? 1.0 : 0.0, early ? 1 : S, S, chk, 1);
+      JacobiArgs J = jargs(c, on_scratch(tile_layout(c, t), scratch), early ? 1.0 : 0.0, early ? 1 : S, S, chk, 1);
       if (m > 0) refine_args(c, &J, 0.0, 0, std::min(S, 4 * m), 0);
       J.trial = 1;
       float ms_best = 1e30f;
@@ -621,6 +656,7 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
     CU(cudaMemsetAsync(&c->ctl->step_flags, 0, sizeof(uint32_t), c->stream));
     CU(cudaMemsetAsync(&c->ctl->abort, 0, sizeof(c->ctl->abort), c->stream));
     CU(cudaStreamSynchronize(c->stream));
+    free_solve_scratch(c, &scratch);
   }
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -645,30 +681,36 @@ int plan_jacobi(cupic_ctx *c) {
   return tune_jacobi(c, P, rows_fit);
 }
 
-JacobiArgs jargs(const cupic_ctx *c, double tol, int mn, int mx, int chk, int field) {
+// a solve on layout l
+JacobiArgs jargs(const cupic_ctx *c, const SolveLayout &l, double tol, int mn, int mx, int chk, int field) {
   JacobiArgs J{};
   J.tol = tol;
   J.min_sweeps = mn;
   J.max_sweeps = mx;
   J.check_every = chk < 1 ? 1 : chk;
-  J.G = c->jG;
-  J.rows_per_cta = c->jB;
-  J.depth = c->jK;
-  J.pitch = c->jP;
+  J.G = l.G;
+  J.rows_per_cta = l.B;
+  J.depth = l.K;
+  J.pitch = l.P;
   J.vec = ((c->a.nnx - 1) % 4 == 0) ? 1 : 0;
-  J.strip = jacobi_strip_rows(c->a.nnx, c->jB + 2 * (c->jG > 1 ? c->jK : 1) - 2);
+  J.strip = jacobi_strip_rows(c->a.nnx, l.B + 2 * (l.G > 1 ? l.K : 1) - 2);
   if (getenv("CUPIC_JACOBI_SCALAR")) J.vec = 0;
-  if (c->jNoStrip || getenv("CUPIC_JACOBI_SCALAR") || getenv("CUPIC_JACOBI_NOSTRIP")) J.strip = 0;
+  if (l.nostrip || getenv("CUPIC_JACOBI_SCALAR") || getenv("CUPIC_JACOBI_NOSTRIP")) J.strip = 0;
   J.do_field = field;
   J.write_stats = 1;
-  J.flags = c->jflags;
-  J.bar = c->jflags + c->jG;
-  J.res_cta = c->jres;
-  J.halo = c->jhalo;
-  J.gmax = c->jgmax;
-  J.tbar = reinterpret_cast<unsigned *>(c->jgmax + 128);
-  if (c->tile.R) tile_args(c->tile, &J);
+  J.flags = l.flags;
+  J.bar = l.flags + l.G;
+  J.res_cta = l.res;
+  J.halo = l.halo;
+  J.gmax = l.gmax;
+  J.tbar = reinterpret_cast<unsigned *>(l.gmax + 128);
+  if (l.tile.R) tile_args(l.tile, &J);
   return J;
+}
+
+// a solve on the context's layout
+JacobiArgs jargs(const cupic_ctx *c, double tol, int mn, int mx, int chk, int field) {
+  return jargs(c, c->lay, tol, mn, mx, chk, field);
 }
 
 // the precision form's solve as one launch of register tiles
@@ -686,7 +728,7 @@ void refine_args(const cupic_ctx *c, JacobiArgs *J, double tol, int mn, int mx, 
 // one solve with the context's layout
 cudaError_t launch_solve(const cupic_ctx *c, const JacobiArgs &J) {
   if (J.max_sweeps < 1 && !J.r64_phi && !J.phi) return launch_field(c->a, J.do_field, J.write_stats, c->stream);
-  return c->tile.R ? launch_tile(c->a, J, c->tile, c->stream) : launch_jacobi(c->a, J, c->stream);
+  return c->lay.tile.R ? launch_tile(c->a, J, c->lay.tile, c->stream) : launch_jacobi(c->a, J, c->stream);
 }
 
 int set_phi_both(cupic_ctx *c, const double *phi) {
@@ -703,7 +745,7 @@ int set_phi_both(cupic_ctx *c, const double *phi) {
     const int nnx = c->a.nnx;
     bool same = true;
     for (int j = 0; j < c->a.nny; ++j) same = same && phi[(size_t)j * nnx] == phi[(size_t)j * nnx + nnx - 1];
-    if (!same && c->tile.R) {
+    if (!same && c->lay.tile.R) {
       c->no_tiles = true;
       destroy_graph(c);
       return plan_jacobi(c);
@@ -811,14 +853,14 @@ int refine_solve_tiles(cupic_ctx *c, double tol, int mn, int mx, int field, int 
   JacobiArgs J = jargs(c, 0.0, 0, 0, 1, field);
   refine_args(c, &J, tol, mn, mx, write_stats);
   J.zero_next = zero_next;
-  CU(launch_tile(c->a, J, c->tile, c->stream));
+  CU(launch_tile(c->a, J, c->lay.tile, c->stream));
   return CUPIC_OK;
 }
 
 // the solve of a step or stage call, FP32 or in the precision form
 int run_solve(cupic_ctx *c, double tol, int mn, int mx, int chk, int field, int write_stats = 1) {
   if (c->p.refine_every > 0) {
-    if (c->tile.R) return refine_solve_tiles(c, tol, mn, mx, field, write_stats, 0);
+    if (c->lay.tile.R) return refine_solve_tiles(c, tol, mn, mx, field, write_stats, 0);
     return refine_on_device(c, mx) ? refine_solve_device(c, tol, mn, mx, field, write_stats)
                                    : refine_solve(c, tol, mn, mx, field, write_stats);
   }
@@ -833,7 +875,7 @@ int run_solve(cupic_ctx *c, double tol, int mn, int mx, int chk, int field, int 
 int run_step_solve(cupic_ctx *c, bool *zeroed) {
   const cupic_params &p = c->p;
   *zeroed = false;
-  if (p.refine_every > 0 && !c->tile.R)
+  if (p.refine_every > 0 && !c->lay.tile.R)
     return run_solve(c, p.tol, p.min_sweeps, p.max_sweeps, p.check_every, 1);
   *zeroed = true;
   if (p.refine_every > 0) return refine_solve_tiles(c, p.tol, p.min_sweeps, p.max_sweeps, 1, 1, 1);
@@ -927,7 +969,7 @@ int enqueue_step(cupic_ctx *c, const cudaEvent_t *marks = nullptr) {
   // Few draws are made beside the solve, where it leaves them two SMs (each of
   // its CTAs fills one): beside the push of a small mesh they were what the end
   // of the step waited for (32x128: 53.5 -> 48.6 us a step).
-  const bool drawn = few_draws(c->a) && c->tile.R && c->tile.G + 2 <= c->num_sms;
+  const bool drawn = few_draws(c->a) && c->lay.tile.R && c->lay.tile.G + 2 <= c->num_sms;
   if (drawn) {
     CU(cudaEventRecord(c->ev_fork, c->stream));
     CU(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
@@ -1396,10 +1438,7 @@ int cupic_destroy(cupic_ctx *c) {
   dfree(c, c->a.rho[0]);
   dfree(c, c->a.rho[1]);
   dfree(c, c->ctl);
-  dfree(c, c->jflags);
-  dfree(c, c->jres);
-  dfree(c, c->jhalo);
-  dfree(c, c->jgmax);
+  free_solve_scratch(c, &c->lay);
   dfree(c, c->io_buf);
   dfree(c, c->phi64);
   dfree(c, c->b64);
@@ -1554,9 +1593,9 @@ int cupic_get_params(cupic_ctx *c, cupic_params *p) {
 
 int cupic_get_solver_plan(cupic_ctx *c, int32_t *ctas, int32_t *rows_per_cta, int32_t *depth) {
   if (!c) return CUPIC_ERR_ARG;
-  if (ctas) *ctas = c->jG;
-  if (rows_per_cta) *rows_per_cta = c->jB;
-  if (depth) *depth = c->jK;
+  if (ctas) *ctas = c->lay.G;
+  if (rows_per_cta) *rows_per_cta = c->lay.B;
+  if (depth) *depth = c->lay.K;
   return CUPIC_OK;
 }
 
@@ -1734,7 +1773,7 @@ int cupic_step(cupic_ctx *c, int32_t nsteps) {
     int rc = deposit_current(c);
     if (rc) return rc;
   }
-  if (c->p.refine_every > 0 && !c->tile.R && !refine_on_device(c, c->p.max_sweeps)) {
+  if (c->p.refine_every > 0 && !c->lay.tile.R && !refine_on_device(c, c->p.max_sweeps)) {
     // the solve reads its residual norm on the host: no graph, and a step
     // that runs out of room is completed before the next one starts
     for (int i = 0; i < nsteps; ++i) {

@@ -12,6 +12,18 @@
 using cupic::Ctl;
 using cupic::SimArgs;
 
+// A layout of the solve, and the scratch it runs in
+struct SolveLayout {
+  int G = 1, B = 1, K = 1, P = 0;  // CTAs, most mesh rows of one, halo depth, row pitch
+  bool nostrip = false;            // the tuner found the shared-memory sweep faster than register strips
+  cupic::TilePlan tile{};          // register tiles (R == 0: the sweeps of jacobi.cu)
+  unsigned *flags = nullptr;       // [G+1]: per-CTA sweep counters, then the barrier
+  float *res = nullptr;            // [2*G]
+  unsigned long long *halo = nullptr;  // halo words, zeroed at allocation
+  size_t halo_words = 0;
+  unsigned long long *gmax = nullptr;  // [128] maxima of checked sweeps, then [4] counters; zeroed
+};
+
 struct cupic_ctx {
   cupic_params p;
   int device = 0;
@@ -25,16 +37,8 @@ struct cupic_ctx {
   std::vector<int64_t> seg[2];
   std::vector<int32_t> cap[2];
   int64_t total_cap[2] = {0, 0};
-  // Jacobi geometry and exchange buffers
-  int jG = 1, jB = 1, jK = 1, jP = 0;
-  cupic::TilePlan tile{};  // register-tile layout (R == 0: the shared-memory sweep of jacobi.cu)
-  bool no_tiles = false;     // the precision form's potential needs the launches of jacobi.cu
-  unsigned long long *jgmax = nullptr;  // [128] maxima of checked sweeps, then [4] counters; zeroed
-  bool jNoStrip = false;  // the tuner found the shared-memory sweep faster than register strips
-  unsigned *jflags = nullptr;  // [G+1]: per-CTA sweep counters, then the barrier
-  float *jres = nullptr;
-  unsigned long long *jhalo = nullptr;  // halo words, zeroed at allocation
-  size_t jhalo_words = 0;
+  SolveLayout lay;
+  bool no_tiles = false;  // the precision form's potential needs the launches of jacobi.cu
   // exchanges enqueued since the halo words were last zeroed (see epoch_guard)
   int64_t epoch_use = 0;
   // precision form of the solve (refine_every > 0): FP64 potential, FP32

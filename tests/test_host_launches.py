@@ -67,3 +67,30 @@ def test_raised_shared_memory_counts_the_static_part(fake):
         sim.init_plasma()
         sim.step(2)
     assert faults(fake) == []
+
+
+def two_columns(p, value=0.5):
+    """A potential whose columns 0 and nnx-1 differ."""
+    phi = np.full((p.nny, p.nnx), 1.25)
+    phi[1:-1, -1] += value
+    return phi
+
+
+MESHES = [(256, 1024), (300, 700), (128, 512), (200, 300), (512, 512), (512, 2048), (64, 90), (3, 5)]
+
+
+@pytest.mark.parametrize("ncx,ncy", MESHES)
+def test_two_seam_columns_keep_launches_inside_their_buffers(fake, ncx, ncy):
+    """A potential with two different columns at the seam takes the precision form
+    off the register tiles: the launches timed and made after that are of their
+    own layout, in scratch of that layout."""
+    p = params(ncx, ncy, refine_every=32, max_sweeps=320)
+    with cg.Sim(p) as sim:
+        sim.init_plasma()
+        assert faults(fake) == []
+        sim.set_phi(two_columns(p))
+        assert faults(fake) == []
+        sim.poisson_solver(1e-9, 1, 320, 32)
+        sim.step(2)
+        assert fake.fake_launches(b"k_jacobi") > 0
+        assert faults(fake) == []
