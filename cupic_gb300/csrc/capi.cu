@@ -539,6 +539,24 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
   CU(cudaEventCreate(&e1));
   float best = 1e30f;
   SolveLayout pick = cands.front();
+  // The precision form may tune in the middle of a run (set_phi_both): its trials
+  // sweep the correction's buffer, put their field where a solve puts its
+  // source, and report to a control block of their own.
+  SimArgs a = c->a;
+  Ctl *ctl = nullptr;
+  if (c->phi64) {
+    cudaError_t e = dalloc(c, &ctl, 1);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ctl, 0, sizeof(Ctl), c->stream);
+    if (e != cudaSuccess) {
+      dfree(c, ctl);
+      free_solve_scratch(c, &scratch);
+      return cuda_status(e);
+    }
+    static_assert(sizeof(float2) == sizeof(double), "field in the place of the source");
+    a.phi = c->dl;
+    a.E = reinterpret_cast<float2 *>(c->b64);
+    a.ctl = ctl;
+  }
   for (const SolveLayout &cd : cands) {
     // write_stats keeps the residual checks of the real solve (a solve with
     // no tolerance that reports nothing skips them); the stats it writes
@@ -549,7 +567,7 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
     bool ok = true;
     for (int rep = 0; rep < 3 && ok; ++rep) {
       ok = cudaEventRecord(e0, c->stream) == cudaSuccess &&
-           launch_jacobi(c->a, J, c->stream) == cudaSuccess &&
+           launch_jacobi(a, J, c->stream) == cudaSuccess &&
            cudaEventRecord(e1, c->stream) == cudaSuccess &&
            cudaEventSynchronize(e1) == cudaSuccess;
       float ms = 0.0f;
@@ -567,8 +585,9 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   // a solve that gave up waiting leaves a flag: clear what the trials raised
-  CU(cudaMemsetAsync(&c->ctl->step_flags, 0, sizeof(uint32_t), c->stream));
+  if (!ctl) CU(cudaMemsetAsync(&c->ctl->step_flags, 0, sizeof(uint32_t), c->stream));
   CU(cudaStreamSynchronize(c->stream));
+  dfree(c, ctl);
   free_solve_scratch(c, &scratch);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -734,11 +753,7 @@ cudaError_t launch_solve(const cupic_ctx *c, const JacobiArgs &J) {
 int set_phi_both(cupic_ctx *c, const double *phi) {
   const size_t n = (size_t)c->a.nnx * c->a.nny;
   CU(cudaStreamSynchronize(c->stream));  // no kernel of the context still uses phi
-  std::vector<float> h(n);
-  for (size_t k = 0; k < n; ++k) h[k] = (float)phi[k];
-  CU(cudaMemcpy(c->a.phi, h.data(), n * sizeof(float), cudaMemcpyHostToDevice));
   if (c->phi64) {
-    CU(cudaMemcpy(c->phi64, phi, n * sizeof(double), cudaMemcpyHostToDevice));
     // the precision form's tiles take column 0 for its mirror, column nnx-1,
     // whose FP64 value otherwise keeps its own start: a potential with two
     // different columns there is solved by the launches that read both
@@ -748,9 +763,17 @@ int set_phi_both(cupic_ctx *c, const double *phi) {
     if (!same && c->lay.tile.R) {
       c->no_tiles = true;
       destroy_graph(c);
-      return plan_jacobi(c);
+      const int rc = plan_jacobi(c);
+      if (rc) {
+        c->no_tiles = false;
+        return rc;
+      }
     }
   }
+  std::vector<float> h(n);
+  for (size_t k = 0; k < n; ++k) h[k] = (float)phi[k];
+  CU(cudaMemcpy(c->a.phi, h.data(), n * sizeof(float), cudaMemcpyHostToDevice));
+  if (c->phi64) CU(cudaMemcpy(c->phi64, phi, n * sizeof(double), cudaMemcpyHostToDevice));
   return CUPIC_OK;
 }
 

@@ -5,9 +5,8 @@
 //
 // Looked at, for every launch: shared memory against the kernel's limit (48 KB
 // of static and dynamic memory together, unless the limit was raised), and for
-// the solves the scratch that the layout reaches.  A solve also leaves marks
-// where it would write: kMark in its potential and field, kMarkSweeps in the
-// report.
+// the solves the scratch that the layout reaches.  A solve also leaves its
+// number where it would write: in its potential and field, and in the report.
 #include <cuda_runtime.h>
 #include <string.h>
 
@@ -27,8 +26,6 @@ namespace {
 constexpr size_t kDefaultSmem = 48 * 1024;
 constexpr size_t kStaticSmem = 720;  // of every kernel
 constexpr int kSms = 152, kMaxSmem = 232448;
-constexpr float kMark = 7.0f;
-constexpr int kMarkSweeps = 77;
 
 struct Kernel {
   std::string name;
@@ -44,6 +41,7 @@ std::vector<std::string> launches;  // names, in order, with those captured
 bool capturing = false;
 int give_up_ctas = -1, give_up_depth = -1;
 float last_ms = 1.0f;
+int solves = 0;
 size_t allocated = 0;
 
 void fault(const std::string &s) { faults.push_back(s); }
@@ -103,18 +101,19 @@ void solve(const std::string &name, const SimArgs &a, const JacobiArgs &J, dim3 
   }
   if (capturing) return;
   const size_t nodes = (size_t)a.nnx * a.nny;
+  const float mark = (float)++solves;
   float *phi = J.phi ? J.phi : a.phi;
   need("phi", phi, nodes * 4, who);
-  if (room(phi) >= nodes * 4) std::fill(phi, phi + nodes, kMark);
+  if (room(phi) >= nodes * 4) std::fill(phi, phi + nodes, mark);
   if (J.do_field) {
     need("E", a.E, nodes * 8, who);
-    if (room(a.E) >= nodes * 8) std::fill(a.E, a.E + nodes, make_float2(kMark, kMark));
+    if (room(a.E) >= nodes * 8) std::fill(a.E, a.E + nodes, make_float2(mark, mark));
   }
   if (J.r64_phi) {
     need("phi64", J.r64_phi, nodes * 8, who);
-    if (room(J.r64_phi) >= nodes * 8) std::fill(J.r64_phi, J.r64_phi + nodes, (double)kMark);
+    if (room(J.r64_phi) >= nodes * 8) std::fill(J.r64_phi, J.r64_phi + nodes, (double)mark);
   }
-  if (J.write_stats || J.r64_stats) a.ctl->sweeps = kMarkSweeps;
+  if (J.write_stats || J.r64_stats) a.ctl->sweeps = solves;
   const bool gave_up = a.ctl->abort != 0;
   if (gave_up) fault(who + ": begins with the flag of a solve that gave up");
   last_ms = gave_up || (J.G == give_up_ctas && J.depth == give_up_depth) ? 1e-3f : 1.0f;

@@ -1,7 +1,7 @@
 """The library's host code without a GPU: its objects linked with a runtime that
 looks at launches instead of running them (fake_cuda/runtime.cu).  Layouts,
 tuner trials and scratch of the solves are held against the buffers that the
-launches get, and a solve leaves marks where it would write."""
+launches get, and a solve leaves its number where it would write."""
 import ctypes
 import glob
 import os
@@ -15,7 +15,6 @@ import cupic_gb300 as cg
 from cupic_gb300 import build
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-MARK = 7.0
 
 
 @pytest.fixture(scope="session")
@@ -93,4 +92,22 @@ def test_two_seam_columns_keep_launches_inside_their_buffers(fake, ncx, ncy):
         sim.poisson_solver(1e-9, 1, 320, 32)
         sim.step(2)
         assert fake.fake_launches(b"k_jacobi") > 0
+        assert faults(fake) == []
+
+
+@pytest.mark.parametrize("ncx,ncy", MESHES)
+def test_two_seam_columns_change_the_potential_alone(fake, ncx, ncy):
+    """The tuner's trials after such a potential leave the field, the report and
+    the potential just set alone."""
+    p = params(ncx, ncy, refine_every=32, max_sweeps=320)
+    with cg.Sim(p) as sim:
+        sim.init_plasma()
+        sim.poisson_solver(1e-9, 1, 320, 32)
+        field = sim.efield()
+        phi = two_columns(p)
+        sim.set_phi(phi)
+        np.testing.assert_array_equal(sim.phi64(), phi)
+        np.testing.assert_array_equal(sim.phi(), phi.astype(np.float32))
+        for g, o in zip(sim.efield(), field):
+            np.testing.assert_array_equal(g, o)
         assert faults(fake) == []
