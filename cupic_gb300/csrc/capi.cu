@@ -416,7 +416,7 @@ TileForm tile_form(const cupic_ctx *c) { return c->p.refine_every > 0 ? kTileRef
 
 // whether the context's solves may run as register tiles
 bool tiles_apply(const cupic_ctx *c) {
-  return !c->no_tiles && !getenv("CUPIC_JACOBI_NOSTRIP") && !getenv("CUPIC_JACOBI_SCALAR");
+  return !c->left.R && !getenv("CUPIC_JACOBI_NOSTRIP") && !getenv("CUPIC_JACOBI_SCALAR");
 }
 
 // The fixed rule, used when tuning is off or a layout is forced with
@@ -750,26 +750,32 @@ cudaError_t launch_solve(const cupic_ctx *c, const JacobiArgs &J) {
   return c->lay.tile.R ? launch_tile(c->a, J, c->lay.tile, c->stream) : launch_jacobi(c->a, J, c->stream);
 }
 
+// Before a potential is stored whose columns 0 and nnx-1 differ (two) or not.  The
+// precision form's tiles take column 0 for its mirror, column nnx-1, whose
+// FP64 value otherwise keeps its own start: two different columns there are
+// solved by the launches that read both.
+int seam_columns(cupic_ctx *c, bool two) {
+  if (!c->phi64 || (two ? !c->lay.tile.R : !c->left.R)) return CUPIC_OK;
+  destroy_graph(c);
+  if (!two) {
+    const int rc = set_tile_plan(c, c->left);
+    if (!rc) c->left.R = 0;
+    return rc;
+  }
+  c->left = c->lay.tile;
+  const int rc = plan_jacobi(c);
+  if (rc) c->left.R = 0;
+  return rc;
+}
+
 int set_phi_both(cupic_ctx *c, const double *phi) {
   const size_t n = (size_t)c->a.nnx * c->a.nny;
   CU(cudaStreamSynchronize(c->stream));  // no kernel of the context still uses phi
-  if (c->phi64) {
-    // the precision form's tiles take column 0 for its mirror, column nnx-1,
-    // whose FP64 value otherwise keeps its own start: a potential with two
-    // different columns there is solved by the launches that read both
-    const int nnx = c->a.nnx;
-    bool same = true;
-    for (int j = 0; j < c->a.nny; ++j) same = same && phi[(size_t)j * nnx] == phi[(size_t)j * nnx + nnx - 1];
-    if (!same && c->lay.tile.R) {
-      c->no_tiles = true;
-      destroy_graph(c);
-      const int rc = plan_jacobi(c);
-      if (rc) {
-        c->no_tiles = false;
-        return rc;
-      }
-    }
-  }
+  const int nnx = c->a.nnx;
+  bool same = true;
+  for (int j = 0; j < c->a.nny; ++j) same = same && phi[(size_t)j * nnx] == phi[(size_t)j * nnx + nnx - 1];
+  const int rc = seam_columns(c, !same);
+  if (rc) return rc;
   std::vector<float> h(n);
   for (size_t k = 0; k < n; ++k) h[k] = (float)phi[k];
   CU(cudaMemcpy(c->a.phi, h.data(), n * sizeof(float), cudaMemcpyHostToDevice));
@@ -778,6 +784,8 @@ int set_phi_both(cupic_ctx *c, const double *phi) {
 }
 
 int set_linear_phi(cupic_ctx *c) {  // init.cu:235-241, on the device
+  const int rc = seam_columns(c, false);
+  if (rc) return rc;
   CU(launch_linear_phi(c->a, c->p.phi_p, c->phi64, c->stream));
   return CUPIC_OK;
 }

@@ -38,7 +38,10 @@ struct cupic_ctx {
   std::vector<int32_t> cap[2];
   int64_t total_cap[2] = {0, 0};
   SolveLayout lay;
-  bool no_tiles = false;  // the precision form's potential needs the launches of jacobi.cu
+  // the register tiles that the precision form has left for the launches of
+  // jacobi.cu, until its potential's two columns at the seam are equal again
+  // (R == 0: not left)
+  cupic::TilePlan left{};
   // exchanges enqueued since the halo words were last zeroed (see epoch_guard)
   int64_t epoch_use = 0;
   // precision form of the solve (refine_every > 0): FP64 potential, FP32

@@ -46,3 +46,31 @@ def test_two_seam_columns_change_the_potential_alone(gpu_lib, monkeypatch, ncx, 
         g, o = sim.stats(1)[0], ora.stats()
         assert g["sweeps"] == o["sweeps"] and g["residual"] == o["residual"]
     ora.close()
+
+
+def test_equal_seam_columns_bring_the_tiles_back(gpu_lib):
+    p = cg.workload_params("tiny", ncx=96, ncy=200, n=2.0, refine_every=8, tol=1e-9, min_sweeps=8, max_sweeps=40,
+                           init_tol=1e-9, init_min_sweeps=8, init_max_sweeps=40)
+    ora = Oracle(p, fp64=False)
+    ora.init_plasma()
+    with cg.Sim(p) as sim:
+        sim.init_plasma()
+        plan = sim.solver_plan()
+        for dphi in (0.125, 0.0, 0.25, None):
+            if dphi is None:
+                sim.init_plasma()
+                ora.init_plasma()
+            else:
+                phi = ora.phi()
+                phi[:, -1] = phi[:, 0]
+                phi[1:-1, -1] += dphi
+                sim.set_phi(phi)
+                ora.set_phi(phi)
+            if not dphi:
+                assert sim.solver_plan() == plan
+            sim.step(2)
+            ora.step(2)
+            np.testing.assert_array_equal(sim.phi64(), ora.phi())
+            for s in (0, 1):
+                np.testing.assert_array_equal(sim.particles(s), ora.particles(s))
+    ora.close()

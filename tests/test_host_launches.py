@@ -111,3 +111,36 @@ def test_two_seam_columns_change_the_potential_alone(fake, ncx, ncy):
         for g, o in zip(sim.efield(), field):
             np.testing.assert_array_equal(g, o)
         assert faults(fake) == []
+
+
+@pytest.mark.parametrize("back", ("set_phi", "init_plasma", "init_mesh"))
+@pytest.mark.parametrize("ctas", (None, "5"))
+def test_equal_seam_columns_bring_the_tiles_back(fake, monkeypatch, back, ctas):
+    """Once the columns at the seam are equal again the solves are tiles again, in
+    the layout of before and without a trial."""
+    if ctas:
+        monkeypatch.setenv("CUPIC_JACOBI_CTAS", ctas)
+    p = params(64, 90, refine_every=32, max_sweeps=320)
+    with cg.Sim(p) as sim:
+        sim.init_plasma()
+        sim.step(1)
+        plan = sim.solver_plan()
+        sim.set_phi(two_columns(p))
+        sim.step(1)
+        for _ in range(2):  # and out again, to the same layout
+            monkeypatch.delenv("CUPIC_JACOBI_CTAS", raising=False)
+            if back == "set_phi":
+                sim.set_phi(two_columns(p, 0.0))
+            fake.fake_reset()
+            if back != "set_phi":
+                getattr(sim, back)()
+            sim.poisson_solver(1e-9, 1, 320, 32)
+            assert fake.fake_launches(b"k_jacobi") == 0
+            assert fake.fake_launches(b"k_tile") == (1 if back == "set_phi" else 2)
+            assert sim.solver_plan() == plan
+            sim.step(1)
+            sim.set_phi(two_columns(p))
+            fake.fake_reset()
+            sim.poisson_solver(1e-9, 1, 320, 32)
+            assert fake.fake_launches(b"k_tile") == 0 and fake.fake_launches(b"k_jacobi") == 11
+        assert faults(fake) == []
