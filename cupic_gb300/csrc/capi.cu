@@ -1448,7 +1448,7 @@ int cupic_create(const cupic_params *pin, int device, cupic_ctx **out) {
   }
   rc = plan_jacobi(c);
   if (rc) return fail(rc);
-  if (push_set_smem(push_smem_bytes(a.nnx)) != cudaSuccess) return fail(CUPIC_ERR_ARG);
+  if (push_set_smem(push_smem_bytes(a.nnx)) != cudaSuccess || tail_set_smem(a) != cudaSuccess) return fail(CUPIC_ERR_ARG);
   rc = cupic_set_time(c, (int64_t)c->p.n_ini + 1, c->p.n_ini * c->p.dt + c->p.dt, -1.0, -1.0);
   if (rc) return fail(rc);
   *out = c;

@@ -32,6 +32,7 @@ cudaError_t launch_inject_append(const SimArgs &a, cudaStream_t st);
 cudaError_t launch_finalize(const SimArgs &a, cudaStream_t st);
 // room check, arrivals, append and bookkeeping in one launch
 bool tail_applies(const SimArgs &a);
+cudaError_t tail_set_smem(const SimArgs &a);
 cudaError_t launch_tail(const SimArgs &a, int num_sms, cudaStream_t st);
 // room check between the push and the arrivals (sets ctl->halt), and the
 // move of a species' rows into a larger layout

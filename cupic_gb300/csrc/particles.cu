@@ -1302,8 +1302,13 @@ cudaError_t launch_inject_draw(const SimArgs &a, cudaStream_t st) {
 }
 
 // The step's end in one launch, where a CTA's shared memory holds the counts of
-// all rows; a warp for every (row, species), two CTAs to an SM at most.
+// all rows (48 KB: 4096 rows; from 4086 on an opt-in, for the static part); a
+// warp for every (row, species), two CTAs to an SM at most.
 bool tail_applies(const SimArgs &a) { return 3 * a.ncy * sizeof(int) <= 48 * 1024; }
+
+cudaError_t tail_set_smem(const SimArgs &a) {
+  return tail_applies(a) ? raise_dyn_smem(reinterpret_cast<const void *>(k_tail), 3 * a.ncy * sizeof(int)) : cudaSuccess;
+}
 
 cudaError_t launch_tail(const SimArgs &a, int num_sms, cudaStream_t st) {
   const int nw = kTailBlock / 32, ctas = min(2 + (2 * a.ncy + nw - 1) / nw, 2 * num_sms);

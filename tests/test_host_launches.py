@@ -144,3 +144,16 @@ def test_equal_seam_columns_bring_the_tiles_back(fake, monkeypatch, back, ctas):
             sim.poisson_solver(1e-9, 1, 320, 32)
             assert fake.fake_launches(b"k_tile") == 0 and fake.fake_launches(b"k_jacobi") == 11
         assert faults(fake) == []
+
+
+@pytest.mark.parametrize("ncy,tail", [(4035, 1), (4036, 1), (4085, 1), (4086, 1), (4096, 1), (4097, 0)])
+def test_end_of_step_at_its_most_rows(fake, ncy, tail):
+    """The end of a step in one launch holds three counts of every row in shared
+    memory, up to 4096 rows; beyond, four launches."""
+    p = params(2, ncy, max_sweeps=10)
+    with cg.Sim(p) as sim:
+        sim.init_plasma()
+        fake.fake_reset()
+        sim.step(1)
+        assert fake.fake_launches(b"k_tail") == tail and fake.fake_launches(b"k_finalize") == 1 - tail
+        assert faults(fake) == []
