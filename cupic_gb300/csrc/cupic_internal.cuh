@@ -143,8 +143,9 @@ struct JGroup {
 
 // Set by the room check of a step whose arrivals do not fit their rows; the
 // host grows those rows and completes the step.  Every kernel of a step
-// reads it first and returns when it is set: the flag changes only between
-// kernels, so the whole grid sees one value.
+// reads it first and returns when it is set.  The flag changes between kernels,
+// so the whole grid sees one value, and in k_tail, whose CTAs agree on the one
+// that they saw.
 __device__ __forceinline__ bool halted(const Ctl *ctl) {
   return *reinterpret_cast<const volatile int32_t *>(&ctl->halt) != 0;
 }

@@ -1125,11 +1125,14 @@ __global__ void __launch_bounds__(kTailBlock, 2) k_tail(SimArgs a) {
     s_live[tid] = 0ull;
     s_rem[tid] = 0u;
   }
-  if (halt) {  // as finalize(): the host reruns the steps counted here
+  // Rank 0 may set the flag (below) while a CTA that starts later reads it, so one
+  // that finds it in any thread returns as a whole: its warps could otherwise
+  // part, and those left would check only their own rows and draws, and append
+  // to a step that the host completes.
+  if (__syncthreads_or(halt)) {  // as finalize(): the host reruns the steps counted here
     if (rank == 0 && tid == 0) ctl->skipped += 1;
     return;
   }
-  __syncthreads();
   for (int sp = 0; sp < 2; ++sp)
     for (int k = tid; k < ne[sp]; k += kTailBlock) {
       const int d = a.sp[sp].inj_d[k];
@@ -1151,7 +1154,7 @@ __global__ void __launch_bounds__(kTailBlock, 2) k_tail(SimArgs a) {
       live[sp] += (unsigned long long)need;
     }
   if (__syncthreads_or(over)) {
-    // every CTA finds the same; one that reads the flag first returns above
+    // every CTA finds the same, or the flag above
     if (rank == 0 && tid == 0) {
       ctl->skipped += 1;
       atomicExch(&ctl->halt, 1);
