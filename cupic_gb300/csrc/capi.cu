@@ -491,6 +491,20 @@ SolveLayout on_scratch(SolveLayout l, const SolveLayout &scratch) {
   return l;
 }
 
+// Whether a trial that has ended gave up a bounded wait.  It has then run a part
+// of its sweeps, so its time says nothing, and its flags, cleared here, would
+// make the trials after it stop early as well.
+int trial_gave_up(cupic_ctx *c, Ctl *ctl, bool *gave_up) {
+  int32_t flag = 0;
+  CU(cudaMemcpyAsync(&flag, &ctl->abort, sizeof(flag), cudaMemcpyDeviceToHost, c->stream));
+  CU(cudaStreamSynchronize(c->stream));
+  *gave_up = flag != 0;
+  if (!flag) return CUPIC_OK;
+  CU(cudaMemsetAsync(&ctl->step_flags, 0, sizeof(ctl->step_flags), c->stream));
+  CU(cudaMemsetAsync(&ctl->abort, 0, sizeof(ctl->abort), c->stream));
+  return CUPIC_OK;
+}
+
 int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
   const int M = c->a.nny - 2;
   const int chk = std::max(1, c->p.check_every);
@@ -538,13 +552,14 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
   float best = 1e30f;
-  SolveLayout pick = cands.front();
+  SolveLayout pick;  // G == 0: none
+  pick.G = 0;
   // The precision form may tune in the middle of a run (set_phi_both): its trials
   // sweep the correction's buffer, put their field where a solve puts its
   // source, and report to a control block of their own.
   SimArgs a = c->a;
-  Ctl *ctl = nullptr;
   if (c->phi64) {
+    Ctl *ctl = nullptr;
     cudaError_t e = dalloc(c, &ctl, 1);
     if (e == cudaSuccess) e = cudaMemsetAsync(ctl, 0, sizeof(Ctl), c->stream);
     if (e != cudaSuccess) {
@@ -577,18 +592,20 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
       cudaGetLastError();
       continue;
     }
-    if (t < best) {
+    bool gave_up = false;
+    rc = trial_gave_up(c, a.ctl, &gave_up);
+    if (rc) break;
+    if (!gave_up && t < best) {
       best = t;
       pick = cd;
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  // a solve that gave up waiting leaves a flag: clear what the trials raised
-  if (!ctl) CU(cudaMemsetAsync(&c->ctl->step_flags, 0, sizeof(uint32_t), c->stream));
-  CU(cudaStreamSynchronize(c->stream));
-  dfree(c, ctl);
+  if (a.ctl != c->ctl) dfree(c, a.ctl);
   free_solve_scratch(c, &scratch);
+  if (rc) return rc;
+  if (!pick.G) return plan_jacobi_rule(c, P, rows_fit);
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tuned[key] = {pick.G, pick.K, pick.nostrip};
@@ -599,7 +616,7 @@ int tune_jacobi(cupic_ctx *c, int P, long long rows_fit) {
 // Register tiles: the layouts with the lowest estimated cost are timed on
 // the context's buffers, with the checks of the solve it will run, and the
 // fastest is kept, per device, mesh shape and check interval.  Returns
-// CUPIC_ERR_CAPACITY when no layout holds the mesh.
+// CUPIC_ERR_CAPACITY when no layout holds the mesh, or none could be timed.
 struct TileKey {
   int device, nnx, nny, chk, sweeps, early, refine;
   bool operator<(const TileKey &o) const {
@@ -640,8 +657,9 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
   TilePlan pick = cands.front();
   if (cands.size() > 1) {
     SolveLayout scratch;
-    const int rc = alloc_solve_scratch(c, &scratch, maxG, words);
+    int rc = alloc_solve_scratch(c, &scratch, maxG, words);
     if (rc) return rc;
+    pick.R = 0;  // none
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     CU(cudaEventCreate(&e0));
     CU(cudaEventCreate(&e1));
@@ -664,18 +682,19 @@ int tune_tiles(cupic_ctx *c, int dev_max) {
         cudaGetLastError();
         continue;
       }
-      if (ms_best < best) {
+      bool gave_up = false;
+      rc = trial_gave_up(c, c->ctl, &gave_up);
+      if (rc) break;
+      if (!gave_up && ms_best < best) {
         best = ms_best;
         pick = t;
       }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    // a solve that gave up waiting leaves two flags: clear what the trials raised
-    CU(cudaMemsetAsync(&c->ctl->step_flags, 0, sizeof(uint32_t), c->stream));
-    CU(cudaMemsetAsync(&c->ctl->abort, 0, sizeof(c->ctl->abort), c->stream));
-    CU(cudaStreamSynchronize(c->stream));
     free_solve_scratch(c, &scratch);
+    if (rc) return rc;
+    if (!pick.R) return CUPIC_ERR_CAPACITY;
   }
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);

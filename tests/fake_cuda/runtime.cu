@@ -114,10 +114,10 @@ void solve(const std::string &name, const SimArgs &a, const JacobiArgs &J, dim3 
     if (room(J.r64_phi) >= nodes * 8) std::fill(J.r64_phi, J.r64_phi + nodes, (double)mark);
   }
   if (J.write_stats || J.r64_stats) a.ctl->sweeps = solves;
-  const bool gave_up = a.ctl->abort != 0;
-  if (gave_up) fault(who + ": begins with the flag of a solve that gave up");
-  last_ms = gave_up || (J.G == give_up_ctas && J.depth == give_up_depth) ? 1e-3f : 1.0f;
-  if (J.G == give_up_ctas && J.depth == give_up_depth) {
+  const bool gives_up = J.G == give_up_ctas && J.depth == give_up_depth;
+  if (a.ctl->abort && !gives_up) fault(who + ": begins with the flag of another that gave up");
+  last_ms = a.ctl->abort || gives_up ? 1e-3f : 1.0f;
+  if (gives_up) {
     a.ctl->abort = 1;
     a.ctl->step_flags |= CUPIC_FLAG_TIMEOUT;
   }

@@ -157,3 +157,22 @@ def test_end_of_step_at_its_most_rows(fake, ncy, tail):
         sim.step(1)
         assert fake.fake_launches(b"k_tail") == tail and fake.fake_launches(b"k_finalize") == 1 - tail
         assert faults(fake) == []
+
+
+@pytest.mark.parametrize("ncx,ncy,form", [(64, 90, "tiles"), (256, 1024, "tiles"), (64, 90, "sweeps"), (256, 1024, "sweeps")])
+def test_trial_that_gives_up_is_left_out(fake, monkeypatch, ncx, ncy, form):
+    """A trial whose bounded wait expired ran only a part of its sweeps: it is no
+    candidate however fast it was, and the trials after it start without its
+    flags, as does the context."""
+    if form == "sweeps":
+        monkeypatch.setenv("CUPIC_JACOBI_NOSTRIP", "1")  # no register tiles
+    p = params(ncx, ncy, max_sweeps=100, init_max_sweeps=100)
+    with cg.Sim(p) as sim:  # the pick without a fault, kept for the shape
+        first = sim.solver_plan()
+    p = params(ncx, ncy, max_sweeps=101, init_max_sweeps=101)  # another solve to the tuner
+    fake.fake_give_up(first[0], first[2])
+    with cg.Sim(p) as sim:
+        sim.init_plasma()
+        assert sim.flags() == 0
+        assert (sim.solver_plan()[0], sim.solver_plan()[2]) != (first[0], first[2])
+    assert faults(fake) == []
