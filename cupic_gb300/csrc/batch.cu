@@ -435,11 +435,22 @@ int tune_solve(cupic_batch *b) {
       pick = k;
     }
   }
+  // Once a trial's bounded wait has expired, it and the trials after it stop
+  // early: their times say nothing, and the default knobs stay.
+  std::vector<int32_t> gave_up(n, 1);
+  for (int i = 0; i < n; ++i)
+    if (cudaMemcpyAsync(&gave_up[i], &b->members[i]->ctl->abort, sizeof(int32_t), cudaMemcpyDeviceToHost, b->stream) !=
+        cudaSuccess)
+      cudaGetLastError();
   e = copy_all(true);
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
   cudaFree(save);
   if (rc) return rc;
   if (e != cudaSuccess) return CUPIC_ERR_CUDA;
+  if (std::any_of(gave_up.begin(), gave_up.end(), [](int32_t v) { return v != 0; })) {
+    b->tuned_n = 0;
+    return layout_solve(b, kDefaultKnobs);
+  }
   {
     std::lock_guard<std::mutex> lk(g_mix_mu);
     g_mix_tuned[{b->device, key}] = pick;

@@ -39,7 +39,7 @@ std::map<const void *, std::pair<void *, size_t>> symbols;
 std::vector<std::string> faults;
 std::vector<std::string> launches;  // names, in order, with those captured
 bool capturing = false;
-int give_up_ctas = -1, give_up_depth = -1;
+int give_up_ctas = -1, give_up_depth = -1, batch_give_up = -1;
 float last_ms = 1.0f;
 int solves = 0;
 size_t allocated = 0;
@@ -135,6 +135,14 @@ cudaError_t launch(const void *fn, dim3 grid, dim3 block, void **args, size_t sm
   if (k.name.find("k_tile") != std::string::npos ||
       (k.name.find("k_jacobi") != std::string::npos && k.name.find("batch") == std::string::npos))
     solve(k.name, *static_cast<const SimArgs *>(args[0]), *static_cast<const JacobiArgs *>(args[1]), grid, smem);
+  if (k.name.find("k_jacobi_batch") != std::string::npos && !capturing) {
+    const SimArgs *inst = *static_cast<const SimArgs *const *>(args[0]);
+    const int n = (int)(room(inst) / sizeof(SimArgs));
+    last_ms = 1.0f;
+    for (int i = 0; i < n; ++i)
+      if (inst[i].ctl->abort) last_ms = 1e-3f;
+    if (batch_give_up >= 0 && batch_give_up-- == 0) inst[n - 1].ctl->abort = 1;
+  }
   return cudaSuccess;
 }
 
@@ -163,10 +171,12 @@ void fake_give_up(int ctas, int depth) {
   give_up_ctas = ctas;
   give_up_depth = depth;
 }
+// the n-th batched solve from now gives up, in its last member
+void fake_batch_give_up(int n) { batch_give_up = n; }
 void fake_reset() {
   faults.clear();
   launches.clear();
-  give_up_ctas = give_up_depth = -1;
+  give_up_ctas = give_up_depth = batch_give_up = -1;
   allocated = 0;
 }
 void *fake_alloc(unsigned long long n) { return take(n); }

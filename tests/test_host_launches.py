@@ -176,3 +176,24 @@ def test_trial_that_gives_up_is_left_out(fake, monkeypatch, ncx, ncy, form):
         assert sim.flags() == 0
         assert (sim.solver_plan()[0], sim.solver_plan()[2]) != (first[0], first[2])
     assert faults(fake) == []
+
+
+def test_batched_trial_that_gives_up_tunes_nothing(fake):
+    """The batched solve's trials run on the members: once one has given up, those
+    after it stop early, so the knobs stay the default ones and are not kept."""
+    p = params(16, 40)
+    sims = [cg.Sim(p) for _ in range(16)]
+    for s in sims:
+        s.init_plasma()
+    plans = []
+    for n in (4, None):  # the second candidate's second launch; no trial
+        if n is not None:
+            fake.fake_batch_give_up(n)
+        with cg.Batch(sims) as b:
+            plans.append((b.plan(), fake.fake_launches(b"k_jacobi_batch")))
+        assert all(s.flags() == 0 for s in sims)
+    assert plans[0][0][:2] == (4, 1)
+    assert plans[1][1] > plans[0][1]  # tuned again
+    for s in sims:
+        s.close()
+    assert faults(fake) == []
