@@ -307,6 +307,7 @@ int layout_solve(cupic_batch *b, const Knobs &kn) {
     J.bar = J.flags + q.G;
     J.res_cta = b->d_res + orr;
     J.halo = b->d_halo + oh;
+    J.gmax = c->lay.gmax;  // cleared by the solve in which the member's epochs start over
     of += q.G + 1;
     orr += 2 * q.G;
     oh += (size_t)4 * q.G * q.K * q.P;

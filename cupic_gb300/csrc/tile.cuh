@@ -766,10 +766,8 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     unsigned next = ebase + (unsigned)used + 2u;
     const bool wrap = next > kEpochEnd;  // start over, above the tags left in gmax
     if (wrap) next = 0u;
-    if (G > 1) {
-      for (int k = 0; k < 4; ++k) J.tbar[k] = 0u;
-      for (int k = 0; k < (wrap ? 128 : REFINE ? 4 : 0); ++k) J.gmax[k] = 0ull;
-    }
+    for (int k = 0; k < (G > 1 ? 4 : 0); ++k) J.tbar[k] = 0u;
+    for (int k = 0; k < (wrap ? 128 : REFINE && G > 1 ? 4 : 0); ++k) J.gmax[k] = 0ull;
     ctl->jepoch = next;
   };
 
