@@ -143,19 +143,17 @@ struct Lane {
   bool full;         // no lane of the warp has a partial strip
 };
 
-// The strips hold s = 4 phi, the sum of a node before its product by 1/4: the
-// product of a neighbour's sum is exact, so a fused multiply-add rounds as the
-// sum with the neighbour's phi does, and a node takes four operations instead
-// of five.  (phi below 2^-124 in size, whose product by 1/4 would be rounded
-// to a subnormal, is carried exactly instead.)
+// A node is formed from quarters, with b a quarter of the source term: a product
+// by 1/4 is exact, so a fused multiply-add rounds a quarter of what the sum does
+// to a quarter of what the sum rounds to, and a node takes four operations
+// instead of five.  (Two differences.  Sums below 2^-124 in size are rounded as
+// subnormals, where the sum would be exact and its quarter rounded once: by
+// 2^-150 at most for each of the four.  Sums of 2^128 and more are finite where
+// their quarter is.)
 __device__ __forceinline__ float node(float b, float w, float e, float n, float s) {
   return __fmaf_rn(0.25f, s, __fmaf_rn(0.25f, n, __fmaf_rn(0.25f, e, __fmaf_rn(0.25f, w, b))));
 }
-__device__ __forceinline__ float times4f(float v) { return __fmul_rn(4.0f, v); }
 __device__ __forceinline__ float quarter(float v) { return __fmul_rn(0.25f, v); }
-__device__ __forceinline__ float4 quarter(const float4 &v) {
-  return make_float4(quarter(v.x), quarter(v.y), quarter(v.z), quarter(v.w));
-}
 
 // The source term of fixed-point charge f, (float)((double)f * cb).  Three FP64
 // operations a node were 13 us of a 512x2048 solve; the product in
@@ -209,7 +207,7 @@ __device__ __forceinline__ double times4(double v) {
   return __hiloint2double(hi + 0x200000, __double2loint(v));
 }
 
-// One sweep of a strip: v = (((b + west) + east) + north) + south on s = 4 phi.
+// One sweep of a strip: v = ((((b + west) + east) + north) + south) / 4.
 // FULL: all R rows of the strip are in the tile (the row above the last is
 // then x[R]'s place, taken from n4); otherwise the rows past the strip's end
 // compute values nothing reads.  FIRST: the solve's first sweep, which reads
@@ -241,7 +239,7 @@ __device__ __forceinline__ float sweep(float4 (&x)[R], const float4 (&b)[R], con
     }
     e.w = rt;
     float mir = 0.0f;
-    if (FIRST && r < g.nvalid) mir = times4f(mirror[r]);
+    if (FIRST && r < g.nvalid) mir = mirror[r];
     if (FIRST && g.me >= 0) {
       e.x = g.me == 0 ? mir : e.x;
       e.y = g.me == 1 ? mir : e.y;
@@ -467,9 +465,9 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     const df cb = df_of(a.cb);
     for (int k = tid; k < 2 * tp; k += nthr) {
       const int up = k >= tp ? 1 : 0, tc = k - up * tp;
-      const float p4 = times4f(timg0[up * (rows + 1) * tp + tc]);
+      const float v = timg0[up * (rows + 1) * tp + tc];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) edge[(2 * q + up) * 128 + tc] = p4;
+      for (int q = 0; q < 4; ++q) edge[(2 * q + up) * 128 + tc] = v;
     }
     // the strip's source terms, in the place of its charges; column 0 (or its
     // image past column W-1) is folded with the mirror column
@@ -485,18 +483,17 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
         u.y += z == 1 ? m : 0ll;
         v.x += z == 2 ? m : 0ll;
         v.y += z == 3 ? m : 0ll;
-        seam = seam || !(times4f(mcol[j]) == times4f(timg[j * tp + 4 * li + z]));
+        seam = seam || !(mcol[j] == timg[j * tp + 4 * li + z]);
       }
-      sts4(reinterpret_cast<float *>(ar), make_float4(source(u.x, a.cb, cb, pow2), source(u.y, a.cb, cb, pow2),
-                                                      source(v.x, a.cb, cb, pow2), source(v.y, a.cb, cb, pow2)));
+      auto b4 = [&](long long f) { return quarter(source(f, a.cb, cb, pow2)); };
+      sts4(reinterpret_cast<float *>(ar), make_float4(b4(u.x), b4(u.y), b4(v.x), b4(v.y)));
     }
     seam = __syncthreads_or(seam);
 #pragma unroll
     for (int r = 0; r < R; ++r)
       if (r < g.nvalid) {
         const int j = g.row0 - lo + r;
-        const float4 v = lds4(timg + j * tp + 4 * li);
-        x[r] = make_float4(times4f(v.x), times4f(v.y), times4f(v.z), times4f(v.w));
+        x[r] = lds4(timg + j * tp + 4 * li);
         b[r] = lds4(reinterpret_cast<const float *>(aimg + j * tp + 4 * li));
       }
   } else {
@@ -849,7 +846,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
             double ev = k == 3 ? ze : zc[k < 3 ? k + 1 : 3];
             if (MODE == kRingRagged && g.me == k) ev = z0;
             const double rr = (cc[k] >= 0 ? src[cc[k]] : 0.0) - (times4(zc[k]) - (((wv + ev) + zn[k]) + zs[k]));
-            v[k] = to_float(rr);
+            v[k] = quarter(to_float(rr));
             const unsigned long long bits = (unsigned long long)__double_as_longlong(rr) & 0x7fffffffffffffffull;
             if (((g.own >> k) & 1u) && ((g.ownrows >> r) & 1u) && bits <= inf64 && bits > mx) mx = bits;
           }
@@ -929,10 +926,10 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       };
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (r < g.nvalid) add_row(q64 + r * tp, quarter(x[r]));
-      if (!idle && south_edge && by > 0) add_row(p64 + 4 * li, quarter(lds4(edge + es * 256 + 4 * li)));
+        if (r < g.nvalid) add_row(q64 + r * tp, x[r]);
+      if (!idle && south_edge && by > 0) add_row(p64 + 4 * li, lds4(edge + es * 256 + 4 * li));
       if (!idle && north_edge && by < nby - 1)
-        add_row(p64 + (rows + 1) * tp + 4 * li, quarter(lds4(edge + es * 256 + 128 + 4 * li)));
+        add_row(p64 + (rows + 1) * tp + 4 * li, lds4(edge + es * 256 + 128 + 4 * li));
       done += todo;
       ++q;
       __syncthreads();
@@ -1108,7 +1105,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     }
     Rows at = rows_at(es, p);
     int m = 0;
-    float md = 0.0f;  // four times a sweep's maximum
+    float md = 0.0f;
     if (seam && start == 0) {  // the first sweep reads the caller's mirror column
       md = sweep<R, MODE, false, true, true>(x, b, lds4(at.sA), lds4(at.nA), g, mcol + (g.row0 - lo));
       const unsigned u = __reduce_max_sync(kFull, __float_as_uint(md));
@@ -1134,7 +1131,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
       const unsigned u = __reduce_max_sync(kFull, __float_as_uint(md));
       if (lane == nsw - 1) keep = u;
     }
-    if ((mask >> lane) & 1u) atomicMax(&js->cm[nq & 3][lane], __float_as_uint(quarter(__uint_as_float(keep))));
+    if ((mask >> lane) & 1u) atomicMax(&js->cm[nq & 3][lane], keep);
     // the last exchange serves the field; a solve of less than K sweeps
     // trades once too, so that no CTA stores its rows before its neighbours
     // have loaded them
@@ -1204,10 +1201,10 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
   // E = -grad phi (mesh.cu:413-468) of the owned nodes ----------------------
 #pragma unroll
   for (int r = 0; r < R; ++r)
-    if (r < g.nvalid) sts4(timg + (g.row0 - lo + r) * tp + 4 * li, quarter(x[r]));
+    if (r < g.nvalid) sts4(timg + (g.row0 - lo + r) * tp + 4 * li, x[r]);
   for (int k = tid; k < 2 * tp; k += nthr) {
     const int up = k >= tp ? 1 : 0, tc = k - up * tp;
-    timg0[up * (rows + 1) * tp + tc] = quarter(edge[es * 256 + up * 128 + tc]);
+    timg0[up * (rows + 1) * tp + tc] = edge[es * 256 + up * 128 + tc];
   }
   __syncthreads();
   // a quotient by a power of two is the product by its inverse, exactly
