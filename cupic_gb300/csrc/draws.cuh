@@ -136,7 +136,11 @@ __device__ __forceinline__ void df_sincos2pi_u01(uint32_t r, df *sn, df *cs) {
 // v rounded to float; clears ok when the FP64 value could round to another
 // one.  kDrawEps bounds the relative distance of the two evaluations: the
 // steps above lose a few units of 2^-45, the FP64 ones a few of 2^-52.
+// (In normal floats: the products' low parts are 2^-48 of them and round off
+// near 2^-149, so the constants that the callers multiply by are bounded,
+// df_plain, and beyond those bounds FP64 decides.)
 constexpr float kDrawEps = 0x1p-38f;
+__device__ __forceinline__ bool df_plain(df c, float least, float most) { return c.h >= least && c.h <= most; }
 __device__ __forceinline__ float df_round(df v, bool &ok) {
   const float e = __fmul_rn(fabsf(v.h), kDrawEps);
   const float a = __fadd_rn(v.h, __fadd_rn(v.l, e)), b = __fadd_rn(v.h, __fsub_rn(v.l, e));

@@ -229,8 +229,8 @@ __device__ __noinline__ float4 init_particle_f64(const SimArgs &a, const uint4 r
 
 // the same four floats (draws.cuh)
 __device__ __forceinline__ float4 init_particle(const SimArgs &a, const uint4 r, int j, double sig, df lx,
-                                                df ds, df sigf) {
-  bool ok = j < 32768;  // df_int takes 48 bits
+                                                df ds, df sigf, bool plain) {
+  bool ok = plain;
   const df ux = df_scale(df_int(2ull * r.x + 1ull), 0x1p-33f);
   const df uy = df_scale(df_int(((unsigned long long)(unsigned)j << 33) + 2ull * r.y + 1ull), 0x1p-33f);
   df sn, cs;
@@ -247,10 +247,13 @@ __global__ void __launch_bounds__(256) k_init_particles(SimArgs a) {
   float4 *row = S.parts + S.seg[j];
   const double sig = a.sig[sp];
   const df lx = df_of(a.Lx_d), ds = df_of(a.ds_d), sigf = df_of(sig);
+  // df_int takes 48 bits; a velocity may be 2^-48 of sig, a place 2^-33 of Lx
+  const bool plain =
+      j < 32768 && df_plain(lx, 0x1p-40f, 0x1p75f) && df_plain(ds, 0x1p-40f, 0x1p75f) && df_plain(sigf, 0x1p-40f, 0x1p75f);
   for (int k = threadIdx.x; k < a.ppr; k += blockDim.x) {
     const uint4 r = philox4x32_10(
         make_uint4((uint32_t)k, (uint32_t)j, 0u, (uint32_t)((kPurposeInit << 8) | sp)), a.k0, a.k1);
-    float4 p = init_particle(a, r, j, sig, lx, ds, sigf);
+    float4 p = init_particle(a, r, j, sig, lx, ds, sigf, plain);
     p.x = wrap_x(a, p.x);
     for (int it = 0; it < 16 && row_of(a, p.y) > j; ++it) p.y = nextafterf(p.y, 0.0f);
     for (int it = 0; it < 16 && row_of(a, p.y) < j; ++it) p.y = nextafterf(p.y, a.Ly);

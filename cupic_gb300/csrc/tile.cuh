@@ -158,15 +158,17 @@ __device__ __forceinline__ float quarter(float v) { return __fmul_rn(0.25f, v); 
 // The source term of fixed-point charge f, (float)((double)f * cb).  Three FP64
 // operations a node were 13 us of a 512x2048 solve; the product in
 // double-float arithmetic rounds to the same float (draws.cuh) but for a few
-// nodes in a million and charges of 2^16 units and more, which take FP64.
+// nodes in a million and charges of `most` on, 2^16 units, which take FP64 (all
+// do, most = 0, where cb is so small or large that the products leave the
+// normal floats).
 // (The FP64 fallbacks here and below are calls: inlined, the compiler computes
 // them always and selects.)
 static __device__ __noinline__ float source_f64(long long f, double cb) { return __double2float_rn((double)f * cb); }
 // pow2: cb is a power of two, so the charge's own rounding is the only one.
-__device__ __forceinline__ float source(long long f, double cb, const df &cbf, bool pow2) {
+__device__ __forceinline__ float source(long long f, double cb, const df &cbf, bool pow2, unsigned long long most) {
   const unsigned long long u = f < 0 ? 0ull - (unsigned long long)f : (unsigned long long)f;
   const df n = df_int(u);
-  bool ok = u < (1ull << 48);
+  bool ok = u < most;
   float v = __fmul_rn(n.h, cbf.h);
   if (!pow2) v = df_round(df_mul(n, cbf), ok);
   if (!ok) return source_f64(f, cb);
@@ -463,6 +465,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
     __syncthreads();
     const bool pow2 = (__double_as_longlong(a.cb) & 0xfffffffffffffll) == 0ll;
     const df cb = df_of(a.cb);
+    const unsigned long long most = df_plain(cb, 0x1p-90f, 0x1p75f) ? 1ull << 48 : 0ull;
     for (int k = tid; k < 2 * tp; k += nthr) {
       const int up = k >= tp ? 1 : 0, tc = k - up * tp;
       const float v = timg0[up * (rows + 1) * tp + tc];
@@ -485,7 +488,7 @@ __device__ __forceinline__ void solve(const SimArgs &a, const JacobiArgs &J, con
         v.y += z == 3 ? m : 0ll;
         seam = seam || !(mcol[j] == timg[j * tp + 4 * li + z]);
       }
-      auto b4 = [&](long long f) { return quarter(source(f, a.cb, cb, pow2)); };
+      auto b4 = [&](long long f) { return quarter(source(f, a.cb, cb, pow2, most)); };
       sts4(reinterpret_cast<float *>(ar), make_float4(b4(u.x), b4(u.y), b4(v.x), b4(v.y)));
     }
     seam = __syncthreads_or(seam);
