@@ -12,9 +12,10 @@
 //
 // Such a call still needs scratch memory for the solver CTAs: per-CTA sweep
 // counters, residual slots, the halo rows they trade, and a small status
-// block. Here that scratch is a file-scope static device array of a fixed
-// 8 MiB. Every GPU that loads this library holds it until the process
-// exits. The entry point rejects meshes whose scratch would not fit.
+// block. Here that scratch is two file-scope static device arrays, 8 MiB for
+// the status block and the halo rows and 25 KB for the counters and slots.
+// Every GPU that loads this library holds them until the process exits. The
+// entry point rejects meshes whose scratch would not fit.
 #include <mutex>
 #include <stdlib.h>
 #include <string.h>
@@ -34,9 +35,17 @@ constexpr size_t kCtlHeadBytes = 256;  // the part of Ctl the solver touches
 static_assert(offsetof(Ctl, ring) <= kCtlHeadBytes, "solver status block");
 
 static __device__ __align__(256) unsigned char g_solver_scratch[kStaticScratchBytes];
-// the register tiles' maxima and counters (JacobiArgs::gmax, tbar), apart
-// from the scratch so that no layout's words lie over them
-static __device__ unsigned long long g_solver_sync[130];
+// The counters of all layouts, apart from the scratch: a halo word is told by
+// the epoch in its upper half, so no layout's words may lie where another one
+// leaves other values.
+constexpr int kMaxCtas = 2048;  // four of the sweeps' CTAs (512 threads) on each of 512 SMs
+struct SolverSync {
+  unsigned long long gmax[128];  // the register tiles' maxima and counters (JacobiArgs::gmax, tbar)
+  unsigned tbar[4];
+  unsigned flags[kMaxCtas + 1];  // the sweeps of jacobi.cu: JacobiArgs::flags, then the barrier
+  float res[2 * kMaxCtas];
+};
+static __device__ SolverSync g_solver_sync;
 
 // device addresses of the arrays for each device, looked up once
 std::mutex g_mu;
@@ -50,7 +59,7 @@ long long g_exchanges[kMaxDevices] = {};
 
 // the array's device address on the current device; *clear: the call must
 // zero the halo words first
-int scratch_for_current_device(unsigned char **out, unsigned long long **sync, long long exchanges, bool *clear) {
+int scratch_for_current_device(unsigned char **out, SolverSync **sync, long long exchanges, bool *clear) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return CUPIC_ERR_CUDA;
   std::lock_guard<std::mutex> lock(g_mu);
@@ -69,7 +78,7 @@ int scratch_for_current_device(unsigned char **out, unsigned long long **sync, l
   *clear = (g_exchanges[dev] += exchanges) > (1ll << 30);
   if (*clear) g_exchanges[dev] = exchanges;
   *out = static_cast<unsigned char *>(g_scratch_addr[dev]);
-  *sync = static_cast<unsigned long long *>(g_sync_addr[dev]);
+  *sync = static_cast<SolverSync *>(g_sync_addr[dev]);
   return CUPIC_OK;
 }
 
@@ -114,7 +123,7 @@ extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t 
   if (p->ncx < 2 || p->ncy < 2 || p->ncx > 4096 || !(p->ds > 0) || !(p->eps0 > 0))
     return CUPIC_ERR_ARG;
   unsigned char *scratch = nullptr;
-  unsigned long long *sync = nullptr;
+  SolverSync *sync = nullptr;
   bool clear_halo = false;
   int rc = scratch_for_current_device(&scratch, &sync, (long long)max_sweeps + 4, &clear_halo);
   if (rc) return rc;
@@ -135,6 +144,8 @@ extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t 
   const int M = a.nny - 2, nnx = a.nnx;
   const int P = (nnx + 3) / 4 * 4;
   const long long rows_fit = (long long)(((size_t)dev_max - 1024) / (3 * sizeof(float) * (size_t)P));
+  // (the counters have an array of their own by now; their share stays in the
+  // count, and with it the meshes that are accepted)
   auto need = [&](int g, int k) {
     return kCtlHeadBytes + align256(sizeof(unsigned) * (size_t)(g + 1)) +
            align256(sizeof(float) * 2 * (size_t)g) + sizeof(unsigned long long) * (size_t)2 * g * 2 * k * P;
@@ -169,16 +180,11 @@ extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t 
   if (jacobi_set_smem(sm) != cudaSuccess) return CUPIC_ERR_CUDA;
   int per_sm = 0;
   if (jacobi_max_ctas(sm, &per_sm) != cudaSuccess) return CUPIC_ERR_CUDA;
-  if (per_sm < 1 || G > per_sm * num_sms) return CUPIC_ERR_ARG;
+  if (per_sm < 1 || G > per_sm * num_sms || G > kMaxCtas) return CUPIC_ERR_ARG;
 
-  // scratch layout: status block | sweep counters + barrier | residual slots | halo rows
+  // scratch layout: status block | halo rows
   Ctl *ctl = reinterpret_cast<Ctl *>(scratch);
-  unsigned char *q = scratch + kCtlHeadBytes;
-  unsigned *flags = reinterpret_cast<unsigned *>(q);
-  q += align256(sizeof(unsigned) * (size_t)(G + 1));
-  float *res = reinterpret_cast<float *>(q);
-  q += align256(sizeof(float) * 2 * (size_t)G);
-  unsigned long long *halo = reinterpret_cast<unsigned long long *>(q);
+  unsigned long long *halo = reinterpret_cast<unsigned long long *>(scratch + kCtlHeadBytes);
 
   unsigned long long *acc = reinterpret_cast<unsigned long long *>(const_cast<int64_t *>(rho_dev));
   a.rho[0] = acc;
@@ -200,21 +206,18 @@ extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t 
   J.strip = jacobi_strip_rows(nnx, B + 2 * (G > 1 ? K : 1) - 2);
   J.do_field = e_dev ? 1 : 0;
   J.write_stats = 1;
-  J.flags = flags;
-  J.bar = flags + G;
-  J.res_cta = res;
+  J.flags = sync->flags;
+  J.bar = sync->flags + G;
+  J.res_cta = sync->res;
   J.halo = halo;
-  J.gmax = sync;
-  J.tbar = reinterpret_cast<unsigned *>(sync + 128);
+  J.gmax = sync->gmax;
+  J.tbar = sync->tbar;
   // the mesh is one that the scratch holds; most run faster as register tiles
   const TileForm form = max_error > 0.0 && min_sweeps < max_sweeps ? kTileEarly : kTileFixed;
   const TilePlan tile = max_sweeps > 0 ? tiles_for(dev, num_sms, dev_max, a.nnx, a.nny,
                                                    std::min(forced > 0 ? forced : num_sms, num_sms), form)
                                        : TilePlan{};
-  if (tile.R) {
-    tile_args(tile, &J);
-    J.halo = reinterpret_cast<unsigned long long *>(scratch + kCtlHeadBytes);
-  }
+  if (tile.R) tile_args(tile, &J);
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // the array keeps the previous call's contents: clear the status block

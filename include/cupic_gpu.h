@@ -295,13 +295,13 @@ int cupic_test_bounded_wait(struct cupic_ctx *ctx);
  *            its own work before returning (it reads sweeps_out and
  *            residual_out back)
  * The solver's scratch (sweep counters, residual slots and the halo rows its
- * CTAs trade) lives in a static 8 MiB device array that every GPU loading
- * this library holds until exit.  The call lowers the halo depth, then the
+ * CTAs trade) lives in static device arrays of 8 MiB and 25 KB that every GPU
+ * loading this library holds until exit.  The call lowers the halo depth, then the
  * CTA count, until the scratch fits; meshes for which nothing fits return
  * CUPIC_ERR_CAPACITY.  The largest ncy accepted is 5321 at ncx = 512, 2433
  * at ncx = 1024, 890 at ncx = 2048 and 127 at ncx = 4096.  The first call on a device
- * looks the array up (cudaGetSymbolAddress); make that first call before any
- * stream capture.  All calls share the array and it keeps the last call's
+ * looks the arrays up (cudaGetSymbolAddress); make that first call before any
+ * stream capture.  All calls share the arrays, which keep the last call's
  * contents: calls that overlap on the GPU (other streams, other host
  * threads) race and must be serialised by the caller.  The environment
  * variable CUPIC_JACOBI_CTAS, when set, caps the number of solver CTAs, as

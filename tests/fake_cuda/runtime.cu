@@ -42,6 +42,9 @@ bool capturing = false;
 int give_up_ctas = -1, give_up_depth = -1, batch_give_up = -1;
 float last_ms = 1.0f;
 int solves = 0;
+// while watched: where exchange words and where counters of any launch lay
+bool watching = false;
+std::vector<std::pair<const char *, size_t>> words, counters;
 size_t allocated = 0;
 
 void fault(const std::string &s) { faults.push_back(s); }
@@ -77,6 +80,14 @@ void need(const char *what, const void *p, size_t bytes, const std::string &who)
     fault(who + ": " + what + " needs " + std::to_string(bytes) + " bytes, has " + std::to_string(room(p)));
 }
 
+void apart(std::vector<std::pair<const char *, size_t>> *mine, const std::vector<std::pair<const char *, size_t>> &others,
+           const void *p, size_t n, const std::string &who) {
+  const char *q = static_cast<const char *>(p);
+  mine->push_back({q, n});
+  for (const auto &o : others)
+    if (q < o.first + o.second && o.first < q + n) return fault(who + ": exchange words and counters in one place");
+}
+
 void solve(const std::string &name, const SimArgs &a, const JacobiArgs &J, dim3 grid, size_t smem) {
   const std::string who = name + " " + std::to_string(a.nnx - 1) + "x" + std::to_string(a.nny - 1) + " G=" +
                           std::to_string(J.G) + " K=" + std::to_string(J.depth);
@@ -98,6 +109,15 @@ void solve(const std::string &name, const SimArgs &a, const JacobiArgs &J, dim3 
   if (!tile) {
     if (J.rows_per_cta < (M + J.G - 1) / J.G) fault(who + ": rows of a block");
     if (smem < jacobi_smem_bytes(J.rows_per_cta, J.G > 1 ? J.depth : 1, J.pitch)) fault(who + ": shared memory");
+  }
+  if (watching) {
+    if (J.G > 1 && !(tile && J.near))
+      apart(&words, counters, J.halo, tile ? 2 * (size_t)J.pwords * 8 : 4 * G * K * J.pitch * 8, who);
+    if (J.G > 1 && !tile) {
+      apart(&counters, words, J.flags, (G + 1) * 4, who);
+      apart(&counters, words, J.res_cta, 2 * G * 4, who);
+    }
+    if (tile) apart(&counters, words, J.gmax, 130 * 8, who);
   }
   if (capturing) return;
   const size_t nodes = (size_t)a.nnx * a.nny;
@@ -173,7 +193,13 @@ void fake_give_up(int ctas, int depth) {
 }
 // the n-th batched solve from now gives up, in its last member
 void fake_batch_give_up(int n) { batch_give_up = n; }
+void fake_watch() {
+  watching = true;
+  words.clear();
+  counters.clear();
+}
 void fake_reset() {
+  watching = false;
   faults.clear();
   launches.clear();
   give_up_ctas = give_up_depth = batch_give_up = -1;

@@ -197,3 +197,27 @@ def test_batched_trial_that_gives_up_tunes_nothing(fake):
     for s in sims:
         s.close()
     assert faults(fake) == []
+
+
+def test_static_scratch_keeps_words_and_counters_apart(fake, monkeypatch):
+    """Calls of the solve on device buffers share one static array, and a halo word
+    is told by the number in its upper half: no call's words lie where another
+    leaves counters or residuals."""
+    fake.fake_watch()
+    fake.fake_alloc.restype = ctypes.c_void_p
+    fake.fake_alloc.argtypes = [ctypes.c_uint64]
+    for ncx, ncy in ((256, 1024), (40, 3000), (1024, 300), (64, 90), (300, 700)):
+        p = params(ncx, ncy)
+        nodes = p.nnx * p.nny
+        rho, phi = fake.fake_alloc(8 * nodes), fake.fake_alloc(4 * nodes)
+        for ctas in (None, "2", "5", "7", "151"):
+            if ctas:
+                monkeypatch.setenv("CUPIC_JACOBI_CTAS", ctas)
+            else:
+                monkeypatch.delenv("CUPIC_JACOBI_CTAS", raising=False)
+            for sweeps in (0, 50):  # no sweeps: the launches of jacobi.cu
+                rc = fake.cupic_poisson_solver_static(ctypes.byref(p), rho, phi, None, 1e-3, 1, sweeps, 1, None, None,
+                                                      None)
+                assert rc in (0, 5), (ncx, ncy, ctas)
+    assert fake.fake_launches(b"k_jacobi") > 0 and fake.fake_launches(b"k_tile") > 0
+    assert faults(fake) == []
