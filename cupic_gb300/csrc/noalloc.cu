@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <map>
+#include <new>
 #include <tuple>
 
 #include "cupic_internal.cuh"
@@ -109,16 +110,9 @@ TilePlan tiles_for(int dev, int num_sms, int dev_max, int nnx, int nny, int max_
   return kept[key] = pick;
 }
 
-}  // namespace
-}  // namespace cupic
-
-using namespace cupic;
-
-extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t *rho_dev,
-                                           float *phi_dev, float *e_dev, double max_error,
-                                           int32_t min_sweeps, int32_t max_sweeps,
-                                           int32_t check_every, void *stream, int32_t *sweeps_out,
-                                           float *residual_out) {
+int solve_static(const cupic_params *p, const int64_t *rho_dev, float *phi_dev, float *e_dev, double max_error,
+                 int32_t min_sweeps, int32_t max_sweeps, int32_t check_every, void *stream, int32_t *sweeps_out,
+                 float *residual_out) {
   if (!p || !rho_dev || !phi_dev || max_sweeps < 0) return CUPIC_ERR_ARG;
   if (p->ncx < 2 || p->ncy < 2 || p->ncx > 4096 || !(p->ds > 0) || !(p->eps0 > 0))
     return CUPIC_ERR_ARG;
@@ -243,4 +237,22 @@ extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t 
   if (residual_out) *residual_out = out.residual;
   if (out.step_flags & CUPIC_FLAG_TIMEOUT) return CUPIC_ERR_TIMEOUT;
   return CUPIC_OK;
+}
+
+}  // namespace
+}  // namespace cupic
+
+// The search for a layout allocates host memory, the first time for each mesh
+// and kernel: no exception of that leaves the C-ABI.
+extern "C" int cupic_poisson_solver_static(const cupic_params *p, const int64_t *rho_dev,
+                                           float *phi_dev, float *e_dev, double max_error,
+                                           int32_t min_sweeps, int32_t max_sweeps,
+                                           int32_t check_every, void *stream, int32_t *sweeps_out,
+                                           float *residual_out) {
+  try {
+    return cupic::solve_static(p, rho_dev, phi_dev, e_dev, max_error, min_sweeps, max_sweeps, check_every, stream,
+                               sweeps_out, residual_out);
+  } catch (const std::bad_alloc &) {
+    return CUPIC_ERR_NOMEM;
+  }
 }

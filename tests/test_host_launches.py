@@ -7,6 +7,7 @@ import glob
 import os
 import shutil
 import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -25,7 +26,8 @@ def fake_path(tmp_path_factory):
     subprocess.run([build.nvcc()] + build.common_flags() + ["-I", build.CSRC, "-D__CUDA_DEVICE_RUNTIME_API_H__", "-c",
                    os.path.join(HERE, "fake_cuda", "runtime.cu"), "-o", obj], check=True)
     objs = [os.path.join(build.OUT, os.path.splitext(s)[0] + ".o") for s in build.SOURCES]
-    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", lib, obj] + objs + ["-lpthread"], check=True)
+    subprocess.run(["g++", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-o", lib, obj,
+                    os.path.join(HERE, "fake_cuda", "new.cpp")] + objs + ["-lpthread"], check=True)
     return lib
 
 
@@ -221,3 +223,27 @@ def test_static_scratch_keeps_words_and_counters_apart(fake, monkeypatch):
                 assert rc in (0, 5), (ncx, ncy, ctas)
     assert fake.fake_launches(b"k_jacobi") > 0 and fake.fake_launches(b"k_tile") > 0
     assert faults(fake) == []
+
+
+def test_static_solve_without_host_memory_returns_a_status(fake):
+    """The layout's search allocates host memory: where that fails, the C entry returns
+    a status, and no exception leaves it (in a child: one would end it)."""
+    run = """
+import ctypes, sys
+import cupic_gb300 as cg
+cg.library_path = lambda: sys.argv[1]
+L = cg.load_library()
+L.fake_alloc.restype = ctypes.c_void_p
+L.fake_alloc.argtypes = [ctypes.c_uint64]
+L.fake_new_left.argtypes = [ctypes.c_longlong]
+p = cg.workload_params("tiny")
+rho, phi = L.fake_alloc(8 * p.nnx * p.nny), L.fake_alloc(4 * p.nnx * p.nny)
+codes = set()
+for left in list(range(40)) + [-1]:
+    L.fake_new_left(left)
+    rc = L.cupic_poisson_solver_static(ctypes.byref(p), rho, phi, None, 1e-3, 1, 50, 1, None, None, None)
+    L.fake_new_left(-1)
+    codes.add(rc)
+assert codes == {0, 3}, codes  # CUPIC_ERR_NOMEM
+"""
+    subprocess.run([sys.executable, "-c", run, cg.library_path()], check=True, cwd=os.path.dirname(HERE))
