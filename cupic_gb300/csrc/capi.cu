@@ -212,7 +212,7 @@ int layout_species(cupic_ctx *c, int sp, const std::vector<int32_t> &capv) {
   CU(dalloc(c, &S.stage_up, (size_t)ncy * S.stage_cap));
   CU(dalloc(c, &S.stage_down, (size_t)ncy * S.stage_cap));
   CU(dalloc(c, &S.inj_tin, (size_t)S.inj_cap));
-  CU(dalloc(c, &S.inj_v, (size_t)3 * S.inj_cap));
+  CU(dalloc(c, &S.inj_v, few_draws(c->a) ? (size_t)3 * S.inj_cap : 0));
   CU(dalloc(c, &S.inj_p, (size_t)S.inj_cap));
   CU(dalloc(c, &S.inj_d, (size_t)S.inj_cap));
   const bool uniform = std::all_of(capv.begin(), capv.end(), [&](int32_t v) { return v == capv[0]; });

@@ -60,7 +60,7 @@ struct SpeciesDev {
   int32_t stage_cap;
   int32_t inj_cap;        // most particles injected per step
   double *inj_tin;        // [inj_cap] scratch: injection time of each draw
-  double *inj_v;          // [inj_cap][3] and its x, vx, vy before the field's kick
+  double *inj_v;          // [inj_cap][3] and its x, vx, vy before the field's kick (few draws)
   float4 *inj_p;          // [inj_cap] scratch: the injected particles of the step
   int32_t *inj_d;         // [inj_cap] scratch: their rows (< 0: removed)
 };

@@ -247,3 +247,18 @@ for left in list(range(40)) + [-1]:
 assert codes == {0, 3}, codes  # CUPIC_ERR_NOMEM
 """
     subprocess.run([sys.executable, "-c", run, cg.library_path()], check=True, cwd=os.path.dirname(HERE))
+
+
+def test_draws_beside_the_solve_take_memory_only_where_they_are_made(fake):
+    """The scratch of few draws made beside the solve (24 bytes each) is for contexts
+    that draw few; one that draws many holds no more than the draws themselves."""
+    sizes = {}
+    for kte in (1.0, 1e10):  # electrons of mass 1
+        p = params(64, 4, kte=kte)
+        fake.fake_reset()
+        with cg.Sim(p):
+            sizes[kte] = fake.fake_allocated()
+    caps = [4 * np.ceil(p.dt * p.n * p.ncx * p.ds ** 2 * (kte / (2 * np.pi)) ** 0.5) + 1024 for kte in sizes]
+    assert caps[0] < 1100 and caps[1] > 2e4
+    # a draw's time, particle and row: 8 + 16 + 4 bytes
+    assert sizes[1e10] - sizes[1.0] <= 28 * (caps[1] - caps[0])
