@@ -1051,7 +1051,8 @@ int capture_steps(cupic_ctx *c, int steps, cudaGraphExec_t *exec) {
 // One graph launch takes 2.5 us of the stream between two steps, so a run of
 // kLongRun steps or more goes in graphs of kStepsPerGraph (32x128 55.7 -> 53.0
 // us a step, 256x1024 212.4 -> 209.3, 301x700 251.0 -> 247.8).  They cost
-// 130 us to capture, once, which a run of 60 steps just earns back.
+// 130 us to capture, once, which a run of 60 steps just earns back; a step of
+// the precision form off the tiles, a launch per correction, goes alone.
 constexpr int kStepsPerGraph = 8, kLongRun = 64;
 
 // n steps, graph-launched where the step is captured
@@ -1064,7 +1065,8 @@ int launch_steps(cupic_ctx *c, int64_t n) {
     c->graph_ok = c->graph != nullptr;  // if not, direct launches
   }
   const int64_t one = solves_of(c, c->p.max_sweeps);
-  if (n >= kLongRun && c->graph_ok && !c->graph_many && kStepsPerGraph * one <= kEpochGuard) {
+  const bool short_step = c->p.refine_every <= 0 || c->lay.tile.R;
+  if (n >= kLongRun && short_step && c->graph_ok && !c->graph_many && kStepsPerGraph * one <= kEpochGuard) {
     const int rc = capture_steps(c, kStepsPerGraph, &c->graph_many);
     if (rc) return rc;
   }

@@ -262,3 +262,22 @@ def test_draws_beside_the_solve_take_memory_only_where_they_are_made(fake):
     assert caps[0] < 1100 and caps[1] > 2e4
     # a draw's time, particle and row: 8 + 16 + 4 bytes
     assert sizes[1e10] - sizes[1.0] <= 28 * (caps[1] - caps[0])
+
+
+def test_steps_of_many_launches_go_one_to_a_graph(fake, monkeypatch):
+    """A graph of several steps saves the time between graph launches, 2.5 us a step;
+    a precision-form step off the tiles is a launch per correction, and eight of
+    them would take longer to capture than that earns."""
+    monkeypatch.setenv("CUPIC_JACOBI_NOSTRIP", "1")  # no tiles
+    p = params(48, 40, refine_every=4, max_sweeps=400)
+    with cg.Sim(p) as sim:
+        sim.init_plasma()
+        fake.fake_reset()
+        sim.step(64)
+        assert fake.fake_launches(b"k_jacobi") == 101  # one step's, captured once
+    monkeypatch.delenv("CUPIC_JACOBI_NOSTRIP")
+    with cg.Sim(p) as sim:
+        sim.init_plasma()
+        fake.fake_reset()
+        sim.step(64)
+        assert fake.fake_launches(b"k_tile") == 1 + 8
