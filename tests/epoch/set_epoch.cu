@@ -4,6 +4,8 @@
 
 #include "ctx.h"
 
+using namespace cupic;
+
 extern "C" int set_epoch(cupic_ctx *c, unsigned v) {
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return 1;
   return cudaMemcpy(&c->ctl->jepoch, &v, sizeof(v), cudaMemcpyHostToDevice) != cudaSuccess;
