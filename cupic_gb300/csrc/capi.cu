@@ -775,6 +775,7 @@ cudaError_t launch_solve(const cupic_ctx *c, const JacobiArgs &J) {
 // solved by the launches that read both.
 int seam_columns(cupic_ctx *c, bool two) {
   if (!c->phi64 || (two ? !c->lay.tile.R : !c->left.R)) return CUPIC_OK;
+  CU(cudaStreamSynchronize(c->stream));  // the graph may be running
   destroy_graph(c);
   if (!two) {
     const int rc = set_tile_plan(c, c->left);
